@@ -59,11 +59,16 @@ constexpr int BX = 128;   // threads per block (4 warps x 128 points)
 
 struct Geo {
   int nx, nz, P, halo, W;
+  int WL, xr;   // x strips: storage columns [0, WL) = columns 1 .. WL, [WL, W) = columns xr + 1 .. (see xcol)
   long long F;  // floats per padded field
   float idx, idz;
   __host__ __device__ __forceinline__ long long lin(int i, int j) const {
     return (long long)(j + ZPAD - 1) * P + (i + XPAD - 1);
   }
+  // Storage column of the x strips' memory variables and coefficients for
+  // grid column i: whole groups of four columns (the points of one thread) on
+  // both sides, so that a thread moves its cells as one float4.
+  __host__ __device__ __forceinline__ int xcol(int i) const { return i - 1 < WL ? i - 1 : WL + (i - 1 - xr); }
 };
 
 struct PArgs {
@@ -74,6 +79,8 @@ struct PArgs {
   long long xs, zs;
   const float* m0;                   // fact_m0 (padded, shared by the shots)
   const float* cp; int cps;          // per shot: axis x then z, [a(na), a_h(nh), b(na), b_h(nh)]
+  const float* cx4;                  // per shot: [a, b, a_h, b_h] of axis x by storage column (4 W)
+  int tz;                            // rows per block
   // adjoint only: correlation with the forward pressure slots
   const float* pc; const float* po;  // p[it], p[it-1], [shot][F]
   float* acc;                        // [shot][3][F]: m0 term, m1 x term, m1 z term
@@ -88,11 +95,30 @@ struct VArgs {
   long long xs, zs;
   const float* m1x; const float* m1z;
   const float* cp; int cps;
+  const float* cx4;
+  int tz;
 };
 
+// (c1 f1 - c2 f2 + c2 f3 - c1 f4) / h.  Every rounding of the stencils is
+// spelled out (left to the compiler, the products that become part of a
+// fused multiply-add change with the registers and the shape of the code
+// around them, and the results with them): c2 f3 is rounded on its own where
+// ROUND3 is set, everything else is a chain of fused multiply-adds.
+template <bool ROUND3>
 __device__ __forceinline__ float d4(float f1, float f2, float f3, float f4, float inv) {
-  const float c1 = 1.0f / 24.0f, c2 = 27.0f / 24.0f;
-  return (c1 * f1 - c2 * f2 + c2 * f3 - c1 * f4) * inv;
+  constexpr float c1 = 1.0f / 24.0f, c2 = 27.0f / 24.0f;
+  const float t = __fmaf_rn(c1, f1, -__fmul_rn(c2, f2));
+  const float u = ROUND3 ? __fadd_rn(t, __fmul_rn(c2, f3)) : __fmaf_rn(c2, f3, t);
+  return __fmul_rn(__fmaf_rn(-c1, f4, u), inv);
+}
+// d4 along x at a thread's four points from the seven values around them; bit
+// e of ROUND3 sets point e's rounding.
+template <unsigned ROUND3>
+__device__ __forceinline__ void d4x(float (&d)[4], const float (&a)[7], float inv) {
+  d[0] = d4<(ROUND3 & 1) != 0>(a[0], a[1], a[2], a[3], inv);
+  d[1] = d4<(ROUND3 & 2) != 0>(a[1], a[2], a[3], a[4], inv);
+  d[2] = d4<(ROUND3 & 4) != 0>(a[2], a[3], a[4], a[5], inv);
+  d[3] = d4<(ROUND3 & 8) != 0>(a[3], a[4], a[5], a[6], inv);
 }
 
 // Coefficient index (1-based, 0 = no memory variable) of fdgen.jl:137-161.
@@ -110,16 +136,21 @@ __host__ __device__ __forceinline__ int k_vel(int pos, int n, int halo) {
   if (pos >= n - halo) return pos - n + 2 * halo + 1;
   return 0;
 }
-// psi = b psi + a dv; returns dv + psi
-__device__ __forceinline__ float cpml_upd(float* psi, float a, float b, float dv) {
-  const float nv = b * (*psi) + a * dv;
-  *psi = nv;
-  return dv + nv;
-}
 
 struct F4 {
   float v[4];
 };
+// psi = b psi + a dv and dv += psi for the points of `mask` among a thread's
+// four (the cells of the other points hold nothing that is read)
+__device__ __forceinline__ void cpml_upd4(float (&dv)[4], F4& psi, const F4& a, const F4& b, unsigned mask) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float nv = __fmaf_rn(a.v[e], dv[e], __fmul_rn(b.v[e], psi.v[e]));
+    psi.v[e] = nv;
+    if (mask >> e & 1) dv[e] = __fadd_rn(dv[e], nv);
+  }
+}
+__device__ __forceinline__ F4 splat4(float x) { return F4{{x, x, x, x}}; }
 __device__ __forceinline__ F4 ld4z(const float* __restrict__ p, long long c, bool ok) {
   F4 r;
   if (ok) {
@@ -156,30 +187,57 @@ __device__ __forceinline__ float ldz(const float* __restrict__ p, long long c, b
 
 constexpr unsigned FULL = 0xffffffffu;
 
+// Which of the thread's four columns i0 .. i0 + 3 hold a memory variable along
+// x: k != 0 of k_pres (2 <= i <= nx - 1) or k_vel (i <= nx - 1).
+__device__ __forceinline__ unsigned xmask_pres(const Geo& g, int i0) {
+  unsigned m = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = i0 + e;
+    if (i >= 2 && i <= g.nx - 1 && (i <= g.halo + 1 || i >= g.nx - g.halo)) m |= 1u << e;
+  }
+  return m;
+}
+__device__ __forceinline__ unsigned xmask_vel(const Geo& g, int i0) {
+  unsigned m = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = i0 + e;
+    if (i <= g.nx - 1 && (i <= g.halo || i >= g.nx - g.halo)) m |= 1u << e;
+  }
+  return m;
+}
+
 // Pressure update (update_p_CPML! on 2:nx-1, 2:nz-1; every other node copies
-// p through) for the shot blockIdx.z: four x points per thread, each warp 128
-// consecutive points, a block 512 points x TZ rows.  The thread walks its
-// columns down the band: vz rows j-2 .. j+1 stay in registers, the x
-// neighbours of vx come from the adjacent lanes.  CORR (adjoint): also
-// acc[0] += -(p_new (pc - po) / dt), acc[1] += vx dpc/dx, acc[2] += vz dpc/dz
-// (pc rows j-1 .. j+2 in registers).
-// Resident blocks per SM: the correlating adjoint kernel runs faster at 7
-// (<= 72 registers; 5.06 against 4.92 TB/s for the adjoint step pair on 64
-// shots), the forward one is left at its own register count (55) by a bound
-// it already meets.
+// p through): four x points per thread, each warp 128 consecutive points, a
+// block 512 points x tz rows of one shot (x tiles fastest, then shots, then
+// bands, so that the shots of a band share the material rows through L2).  The
+// thread walks its columns down the band: vz rows j-2 .. j+1 stay in
+// registers, the x neighbours of vx come from the adjacent lanes.  CORR
+// (adjoint): also acc[0] += -(p_new (pc - po) / dt), acc[1] += vx dpc/dx,
+// acc[2] += vz dpc/dz (pc rows j-1 .. j+2 in registers).
+// The memory variables of a thread's four points are one float4 along either
+// axis, loaded with the rest of the row before anything is computed: point by
+// point they were a chain of four dependent loads per axis and row, which set
+// the time of every row next to a strip (one shot of 402 x 301, 600 steps:
+// 27.4 -> 14.9 ms with the same 8-row bands; 8 shots of 2001 x 801, 300 steps,
+// gradient: 120.8 -> 97.1 ms).  Bound by HBM latency and bandwidth: 7 resident
+// blocks per SM (6 for the correlating kernel, which holds two z windows)
+// against 96.0 ms run 99.1 at 6 / 6 and 96.3 at 7 / 5; at 8 / 7 the kernels spill.
 template <bool CORR>
 struct VdPBounds {
-  static constexpr int MINB = CORR ? 7 : 8;
+  static constexpr int MINB = CORR ? 6 : 7;
 };
 
-template <int TZ, bool CORR>
+template <bool CORR>
 __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs A) {
   const Geo g = A.g;
-  const int s = blockIdx.z;
+  const int tx = (g.nx + 511) / 512;
+  const int s = blockIdx.x / tx;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wx0 = (blockIdx.x * 4 + warp) * 128;
-  const int j0 = blockIdx.y * TZ + 1;
-  const int j1 = min(j0 + TZ - 1, g.nz);
+  const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
+  const int j0 = blockIdx.y * A.tz + 1;
+  const int j1 = min(j0 + A.tz - 1, g.nz);
   if (j0 > j1 || wx0 >= g.nx) return;  // warp uniform (no block-level synchronisation below)
   const int i0 = wx0 + lane * 4 + 1;
   const bool ldok = i0 <= g.nx + 2;
@@ -189,15 +247,17 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
   const float* pin = A.pin + so;
   float* pout = A.pout + so;
   const int na = 2 * g.halo + 2, nh = 2 * g.halo;
-  const float* cx = A.cp + (long long)s * A.cps;
-  const float* cz = cx + 2 * na + 2 * nh;
-  float* xix = A.xi_x + (long long)s * A.xs;
-  float* xiz = A.xi_z + (long long)s * A.zs;
+  const float* cz = A.cp + (long long)s * A.cps + 2 * na + 2 * nh;
   const int P = g.P;
-  const bool xstrip = i0 <= g.halo + 1 || i0 + 3 >= g.nx - g.halo;
+  const unsigned mx = xmask_pres(g, i0);
+  const float* cx4 = A.cx4 + (long long)s * (4 * g.W) + (mx ? g.xcol(i0) : 0);
+  float* xix = A.xi_x + (long long)s * A.xs + (mx ? g.xcol(i0) : 0);
+  float* xiz = A.xi_z + (long long)s * A.zs + (i0 - 1);
   const float* __restrict__ pc = CORR ? A.pc + so : nullptr;
   const float* __restrict__ po = CORR ? A.po + so : nullptr;
   float* acc = CORR ? A.acc + 3 * so : nullptr;
+  const bool edge = (lane == 0 || lane == 31) && ldok;
+  const int eo = lane == 0 ? -1 : 4;  // the edge lanes' own x neighbours (loaded; the others are shuffled)
   long long c = g.lin(i0, j0);
   F4 z0 = ld4z(vz, c - 2 * P, ldok), z1 = ld4z(vz, c - P, ldok), z2 = ld4z(vz, c, ldok), z3 = ld4z(vz, c + P, ldok);
   F4 q0, q1, q2, q3;
@@ -206,41 +266,47 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
   }
   for (int j = j0; j <= j1; ++j, c += P) {
     const bool more = j + 1 <= j1;
+    const bool jin = j >= 2 && j <= g.nz - 1;
+    const int kz = jin ? k_pres(j, g.nz, g.halo) : 0;
+    const F4 X = ld4z(vx, c, ldok);
+    const float ex1 = ldz(vx, c + eo, edge), ex0 = ldz(vx, c - 2, edge && lane == 0);
+    const F4 PI = ld4p(pin, c, ldok), M0 = ld4z(A.m0, c, ldok);
+    F4 XI, ZI;
+    const bool xs = mx && jin, zs = kz && ldok;
+    if (xs) XI = ld4rw(xix, (long long)(j - 1) * g.W);
+    if (zs) ZI = ld4rw(xiz, (long long)(kz - 1) * P);
     const F4 zn = ld4z(vz, c + 2 * P, ldok && more);
     F4 qn;
     if (CORR) qn = ld4z(pc, c + 3 * P, ldok && more);
-    const F4 X = ld4z(vx, c, ldok);
     // vx at i0-2 .. i0+4 (row j)
     float xa[7];
     xa[0] = __shfl_up_sync(FULL, X.v[2], 1);
     xa[1] = __shfl_up_sync(FULL, X.v[3], 1);
     xa[6] = __shfl_down_sync(FULL, X.v[0], 1);
     if (lane == 0) {
-      xa[0] = ldz(vx, c - 2, ldok);
-      xa[1] = ldz(vx, c - 1, ldok);
+      xa[0] = ex0;
+      xa[1] = ex1;
     }
-    if (lane == 31) xa[6] = ldz(vx, c + 4, ldok);
+    if (lane == 31) xa[6] = ex1;
+    float dvx[4], dvz[4], out[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) xa[2 + e] = X.v[e];
-    const F4 PI = ld4p(pin, c, ldok), M0 = ld4z(A.m0, c, ldok);
-    const bool jin = j >= 2 && j <= g.nz - 1;
-    const int kz = jin ? k_pres(j, g.nz, g.halo) : 0;
-    float out[4];
+    d4x<CORR ? 0u : 2u>(dvx, xa, g.idx);  // vx[i-2 .. i+1]
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dvz[e] = d4<false>(z0.v[e], z1.v[e], z2.v[e], z3.v[e], g.idz);  // vz rows j-2 .. j+1
+    if (xs) {
+      cpml_upd4(dvx, XI, ld4z(cx4, 0, true), ld4z(cx4, g.W, true), mx);
+      st4v(xix, (long long)(j - 1) * g.W, XI.v);
+    }
+    if (zs) {
+      cpml_upd4(dvz, ZI, splat4(cz[kz - 1]), splat4(cz[na + nh + kz - 1]), 15u);
+      st4v(xiz, (long long)(kz - 1) * P, ZI.v);
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int i = i0 + e;
-      float dvx = d4(xa[e], xa[e + 1], xa[e + 2], xa[e + 3], g.idx);  // vx[i-2 .. i+1]
-      float dvz = d4(z0.v[e], z1.v[e], z2.v[e], z3.v[e], g.idz);      // vz rows j-2 .. j+1
-      if (jin && i >= 2 && i <= g.nx - 1) {
-        if (xstrip) {
-          const int kx = k_pres(i, g.nx, g.halo);
-          if (kx) dvx = cpml_upd(xix + (long long)(j - 1) * g.W + (kx - 1), cx[kx - 1], cx[na + nh + kx - 1], dvx);
-        }
-        if (kz) dvz = cpml_upd(xiz + (long long)(kz - 1) * P + (i - 1), cz[kz - 1], cz[na + nh + kz - 1], dvz);
-        out[e] = PI.v[e] - M0.v[e] * (dvx + dvz);
-      } else {
-        out[e] = PI.v[e];
-      }
+      const float v = __fmaf_rn(-M0.v[e], __fadd_rn(dvx[e], dvz[e]), PI.v[e]);
+      out[e] = (jin && i >= 2 && i <= g.nx - 1) ? v : PI.v[e];
     }
     if (ldok) {
       if (i0 + 3 <= g.nx) {
@@ -269,12 +335,13 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
         // vx(nx, .) / vz(., nz)), so whole float4s are updated.
         const F4 PO = ld4z(po, c, true);
         F4 G0 = ld4rw(acc, c), G1 = ld4rw(acc + g.F, c), G2 = ld4rw(acc + 2 * g.F, c);
-        float n0[4], n1[4], n2[4];
+        float n0[4], n1[4], n2[4], dp[4];
+        d4x<7u>(dp, pa, g.idx);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          n0[e] = G0.v[e] + (-(out[e] * (q1.v[e] - PO.v[e]) * A.idt));
-          n1[e] = G1.v[e] + X.v[e] * d4(pa[e], pa[e + 1], pa[e + 2], pa[e + 3], g.idx);
-          n2[e] = G2.v[e] + z2.v[e] * d4(q0.v[e], q1.v[e], q2.v[e], q3.v[e], g.idz);
+          n0[e] = __fmaf_rn(-__fmul_rn(out[e], __fsub_rn(q1.v[e], PO.v[e])), A.idt, G0.v[e]);
+          n1[e] = __fmaf_rn(X.v[e], dp[e], G1.v[e]);
+          n2[e] = __fmaf_rn(z2.v[e], d4<false>(q0.v[e], q1.v[e], q2.v[e], q3.v[e], g.idz), G2.v[e]);
         }
         st4v(acc, c, n0);
         st4v(acc + g.F, c, n1);
@@ -287,15 +354,16 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
 }
 
 // Velocity update (update_vx_CPML! on 1:nx-1 x 1:nz, update_vy_CPML! on
-// 1:nx x 1:nz-1) for the shot blockIdx.z; p rows j-1 .. j+2 in registers.
-template <int TZ>
-__global__ void __launch_bounds__(BX) k_vd_v(const VArgs A) {
+// 1:nx x 1:nz-1); p rows j-1 .. j+2 in registers, the same split and the same
+// handling of the memory variables as k_vd_p.
+__global__ void __launch_bounds__(BX, 7) k_vd_v(const VArgs A) {
   const Geo g = A.g;
-  const int s = blockIdx.z;
+  const int tx = (g.nx + 511) / 512;
+  const int s = blockIdx.x / tx;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wx0 = (blockIdx.x * 4 + warp) * 128;
-  const int j0 = blockIdx.y * TZ + 1;
-  const int j1 = min(j0 + TZ - 1, g.nz);
+  const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
+  const int j0 = blockIdx.y * A.tz + 1;
+  const int j1 = min(j0 + A.tz - 1, g.nz);
   if (j0 > j1 || wx0 >= g.nx) return;
   const int i0 = wx0 + lane * 4 + 1;
   const bool ldok = i0 <= g.nx + 2;
@@ -304,67 +372,70 @@ __global__ void __launch_bounds__(BX) k_vd_v(const VArgs A) {
   float* vx = A.vx + so;
   float* vz = A.vz + so;
   const int na = 2 * g.halo + 2, nh = 2 * g.halo;
-  const float* cx = A.cp + (long long)s * A.cps;
-  const float* cz = cx + 2 * na + 2 * nh;
-  float* psx = A.psi_x + (long long)s * A.xs;
-  float* psz = A.psi_z + (long long)s * A.zs;
+  const float* cz = A.cp + (long long)s * A.cps + 2 * na + 2 * nh;
   const int P = g.P;
-  const bool xstrip = i0 <= g.halo || i0 + 3 >= g.nx - g.halo;
+  const unsigned mx = xmask_vel(g, i0);
+  const float* cx4 = A.cx4 + (long long)s * (4 * g.W) + 2 * g.W + (mx ? g.xcol(i0) : 0);
+  float* psx = A.psi_x + (long long)s * A.xs + (mx ? g.xcol(i0) : 0);
+  float* psz = A.psi_z + (long long)s * A.zs + (i0 - 1);
+  const bool edge = (lane == 0 || lane == 31) && ldok;
+  const int eo = lane == 0 ? -1 : 4;
   long long c = g.lin(i0, j0);
   F4 w0 = ld4z(p, c - P, ldok), w1 = ld4z(p, c, ldok), w2 = ld4z(p, c + P, ldok), w3 = ld4z(p, c + 2 * P, ldok);
   for (int j = j0; j <= j1; ++j, c += P) {
     const bool more = j + 1 <= j1;
+    const bool zrow = j <= g.nz - 1;
+    const int kz = zrow ? k_vel(j, g.nz, g.halo) : 0;
+    const float e1 = ldz(p, c + eo, edge), e2 = ldz(p, c + 5, edge && lane == 31);
+    const F4 VX = ld4p(vx, c, ldok), MX = ld4z(A.m1x, c, ldok);
+    const F4 VZ = ld4p(vz, c, ldok && zrow), MZ = ld4z(A.m1z, c, ldok && zrow);
+    F4 XI, ZI;
+    const bool zs = kz && ldok;
+    if (mx) XI = ld4rw(psx, (long long)(j - 1) * g.W);
+    if (zs) ZI = ld4rw(psz, (long long)(kz - 1) * P);
     const F4 wn = ld4z(p, c + 3 * P, ldok && more);
     // p at i0-1 .. i0+5 (row j)
     float pa[7];
     pa[0] = __shfl_up_sync(FULL, w1.v[3], 1);
     pa[5] = __shfl_down_sync(FULL, w1.v[0], 1);
     pa[6] = __shfl_down_sync(FULL, w1.v[1], 1);
-    if (lane == 0) pa[0] = ldz(p, c - 1, ldok);
+    if (lane == 0) pa[0] = e1;
     if (lane == 31) {
-      pa[5] = ldz(p, c + 4, ldok);
-      pa[6] = ldz(p, c + 5, ldok);
+      pa[5] = e1;
+      pa[6] = e2;
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) pa[1 + e] = w1.v[e];
-    if (ldok) {
-      const F4 VX = ld4rw(vx, c), MX = ld4z(A.m1x, c, true);
-      float nv[4];
+    float d[4], nv[4];
+    d4x<7u>(d, pa, g.idx);  // p[i-1 .. i+2]
+    if (mx) {
+      cpml_upd4(d, XI, ld4z(cx4, 0, true), ld4z(cx4, g.W, true), mx);
+      st4v(psx, (long long)(j - 1) * g.W, XI.v);
+    }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = i0 + e;
-        float d = d4(pa[e], pa[e + 1], pa[e + 2], pa[e + 3], g.idx);  // p[i-1 .. i+2]
-        if (xstrip && i <= g.nx - 1) {
-          const int kx = k_vel(i, g.nx, g.halo);
-          if (kx) d = cpml_upd(psx + (long long)(j - 1) * g.W + (kx - 1), cx[na + kx - 1], cx[2 * na + nh + kx - 1], d);
-        }
-        nv[e] = VX.v[e] - MX.v[e] * d;
+    for (int e = 0; e < 4; ++e) nv[e] = __fmaf_rn(-MX.v[e], d[e], VX.v[e]);
+    if (i0 + 3 <= g.nx - 1) {
+      st4v(vx, c, nv);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (i0 + e <= g.nx - 1) vx[c + e] = nv[e];
+    }
+    if (zrow) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) d[e] = d4<false>(w0.v[e], w1.v[e], w2.v[e], w3.v[e], g.idz);  // p rows j-1 .. j+2
+      if (zs) {
+        cpml_upd4(d, ZI, splat4(cz[na + kz - 1]), splat4(cz[2 * na + nh + kz - 1]), 15u);
+        st4v(psz, (long long)(kz - 1) * P, ZI.v);
       }
-      if (i0 + 3 <= g.nx - 1) {
-        st4v(vx, c, nv);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) nv[e] = __fmaf_rn(-MZ.v[e], d[e], VZ.v[e]);
+      if (i0 + 3 <= g.nx) {
+        st4v(vz, c, nv);
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (i0 + e <= g.nx - 1) vx[c + e] = nv[e];
-      }
-      if (j <= g.nz - 1) {
-        const int kz = k_vel(j, g.nz, g.halo);
-        const F4 VZ = ld4rw(vz, c), MZ = ld4z(A.m1z, c, true);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = i0 + e;
-          float d = d4(w0.v[e], w1.v[e], w2.v[e], w3.v[e], g.idz);  // p rows j-1 .. j+2
-          if (kz && i <= g.nx)
-            d = cpml_upd(psz + (long long)(kz - 1) * P + (i - 1), cz[na + kz - 1], cz[2 * na + nh + kz - 1], d);
-          nv[e] = VZ.v[e] - MZ.v[e] * d;
-        }
-        if (i0 + 3 <= g.nx) {
-          st4v(vz, c, nv);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (i0 + e <= g.nx) vz[c + e] = nv[e];
-        }
+          if (i0 + e <= g.nx) vz[c + e] = nv[e];
       }
     }
     w0 = w1; w1 = w2; w2 = w3; w3 = wn;
@@ -482,7 +553,7 @@ __global__ void __launch_bounds__(BX) k_vd_p_hp(const HArgs A) {
         ff dvz = ffd4(ff{z0.v[e], l0.v[e]}, ff{z1.v[e], l1.v[e]}, ff{z2.v[e], l2.v[e]}, ff{z3.v[e], l3.v[e]}, idz);
         if (xstrip) {
           const int kx = k_pres(i, g.nx, g.halo);
-          if (kx) dvx = cpml_upd64(xix + (long long)(j - 1) * g.W + (kx - 1), cx[kx - 1], cx[na + nh + kx - 1], dvx);
+          if (kx) dvx = cpml_upd64(xix + (long long)(j - 1) * g.W + g.xcol(i), cx[kx - 1], cx[na + nh + kx - 1], dvx);
         }
         if (kz) dvz = cpml_upd64(xiz + (long long)(kz - 1) * P + (i - 1), cz[kz - 1], cz[na + nh + kz - 1], dvz);
         const ff o = ff_sub(ff{PI.v[e], PL.v[e]}, ff_mul(ff{M0.v[e], M0L.v[e]}, ff_add(dvx, dvz)));
@@ -569,7 +640,7 @@ __global__ void __launch_bounds__(BX) k_vd_v_hp(const HArgs A) {
         ff d = ffd4(ff{pa[e], pb[e]}, ff{pa[e + 1], pb[e + 1]}, ff{pa[e + 2], pb[e + 2]}, ff{pa[e + 3], pb[e + 3]}, idx);
         if (xstrip) {
           const int kx = k_vel(i, g.nx, g.halo);
-          if (kx) d = cpml_upd64(psx + (long long)(j - 1) * g.W + (kx - 1), cx[na + kx - 1], cx[2 * na + nh + kx - 1], d);
+          if (kx) d = cpml_upd64(psx + (long long)(j - 1) * g.W + g.xcol(i), cx[na + kx - 1], cx[2 * na + nh + kx - 1], d);
         }
         const ff nv = ff_sub(ff{VX.v[e], VXL.v[e]}, ff_mul(ff{MX.v[e], MXL.v[e]}, d));
         vx[c + e] = nv.hi;
@@ -883,11 +954,11 @@ struct sw_acoustic_vd {
   DevMem ck;                   // [M-2][p, vx, vz][cap][F] then 4 strips [cap][xs|zs]
   DevMem acc;                  // [cap][3][F]
   DevMem tot;                  // [groups][3][F] double
-  DevMem d_desc, d_ll, d_int, d_flt, d_tf, d_tr, d_obs, d_ic, d_adj, d_cp, d_partial, d_balls, d_ball_ptr;
+  DevMem d_desc, d_ll, d_int, d_flt, d_tf, d_tr, d_obs, d_ic, d_adj, d_cp, d_cx4, d_partial, d_balls, d_ball_ptr;
   DevMem d_icd, d_dres, d_snap, d_ccts, d_partial2;
   int snapevery = 0;
   float* const* snap_out = nullptr;
-  int tz = 8;
+  int tz = 0;  // rows per block (0: band_rows)
   // compensated forward (precision 1): low parts of p, vx, vz and of the
   // material factors, FP64 memory variables and coefficients
   int precision = 0;
@@ -1146,6 +1217,26 @@ void build_tables(sw_acoustic_vd* vd, const sw_acoustic_shot* shots, const std::
       for (int q = 0; q < vd->cps; ++q) cps64[(size_t)k * vd->cps + q] = s.cpml64 ? s.cpml64[q] : (double)s.cpml[q];
   }
   upload(vd, vd->d_cp, cps, "C-PML coefficients");
+  {  // axis x by storage column: [a, b] of the pressure update, [a_h, b_h] of the velocity update
+    const Geo& g = vd->g;
+    std::vector<float> cx4((size_t)S * 4 * g.W, 0.0f);
+    for (int k = 0; k < S; ++k) {
+      const float* cx = &cps[(size_t)k * vd->cps];
+      float* o = &cx4[(size_t)k * 4 * g.W];
+      for (int i = 1; i <= g.nx; ++i) {
+        const int kp = k_pres(i, g.nx, g.halo), kv = k_vel(i, g.nx, g.halo);
+        if (kp) {
+          o[g.xcol(i)] = cx[kp - 1];
+          o[g.W + g.xcol(i)] = cx[vd->na + vd->nh + kp - 1];
+        }
+        if (kv && i <= g.nx - 1) {
+          o[2 * g.W + g.xcol(i)] = cx[vd->na + kv - 1];
+          o[3 * g.W + g.xcol(i)] = cx[2 * vd->na + vd->nh + kv - 1];
+        }
+      }
+    }
+    upload(vd, vd->d_cx4, cx4, "C-PML coefficients by column");
+  }
   if (vd->precision == 1) upload(vd, vd->d_cp64, cps64, "C-PML coefficients (FP64)");
   check_cuda(cudaMemsetAsync(vd->d_tr.p, 0, (size_t)std::max<long long>(tr_total, 4) * sizeof(float), st), "traces clear");
   const long long* LL = vd->d_ll.as<long long>();
@@ -1259,18 +1350,19 @@ void zero_state(sw_acoustic_vd* vd, int S, bool adjoint) {
   }
 }
 
-template <int TZ>
-void launch_p_tz(const sw_acoustic_vd* vd, cudaStream_t st, const PArgs& a, int S, bool corr) {
-  const dim3 grid((vd->g.nx + 511) / 512, (vd->g.nz + TZ - 1) / TZ, S);
-  if (corr) k_vd_p<TZ, true><<<grid, BX, 0, st>>>(a);
-  else k_vd_p<TZ, false><<<grid, BX, 0, st>>>(a);
-  check_cuda(cudaGetLastError(), "pressure update launch");
-}
-template <int TZ>
-void launch_v_tz(const sw_acoustic_vd* vd, cudaStream_t st, const VArgs& a, int S) {
-  const dim3 grid((vd->g.nx + 511) / 512, (vd->g.nz + TZ - 1) / TZ, S);
-  k_vd_v<TZ><<<grid, BX, 0, st>>>(a);
-  check_cuda(cudaGetLastError(), "velocity update launch");
+// Rows per block of the VD stencils.  A warp's rows run one after the other
+// (about 2 us each where the fields sit in L2), and a band re-reads the 3 rows
+// of its z window: 4 rows are fastest where the launch fills the GPU (8 x 2001
+// x 801 gradient: 97.9 ms with 2 rows, 96.0 with 4, 98.4 with 8); a launch of
+// fewer than 16 warps per SM takes shorter bands (one shot of 402 x 301: 14.9
+// us per step with 8 rows, 10.0 with 4, 7.5 with 1).
+int band_rows(const sw_acoustic_vd* vd, int S) {
+  if (vd->tz > 0) return vd->tz;
+  const int sms = vd->ctx->num_sms > 0 ? vd->ctx->num_sms : 148;
+  const long long wx = (vd->g.nx + 127) / 128;
+  int tz = 4;
+  while (tz > 1 && S * wx * ((vd->g.nz + tz - 1) / tz) < 16LL * sms) tz /= 2;
+  return tz;
 }
 
 struct Run {
@@ -1293,6 +1385,7 @@ struct Run {
     a.m0 = vd->m0.as<float>();
     a.cp = vd->d_cp.as<float>();
     a.cps = vd->cps;
+    a.cx4 = vd->d_cx4.as<float>();
     a.idt = (float)(1.0 / vd->prm.dt);
     return a;
   }
@@ -1311,17 +1404,22 @@ struct Run {
     a.m1z = vd->m1z.as<float>();
     a.cp = vd->d_cp.as<float>();
     a.cps = vd->cps;
+    a.cx4 = vd->d_cx4.as<float>();
     return a;
   }
-  void launch_p(const PArgs& a, int S, bool corr) const {
-    if (vd->tz == 16) launch_p_tz<16>(vd, st, a, S, corr);
-    else if (vd->tz == 32) launch_p_tz<32>(vd, st, a, S, corr);
-    else launch_p_tz<8>(vd, st, a, S, corr);
+  dim3 grid(int S, int tz) const {
+    return dim3((unsigned)((vd->g.nx + 511) / 512 * S), (unsigned)((vd->g.nz + tz - 1) / tz));
   }
-  void launch_v(const VArgs& a, int S) const {
-    if (vd->tz == 16) launch_v_tz<16>(vd, st, a, S);
-    else if (vd->tz == 32) launch_v_tz<32>(vd, st, a, S);
-    else launch_v_tz<8>(vd, st, a, S);
+  void launch_p(PArgs a, int S, bool corr) const {
+    a.tz = band_rows(vd, S);
+    if (corr) k_vd_p<true><<<grid(S, a.tz), BX, 0, st>>>(a);
+    else k_vd_p<false><<<grid(S, a.tz), BX, 0, st>>>(a);
+    check_cuda(cudaGetLastError(), "pressure update launch");
+  }
+  void launch_v(VArgs a, int S) const {
+    a.tz = band_rows(vd, S);
+    k_vd_v<<<grid(S, a.tz), BX, 0, st>>>(a);
+    check_cuda(cudaGetLastError(), "velocity update launch");
   }
   // algorithmic bytes per node and shot: pressure R vx vz p, W p (16); velocity
   // R p vx vz, W vx vz (20); shared by the shots: fact_m0, fact_m1 x2 (12)
@@ -1493,7 +1591,9 @@ void vd_init(sw_acoustic_vd* vd, sw_ctx* ctx, const sw_acoustic_params* p, int i
   g.halo = p->halo;
   g.P = (int)round_up(g.nx + XPAD + 8, 32);  // the kernels read up to column nx + 38
   g.F = (long long)g.P * (g.nz + 2 * ZPAD);
-  g.W = (int)round_up(2 * g.halo + 2, 4);
+  g.WL = (int)round_up(g.halo + 1, 4);
+  g.xr = std::max(g.WL, (g.nx - g.halo - 1) / 4 * 4);
+  g.W = g.WL + std::max((int)round_up(g.nx, 4) - g.xr, 0);
   g.idx = (float)(1.0 / p->h[0]);
   g.idz = (float)(1.0 / p->h[1]);
   vd->na = 2 * g.halo + 2;
@@ -1854,7 +1954,7 @@ void vd_gradient(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, 
 
 void vd_set_tuning(sw_acoustic_vd* vd, int tz) {
   if (tz != 0 && tz != 8 && tz != 16 && tz != 32) fail(SW_ERR_ARG, "tz must be 0, 8, 16 or 32");
-  vd->tz = tz == 0 ? 8 : tz;
+  vd->tz = tz;
 }
 sw_ctx* vd_ctx(sw_acoustic_vd* vd) { return vd->ctx; }
 sw_acoustic_vd* vd_new() { return new sw_acoustic_vd(); }
