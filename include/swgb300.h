@@ -370,11 +370,11 @@ int sw_elastic_forward_snapshots(sw_elastic* es, int32_t nshots, const sw_elasti
                                  int32_t snapevery, float* const* snapshots);
 
 /* Rows per thread block of the elastic stencil kernels: 8, 16 or 32 (0 =
- * default 8); + 64 selects the one-point-per-thread kernels instead of the
- * four-points-per-thread ones.  The four-point displacement update runs as
- * two launches (ux, then uz; 72 registers each, 7 resident blocks per SM,
- * 5 % faster than one launch of both at 96); + 128 selects the single
- * launch.  A tuning knob of this backend; no reference counterpart. */
+ * default: 4, fewer for launches that would leave SMs short of warps; 8 for
+ * the one-point kernels); + 64 selects the one-point-per-thread kernels
+ * instead of the four-points-per-thread ones.  The four-point displacement
+ * update runs as two launches (ux, then uz; 80 registers each, 6 resident
+ * blocks per SM); + 128 selects the single launch.  A tuning knob of this backend; no reference counterpart. */
 int sw_elastic_set_tuning(sw_elastic* es, int32_t tz);
 
 /* ---------------------------------------------------------------------------

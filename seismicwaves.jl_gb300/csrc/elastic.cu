@@ -64,11 +64,17 @@ constexpr int CTZ = 2;   // rows per block (correlation); the stencil kernels ta
 
 struct Geo {
   int nx, nz, P, halo, ft, W;
+  int WL, xr;   // x strips: storage columns [0, WL) = columns 1 .. WL, [WL, W) = columns xr + 1 .. (see xcol)
   long long F;  // floats per padded field
   float idx, idz;
   __host__ __device__ __forceinline__ long long lin(int i, int j) const {
     return (long long)(j + ZPAD - 1) * P + (i + XPAD - 1);
   }
+  // Storage column of the x strips' memory variables and coefficients for
+  // grid column i: whole groups of four columns (the points of one thread of
+  // the vector kernels) on both sides, so that a thread moves its cells as
+  // one float4.
+  __host__ __device__ __forceinline__ int xcol(int i) const { return i - 1 < WL ? i - 1 : WL + (i - 1 - xr); }
 };
 
 struct Args {
@@ -85,6 +91,8 @@ struct Args {
   const float* lam; const float* mu; const float* dtr_i; const float* dtr_j; const float* mu_ij;
   // C-PML coefficients of each shot: axis x then z, each [a(na), a_h(nh), b(na), b_h(nh)]
   const float* cp; int cps;
+  const float* cx4;  // per shot: [a, b, a_h, b_h] of axis x by storage column (4 W)
+  int tz;            // rows per block of the vector kernels
   // gradient slots (u[it-1] and D(it) of this step), [shot][F]; null when not written
   float* sUx; float* sUz; float* sDx; float* sDz;
 };
@@ -99,12 +107,12 @@ __device__ __forceinline__ float d4(float f1, float f2, float f3, float f4, floa
 // coefficient index k = pos - n + 2 halo + 1); "full": half = true on an array
 // of n-1 points (left pos <= halo+1, right pos >= n-1-halo, k = pos - n + 2 halo + 2).
 // Returns k (1-based, 0 = outside the strips) and the storage column.
-__device__ __forceinline__ int cpml_half(int pos, int n, int halo, int& col) {
+__host__ __device__ __forceinline__ int cpml_half(int pos, int n, int halo, int& col) {
   if (pos <= halo) { col = pos - 1; return pos; }
   if (pos >= n - halo) { const int k = pos - n + 2 * halo + 1; col = k - 1; return k; }
   return 0;
 }
-__device__ __forceinline__ int cpml_full(int pos, int n, int halo, int& col) {
+__host__ __device__ __forceinline__ int cpml_full(int pos, int n, int halo, int& col) {
   if (pos <= halo + 1) { col = pos - 1; return pos; }
   if (pos >= n - 1 - halo) { const int k = pos - n + 2 * halo + 2; col = k; return k; }
   return 0;
@@ -207,7 +215,7 @@ __global__ void __launch_bounds__(BX) k_el_stress(const Args A) {
         else if (g.ft && j == 2) duz = d4(zu1, zu1, zu2, zu3, g.idz);
         else duz = d4(zu0, zu1, zu2, zu3, g.idz);
         float duxc = dux, duzc = duz;
-        if (kE) duxc = cpml_upd(pxE + (long long)(j - 1) * g.W + colE, cx[kE - 1], cx[na + nh + kE - 1], dux);
+        if (kE) duxc = cpml_upd(pxE + (long long)(j - 1) * g.W + g.xcol(i), cx[kE - 1], cx[na + nh + kE - 1], dux);
         int colF = 0;
         const int kF = cpml_full(j, g.nz, g.halo, colF);  // duz/dz (uz has nz-1 points)
         if (kF) duzc = cpml_upd(pzF + (long long)colF * P + (i - 1), cz[kF - 1], cz[na + nh + kF - 1], duz);
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(BX) k_el_stress(const Args A) {
       const float dzx = d4(uzm1, zu2, uzp1, uzp2, g.idx);
       const float dxz = (g.ft && j == 1) ? d4(xu2, xu1, xu2, xu3, g.idz) : d4(xu0, xu1, xu2, xu3, g.idz);
       float dzxc = dzx, dxzc = dxz;
-      if (kG) dzxc = cpml_upd(pxG + (long long)(j - 1) * g.W + colG, cx[na + kG - 1], cx[2 * na + nh + kG - 1], dzx);
+      if (kG) dzxc = cpml_upd(pxG + (long long)(j - 1) * g.W + g.xcol(i), cx[na + kG - 1], cx[2 * na + nh + kG - 1], dzx);
       int colH = 0;
       const int kH = cpml_half(j, g.nz, g.halo, colH);  // dux/dz (ux has nz points)
       if (kH) dxzc = cpml_upd(pzH + (long long)colH * P + (i - 1), cz[na + kH - 1], cz[2 * na + nh + kH - 1], dxz);
@@ -287,7 +295,7 @@ __global__ void __launch_bounds__(BX) k_el_disp(const Args A) {
       else if (g.ft && j == 2) d2 = d4(-q1, q1, q2, q3, g.idz);
       else d2 = d4(q0, q1, q2, q3, g.idz);
       float d1c = d1, d2c = d2;
-      if (kA) d1c = cpml_upd(pxA + (long long)(j - 1) * g.W + colA, cx[na + kA - 1], cx[2 * na + nh + kA - 1], d1);
+      if (kA) d1c = cpml_upd(pxA + (long long)(j - 1) * g.W + g.xcol(i), cx[na + kA - 1], cx[2 * na + nh + kA - 1], d1);
       int colB = 0;
       const int kB = cpml_full(j, g.nz, g.halo, colB);  // dsxz/dz (sigma_xz has nz-1 points)
       if (kB) d2c = cpml_upd(pzB + (long long)colB * P + (i - 1), cz[kB - 1], cz[na + nh + kB - 1], d2);
@@ -305,7 +313,7 @@ __global__ void __launch_bounds__(BX) k_el_disp(const Args A) {
       const float d1 = d4(qm2, qm1, q2, qp1, g.idx);
       const float d2 = (g.ft && j == 1) ? d4(-w2, w1, w2, w3, g.idz) : d4(w0, w1, w2, w3, g.idz);
       float d1c = d1, d2c = d2;
-      if (kC) d1c = cpml_upd(pxC + (long long)(j - 1) * g.W + colC, cx[kC - 1], cx[na + nh + kC - 1], d1);
+      if (kC) d1c = cpml_upd(pxC + (long long)(j - 1) * g.W + g.xcol(i), cx[kC - 1], cx[na + nh + kC - 1], d1);
       int colD = 0;
       const int kD = cpml_half(j, g.nz, g.halo, colD);  // dszz/dz (sigma_zz has nz points)
       if (kD) d2c = cpml_upd(pzD + (long long)colD * P + (i - 1), cz[na + kD - 1], cz[2 * na + nh + kD - 1], d2);
@@ -356,14 +364,89 @@ __device__ __forceinline__ void st4v(float* p, long long c, const float (&v)[4])
   *reinterpret_cast<float4*>(p + c) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <int TZ>
-__global__ void __launch_bounds__(BX, 6) k_el_stress4(const Args A) {
+// plain (coherent) load for arrays the kernel also writes
+__device__ __forceinline__ F4 ld4p(const float* p, long long c, bool ok) {
+  F4 r;
+  if (ok) {
+    const float4 t = *reinterpret_cast<const float4*>(p + c);
+    r.v[0] = t.x; r.v[1] = t.y; r.v[2] = t.z; r.v[3] = t.w;
+  } else {
+    r.v[0] = r.v[1] = r.v[2] = r.v[3] = 0.0f;
+  }
+  return r;
+}
+
+// d4 with every rounding spelled out (left to the compiler, the products that
+// become part of a fused multiply-add change with the registers and the shape
+// of the code around them, and the results with them): c2 f3 is rounded on its
+// own where ROUND3 is set, everything else is a chain of fused multiply-adds.
+template <bool ROUND3 = false>
+__device__ __forceinline__ float d4r(float f1, float f2, float f3, float f4, float inv) {
+  constexpr float c1 = 1.0f / 24.0f, c2 = 27.0f / 24.0f;
+  const float t = __fmaf_rn(c1, f1, -__fmul_rn(c2, f2));
+  const float u = ROUND3 ? __fadd_rn(t, __fmul_rn(c2, f3)) : __fmaf_rn(c2, f3, t);
+  return __fmul_rn(__fmaf_rn(-c1, f4, u), inv);
+}
+// d4 along x at a thread's four points from the seven values around them; bit
+// e of ROUND3 sets point e's rounding.
+template <unsigned ROUND3>
+__device__ __forceinline__ void d4x(float (&d)[4], const float (&a)[7], float inv) {
+  d[0] = d4r<(ROUND3 & 1) != 0>(a[0], a[1], a[2], a[3], inv);
+  d[1] = d4r<(ROUND3 & 2) != 0>(a[1], a[2], a[3], a[4], inv);
+  d[2] = d4r<(ROUND3 & 4) != 0>(a[2], a[3], a[4], a[5], inv);
+  d[3] = d4r<(ROUND3 & 8) != 0>(a[3], a[4], a[5], a[6], inv);
+}
+// psi = b psi + a dv and dv += psi for the points of `mask` among a thread's
+// four (the cells of the other points hold nothing that is read)
+__device__ __forceinline__ void cpml_upd4(float (&dv)[4], F4& psi, const F4& a, const F4& b, unsigned mask) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float nv = __fmaf_rn(a.v[e], dv[e], __fmul_rn(b.v[e], psi.v[e]));
+    psi.v[e] = nv;
+    if (mask >> e & 1) dv[e] = __fadd_rn(dv[e], nv);
+  }
+}
+__device__ __forceinline__ F4 splat4(float x) { return F4{{x, x, x, x}}; }
+// Which of the thread's four columns i0 .. i0 + 3 hold a memory variable along
+// x: cpml_full on lo .. nx-1 (or nx), cpml_half on 1 .. nx-1.
+__device__ __forceinline__ unsigned xmask_full(const Geo& g, int i0, int lo, int hi) {
+  unsigned m = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = i0 + e;
+    if (i >= lo && i <= hi && (i <= g.halo + 1 || i >= g.nx - 1 - g.halo)) m |= 1u << e;
+  }
+  return m;
+}
+__device__ __forceinline__ unsigned xmask_half(const Geo& g, int i0) {
+  unsigned m = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = i0 + e;
+    if (i <= g.nx - 1 && (i <= g.halo || i >= g.nx - g.halo)) m |= 1u << e;
+  }
+  return m;
+}
+
+// Blocks of 512 points x A.tz rows of one shot, x tiles fastest, then shots,
+// then bands (the shots of a band share the material rows through L2).  The
+// memory variables of a thread's four points are one float4 along either
+// axis, loaded with the rest of the row before anything is computed: point by
+// point they were a chain of four dependent loads per axis and row, which set
+// the time of every row next to a strip (one shot of 333 x 217, 400-step
+// gradient: 94.3 -> 44.7 ms with the same 8-row bands; 8 shots of 1200 x 600, 200
+// steps, gradient: 107.3 -> 82.1 ms).  Bound by HBM latency and bandwidth; 5
+// resident blocks per SM and 6 of the displacement halves: with 6 / 7 the
+// kernels spill (80.2 against 77.3 ms), with 4 / 5 too few rows are in flight
+// (79.4 ms).
+__global__ void __launch_bounds__(BX, 5) k_el_stress4(const Args A) {
   const Geo g = A.g;
-  const int s = blockIdx.z;
+  const int tx = (g.nx + 511) / 512;
+  const int s = blockIdx.x / tx;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wx0 = (blockIdx.x * 4 + warp) * 128;
-  const int j0 = blockIdx.y * TZ + 1;
-  const int j1 = min(j0 + TZ - 1, g.nz - 1);
+  const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
+  const int j0 = blockIdx.y * A.tz + 1;
+  const int j1 = min(j0 + A.tz - 1, g.nz - 1);
   if (j0 > j1 || wx0 >= g.nx) return;  // block / warp uniform
   const int i0 = wx0 + lane * 4 + 1;
   const bool ldok = i0 <= g.nx + 2;
@@ -374,104 +457,119 @@ __global__ void __launch_bounds__(BX, 6) k_el_stress4(const Args A) {
   float* __restrict__ szz = A.szz + so;
   float* __restrict__ sxz = A.sxz + so;
   const int na = 2 * g.halo + 2, nh = 2 * g.halo;
-  const float* cx = A.cp + (long long)s * A.cps;
-  const float* cz = cx + 2 * na + 2 * nh;
+  const float* cz = A.cp + (long long)s * A.cps + 2 * na + 2 * nh;
   const int jlo = g.ft ? 1 : 2;
   const int P = g.P;
-  // x strips touch this thread's points only near the left and right edges
-  const bool xstrip = i0 <= g.halo + 1 || i0 + 3 >= g.nx - 1 - g.halo;
+  const unsigned mE = xmask_full(g, i0, 2, g.nx - 1), mG = xmask_half(g, i0);
+  const bool xs = (mE | mG) != 0;
+  const int sc = xs ? g.xcol(i0) : 0;
+  const float* cx4 = A.cx4 + (long long)s * (4 * g.W) + sc;
+  float* psE = A.px[2] + (long long)s * A.xs + sc;
+  float* psG = A.px[3] + (long long)s * A.xs + sc;
+  float* psF = A.pz[3] + (long long)s * A.zs + (i0 - 1);
+  float* psH = A.pz[2] + (long long)s * A.zs + (i0 - 1);
   const bool xx_all = i0 >= 2 && i0 + 3 <= g.nx - 1;  // all four points are sigma_xx nodes
   const bool xz_all = i0 + 3 <= g.nx - 1;             // all four points are sigma_xz nodes
+  // the edge lanes' own x neighbours (loaded; the others are shuffled)
+  const bool edge = (lane == 0 || lane == 31) && ldok;
+  const int eo1 = lane == 0 ? -1 : 4, eo2 = lane == 0 ? -2 : 5;
   long long c = g.lin(i0, j0);
   F4 xu0 = ld4z(ux, c - P, ldok), xu1 = ld4z(ux, c, ldok), xu2 = ld4z(ux, c + P, ldok), xu3 = ld4z(ux, c + 2 * P, ldok);
   F4 zu0 = ld4z(uz, c - 2 * P, ldok), zu1 = ld4z(uz, c - P, ldok), zu2 = ld4z(uz, c, ldok), zu3 = ld4z(uz, c + P, ldok);
   for (int j = j0; j <= j1; ++j, c += P) {
     const bool more = j + 1 <= j1;
-    F4 xun = ld4z(ux, c + 3 * P, ldok && more);
-    F4 zun = ld4z(uz, c + 2 * P, ldok && more);
-    // ux at i0-2 .. i0+4, uz at i0-1 .. i0+5 (row j)
-    float ua[7], za[7];
-    ua[0] = __shfl_up_sync(FULL, xu1.v[2], 1);
-    ua[1] = __shfl_up_sync(FULL, xu1.v[3], 1);
-    ua[6] = __shfl_down_sync(FULL, xu1.v[0], 1);
-    za[0] = __shfl_up_sync(FULL, zu2.v[3], 1);
-    za[5] = __shfl_down_sync(FULL, zu2.v[0], 1);
-    za[6] = __shfl_down_sync(FULL, zu2.v[1], 1);
-    if (lane == 0) {
-      ua[0] = ldz(ux, c - 2, ldok);
-      ua[1] = ldz(ux, c - 1, ldok);
-      za[0] = ldz(uz, c - 1, ldok);
-    }
-    if (lane == 31) {
-      ua[6] = ldz(ux, c + 4, ldok);
-      za[5] = ldz(uz, c + 4, ldok);
-      za[6] = ldz(uz, c + 5, ldok);
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      ua[2 + e] = xu1.v[e];
-      za[1 + e] = zu2.v[e];
-    }
-    const F4 L4 = ld4z(A.lam, c, ldok), M4 = ld4z(A.mu, c, ldok), MIJ = ld4z(A.mu_ij, c, ldok);
     int colF = 0, colH = 0;
-    const int kF = cpml_full(j, g.nz, g.halo, colF);  // duz/dz at sigma_xx nodes (uz has nz-1 points)
-    const int kH = cpml_half(j, g.nz, g.halo, colH);  // dux/dz at sigma_xz nodes (ux has nz points)
-    float oxx[4], ozz[4], oxz[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = i0 + e;
-      const float l = L4.v[e], m = M4.v[e];
-      const float l2m = l + 2.0f * m;
-      // sigma_xx, sigma_zz
-      const float dux = d4(ua[e], ua[e + 1], ua[e + 2], ua[e + 3], g.idx);
-      float duz;
-      if (g.ft && j == 1) duz = (-l / l2m) * dux;
-      else if (g.ft && j == 2) duz = d4(zu1.v[e], zu1.v[e], zu2.v[e], zu3.v[e], g.idz);
-      else duz = d4(zu0.v[e], zu1.v[e], zu2.v[e], zu3.v[e], g.idz);
-      const bool xx = i >= 2 && i <= g.nx - 1 && j >= jlo;
-      float duxc = dux, duzc = duz;
-      if (xstrip && xx) {
-        int colE = 0;
-        const int kE = cpml_full(i, g.nx, g.halo, colE);
-        if (kE) duxc = cpml_upd(A.px[2] + (long long)s * A.xs + (long long)(j - 1) * g.W + colE, cx[kE - 1],
-                                cx[na + nh + kE - 1], dux);
+    const int kF = j >= jlo ? cpml_full(j, g.nz, g.halo, colF) : 0;  // duz/dz at sigma_xx nodes (uz has nz-1 points)
+    const int kH = cpml_half(j, g.nz, g.halo, colH);                 // dux/dz at sigma_xz nodes (ux has nz points)
+    const float eu1 = ldz(ux, c + eo1, edge), eu2 = ldz(ux, c - 2, edge && lane == 0);
+    const float ez1 = ldz(uz, c + eo1, edge), ez2 = ldz(uz, c + eo2, edge && lane == 31);
+    F4 E4, G4, F4v, H4;
+    const bool xe = mE && j >= jlo, zf = kF && ldok, zh = kH && ldok;
+    if (xe) E4 = ld4rwz(psE, (long long)(j - 1) * g.W);
+    if (mG) G4 = ld4rwz(psG, (long long)(j - 1) * g.W);
+    if (zf) F4v = ld4rwz(psF, (long long)colF * P);
+    if (zh) H4 = ld4rwz(psH, (long long)colH * P);
+    const F4 L4 = ld4z(A.lam, c, ldok), M4 = ld4z(A.mu, c, ldok), MIJ = ld4z(A.mu_ij, c, ldok);
+    const F4 xun = ld4z(ux, c + 3 * P, ldok && more);
+    const F4 zun = ld4z(uz, c + 2 * P, ldok && more);
+    float d1[4], d2[4];
+    {  // sigma_xx, sigma_zz; ux at i0-2 .. i0+4 (row j)
+      float ua[7];
+      ua[0] = __shfl_up_sync(FULL, xu1.v[2], 1);
+      ua[1] = __shfl_up_sync(FULL, xu1.v[3], 1);
+      ua[6] = __shfl_down_sync(FULL, xu1.v[0], 1);
+      if (lane == 0) {
+        ua[0] = eu2;
+        ua[1] = eu1;
       }
-      if (kF && xx)
-        duzc = cpml_upd(A.pz[3] + (long long)s * A.zs + (long long)colF * P + (i - 1), cz[kF - 1],
-                        cz[na + nh + kF - 1], duz);
-      oxx[e] = l2m * duxc + l * duzc;
-      ozz[e] = (j == 1) ? 0.0f : l * duxc + l2m * duzc;
-      // sigma_xz
-      const float dzx = d4(za[e], za[e + 1], za[e + 2], za[e + 3], g.idx);
-      const float dxz = (g.ft && j == 1) ? d4(xu2.v[e], xu1.v[e], xu2.v[e], xu3.v[e], g.idz)
-                                         : d4(xu0.v[e], xu1.v[e], xu2.v[e], xu3.v[e], g.idz);
-      const bool xz = i <= g.nx - 1;
-      float dzxc = dzx, dxzc = dxz;
-      if (xstrip && xz) {
-        int colG = 0;
-        const int kG = cpml_half(i, g.nx, g.halo, colG);
-        if (kG) dzxc = cpml_upd(A.px[3] + (long long)s * A.xs + (long long)(j - 1) * g.W + colG, cx[na + kG - 1],
-                                cx[2 * na + nh + kG - 1], dzx);
-      }
-      if (kH && xz)
-        dxzc = cpml_upd(A.pz[2] + (long long)s * A.zs + (long long)colH * P + (i - 1), cz[na + kH - 1],
-                        cz[2 * na + nh + kH - 1], dxz);
-      oxz[e] = MIJ.v[e] * (dzxc + dxzc);
-    }
-    if (ldok) {
-      if (xx_all && j >= jlo) {
-        st4v(sxx, c, oxx);
-        st4v(szz, c, ozz);
-      } else {
+      if (lane == 31) ua[6] = eu1;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = i0 + e;
-          if (i >= 2 && i <= g.nx - 1 && j >= jlo) {
-            sxx[c + e] = oxx[e];
-            szz[c + e] = ozz[e];
+      for (int e = 0; e < 4; ++e) ua[2 + e] = xu1.v[e];
+      d4x<0u>(d1, ua, g.idx);
+      const bool fs1 = g.ft && j == 1, fs2 = g.ft && j == 2;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (fs1) d2[e] = __fmul_rn(-L4.v[e] / __fmaf_rn(2.0f, M4.v[e], L4.v[e]), d1[e]);
+        else d2[e] = d4r(fs2 ? zu1.v[e] : zu0.v[e], zu1.v[e], zu2.v[e], zu3.v[e], g.idz);
+      }
+      if (xe) {
+        cpml_upd4(d1, E4, ld4z(cx4, 0, true), ld4z(cx4, g.W, true), mE);
+        st4v(psE, (long long)(j - 1) * g.W, E4.v);
+      }
+      if (zf) {
+        cpml_upd4(d2, F4v, splat4(cz[kF - 1]), splat4(cz[na + nh + kF - 1]), 15u);
+        st4v(psF, (long long)colF * P, F4v.v);
+      }
+      float oxx[4], ozz[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float l = L4.v[e], l2m = __fmaf_rn(2.0f, M4.v[e], l);
+        oxx[e] = __fmaf_rn(l2m, d1[e], __fmul_rn(l, d2[e]));
+        ozz[e] = j == 1 ? 0.0f : __fmaf_rn(l, d1[e], __fmul_rn(l2m, d2[e]));
+      }
+      if (j >= jlo) {
+        if (xx_all) {
+          st4v(sxx, c, oxx);
+          st4v(szz, c, ozz);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = i0 + e;
+            if (i >= 2 && i <= g.nx - 1) {
+              sxx[c + e] = oxx[e];
+              szz[c + e] = ozz[e];
+            }
           }
         }
       }
+    }
+    {  // sigma_xz; uz at i0-1 .. i0+5 (row j)
+      float za[7];
+      za[0] = __shfl_up_sync(FULL, zu2.v[3], 1);
+      za[5] = __shfl_down_sync(FULL, zu2.v[0], 1);
+      za[6] = __shfl_down_sync(FULL, zu2.v[1], 1);
+      if (lane == 0) za[0] = ez1;
+      if (lane == 31) {
+        za[5] = ez1;
+        za[6] = ez2;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) za[1 + e] = zu2.v[e];
+      d4x<0u>(d1, za, g.idx);
+      const bool fs1 = g.ft && j == 1;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) d2[e] = d4r(fs1 ? xu2.v[e] : xu0.v[e], xu1.v[e], xu2.v[e], xu3.v[e], g.idz);
+      if (mG) {
+        cpml_upd4(d1, G4, ld4z(cx4, 2 * g.W, true), ld4z(cx4, 3 * g.W, true), mG);
+        st4v(psG, (long long)(j - 1) * g.W, G4.v);
+      }
+      if (zh) {
+        cpml_upd4(d2, H4, splat4(cz[na + kH - 1]), splat4(cz[2 * na + nh + kH - 1]), 15u);
+        st4v(psH, (long long)colH * P, H4.v);
+      }
+      float oxz[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) oxz[e] = __fmul_rn(MIJ.v[e], __fadd_rn(d1[e], d2[e]));
       if (xz_all) {
         st4v(sxz, c, oxz);
       } else {
@@ -490,16 +588,17 @@ __global__ void __launch_bounds__(BX, 6) k_el_stress4(const Args A) {
 // half no sigma_zz)
 template <int COMP>
 struct ElDispBounds {
-  static constexpr int MINB = COMP == 2 ? 5 : 7;
+  static constexpr int MINB = COMP == 2 ? 5 : 6;
 };
-template <int TZ, int COMP = 2>
+template <int COMP>
 __global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const Args A) {
   const Geo g = A.g;
-  const int s = blockIdx.z;
+  const int tx = (g.nx + 511) / 512;
+  const int s = blockIdx.x / tx;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wx0 = (blockIdx.x * 4 + warp) * 128;
-  const int j0 = blockIdx.y * TZ + 1;
-  const int j1 = min(j0 + TZ - 1, g.nz);
+  const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
+  const int j0 = blockIdx.y * A.tz + 1;
+  const int j1 = min(j0 + A.tz - 1, g.nz);
   if (j0 > j1 || wx0 >= g.nx) return;
   const int i0 = wx0 + lane * 4 + 1;
   const bool ldok = i0 <= g.nx + 2;
@@ -512,14 +611,21 @@ __global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const
   const float* __restrict__ szz = A.szz + so;
   const float* __restrict__ sxz = A.sxz + so;
   const int na = 2 * g.halo + 2, nh = 2 * g.halo;
-  const float* cx = A.cp + (long long)s * A.cps;
-  const float* cz = cx + 2 * na + 2 * nh;
+  const float* cz = A.cp + (long long)s * A.cps + 2 * na + 2 * nh;
   const bool slots = A.sUx != nullptr;
   const int P = g.P;
-  const bool xstrip = i0 <= g.halo + 1 || i0 + 3 >= g.nx - 1 - g.halo;
+  constexpr bool DOX = COMP != 1, DOZ = COMP != 0;
+  const unsigned mA = DOX ? xmask_half(g, i0) : 0u, mC = DOZ ? xmask_full(g, i0, 1, g.nx) : 0u;
+  const int sc = (mA | mC) ? g.xcol(i0) : 0;
+  const float* cx4 = A.cx4 + (long long)s * (4 * g.W) + sc;
+  float* psA = A.px[0] + (long long)s * A.xs + sc;
+  float* psC = A.px[1] + (long long)s * A.xs + sc;
+  float* psD = A.pz[0] + (long long)s * A.zs + (i0 - 1);
+  float* psB = A.pz[1] + (long long)s * A.zs + (i0 - 1);
   const bool ux_all = i0 + 3 <= g.nx - 1;  // all four points are ux nodes
   const bool uz_all = i0 + 3 <= g.nx;      // all four points are uz nodes
-  constexpr bool DOX = COMP != 1, DOZ = COMP != 0;
+  const bool edge = (lane == 0 || lane == 31) && ldok;
+  const int eo1 = lane == 0 ? -1 : 4;
   long long c = g.lin(i0, j0);
   F4 q0{}, q1{}, q3{}, w0{}, w1{}, w2{}, w3{}, xc{};
   if (DOX) {
@@ -537,7 +643,30 @@ __global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const
   }
   for (int j = j0; j <= j1; ++j, c += P) {
     const bool more = j + 1 <= j1;
-    F4 qn{}, wn{}, xcn{};
+    const bool zrow = j <= g.nz - 1;
+    int colB = 0, colD = 0;
+    const int kB = DOX ? cpml_full(j, g.nz, g.halo, colB) : 0;           // dsxz/dz at ux nodes (sigma_xz has nz-1 points)
+    const int kD = DOZ && zrow ? cpml_half(j, g.nz, g.halo, colD) : 0;  // dszz/dz at uz nodes (sigma_zz has nz points)
+    F4 qn{}, wn{}, xcn{}, A4, B4, C4, D4, R, U, DU, Rj, V, DV;
+    float ex1 = 0.f, ex2 = 0.f, eq1 = 0.f, eq2 = 0.f;
+    if (DOX) {
+      ex1 = ldz(sxx, c + eo1, edge);
+      ex2 = ldz(sxx, c + 5, edge && lane == 31);
+      R = ld4z(A.dtr_i, c, ldok);
+      U = ld4p(ux, c, ldok);
+      DU = ld4p(dux, c, ldok);
+      if (mA) A4 = ld4rwz(psA, (long long)(j - 1) * g.W);
+      if (kB && ldok) B4 = ld4rwz(psB, (long long)colB * P);
+    }
+    if (DOZ) {
+      eq1 = ldz(sxz, c + eo1, edge);
+      eq2 = ldz(sxz, c - 2, edge && lane == 0);
+      Rj = ld4z(A.dtr_j, c, ldok && zrow);
+      V = ld4p(uz, c, ldok && zrow);
+      DV = ld4p(duz, c, ldok && zrow);
+      if (mC && zrow) C4 = ld4rwz(psC, (long long)(j - 1) * g.W);
+      if (kD && ldok) D4 = ld4rwz(psD, (long long)colD * P);
+    }
     if (DOX) {
       qn = ld4z(sxz, c + 2 * P, ldok && more);
       xcn = ld4z(sxx, c + P, ldok && more);
@@ -545,62 +674,40 @@ __global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const
       qn = ld4z(sxz, c + P, ldok && more);  // only row j+1 (next q2)
     }
     if (DOZ) wn = ld4z(szz, c + 3 * P, ldok && more);
-    // sigma_xx at i0-1 .. i0+5, sigma_xz at i0-2 .. i0+4 (row j)
-    float xa[7], qa[7];
-    if (DOX) {
+    float d1[4], d2[4];
+    if (DOX) {  // ux nodes; sigma_xx at i0-1 .. i0+5 (row j)
+      float xa[7];
       xa[0] = __shfl_up_sync(FULL, xc.v[3], 1);
       xa[5] = __shfl_down_sync(FULL, xc.v[0], 1);
       xa[6] = __shfl_down_sync(FULL, xc.v[1], 1);
-      if (lane == 0) xa[0] = ldz(sxx, c - 1, ldok);
+      if (lane == 0) xa[0] = ex1;
       if (lane == 31) {
-        xa[5] = ldz(sxx, c + 4, ldok);
-        xa[6] = ldz(sxx, c + 5, ldok);
+        xa[5] = ex1;
+        xa[6] = ex2;
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) xa[1 + e] = xc.v[e];
-    }
-    if (DOZ) {
-      qa[0] = __shfl_up_sync(FULL, q2.v[2], 1);
-      qa[1] = __shfl_up_sync(FULL, q2.v[3], 1);
-      qa[6] = __shfl_down_sync(FULL, q2.v[0], 1);
-      if (lane == 0) {
-        qa[0] = ldz(sxz, c - 2, ldok);
-        qa[1] = ldz(sxz, c - 1, ldok);
-      }
-      if (lane == 31) qa[6] = ldz(sxz, c + 4, ldok);
+      d4x<2u>(d1, xa, g.idx);
+      const bool fs1 = g.ft && j == 1, fs2 = g.ft && j == 2;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) qa[2 + e] = q2.v[e];
-    }
-    int colB = 0, colD = 0;
-    const int kB = cpml_full(j, g.nz, g.halo, colB);  // dsxz/dz at ux nodes (sigma_xz has nz-1 points)
-    const int kD = cpml_half(j, g.nz, g.halo, colD);  // dszz/dz at uz nodes (sigma_zz has nz points)
-    if (ldok && DOX) {
-      // ux nodes
-      const F4 R = ld4z(A.dtr_i, c, true);
-      F4 U = ld4rwz(ux, c), DU = ld4rwz(dux, c);
+      for (int e = 0; e < 4; ++e) {
+        const float f1 = fs1 ? -q3.v[e] : fs2 ? -q1.v[e] : q0.v[e], f2 = fs1 ? -q2.v[e] : q1.v[e];
+        d2[e] = d4r(f1, f2, q2.v[e], q3.v[e], g.idz);
+      }
+      if (mA) {
+        cpml_upd4(d1, A4, ld4z(cx4, 2 * g.W, true), ld4z(cx4, 3 * g.W, true), mA);
+        st4v(psA, (long long)(j - 1) * g.W, A4.v);
+      }
+      if (kB && ldok) {
+        cpml_upd4(d2, B4, splat4(cz[kB - 1]), splat4(cz[na + nh + kB - 1]), 15u);
+        st4v(psB, (long long)colB * P, B4.v);
+      }
       float nu[4], ndu[4], Dv[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int i = i0 + e;
-        const float d1 = d4(xa[e], xa[e + 1], xa[e + 2], xa[e + 3], g.idx);
-        float d2;
-        if (g.ft && j == 1) d2 = d4(-q3.v[e], -q2.v[e], q2.v[e], q3.v[e], g.idz);
-        else if (g.ft && j == 2) d2 = d4(-q1.v[e], q1.v[e], q2.v[e], q3.v[e], g.idz);
-        else d2 = d4(q0.v[e], q1.v[e], q2.v[e], q3.v[e], g.idz);
-        const bool on = i <= g.nx - 1;
-        float d1c = d1, d2c = d2;
-        if (xstrip && on) {
-          int colA = 0;
-          const int kA = cpml_half(i, g.nx, g.halo, colA);
-          if (kA) d1c = cpml_upd(A.px[0] + (long long)s * A.xs + (long long)(j - 1) * g.W + colA, cx[na + kA - 1],
-                                 cx[2 * na + nh + kA - 1], d1);
-        }
-        if (kB && on)
-          d2c = cpml_upd(A.pz[1] + (long long)s * A.zs + (long long)colB * P + (i - 1), cz[kB - 1],
-                         cz[na + nh + kB - 1], d2);
-        Dv[e] = R.v[e] * (d1c + d2c);
-        ndu[e] = DU.v[e] + Dv[e];
-        nu[e] = U.v[e] + ndu[e];
+        Dv[e] = __fmul_rn(R.v[e], __fadd_rn(d1[e], d2[e]));
+        ndu[e] = __fadd_rn(DU.v[e], Dv[e]);
+        nu[e] = __fadd_rn(U.v[e], ndu[e]);
       }
       if (ux_all) {
         if (slots) {
@@ -622,32 +729,37 @@ __global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const
           }
       }
     }
-    if (ldok && DOZ) {
-      // uz nodes
-      if (j <= g.nz - 1) {
-        const F4 Rj = ld4z(A.dtr_j, c, true);
-        F4 V = ld4rwz(uz, c), DV = ld4rwz(duz, c);
+    if (DOZ) {  // uz nodes; sigma_xz at i0-2 .. i0+4 (row j)
+      float qa[7];
+      qa[0] = __shfl_up_sync(FULL, q2.v[2], 1);
+      qa[1] = __shfl_up_sync(FULL, q2.v[3], 1);
+      qa[6] = __shfl_down_sync(FULL, q2.v[0], 1);
+      if (zrow) {
+        if (lane == 0) {
+          qa[0] = eq2;
+          qa[1] = eq1;
+        }
+        if (lane == 31) qa[6] = eq1;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) qa[2 + e] = q2.v[e];
+        d4x<2u>(d1, qa, g.idx);
+        const bool fs1 = g.ft && j == 1;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d2[e] = d4r(fs1 ? -w2.v[e] : w0.v[e], w1.v[e], w2.v[e], w3.v[e], g.idz);
+        if (mC) {
+          cpml_upd4(d1, C4, ld4z(cx4, 0, true), ld4z(cx4, g.W, true), mC);
+          st4v(psC, (long long)(j - 1) * g.W, C4.v);
+        }
+        if (kD && ldok) {
+          cpml_upd4(d2, D4, splat4(cz[na + kD - 1]), splat4(cz[2 * na + nh + kD - 1]), 15u);
+          st4v(psD, (long long)colD * P, D4.v);
+        }
         float nv[4], ndv[4], Dz[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int i = i0 + e;
-          const float d1 = d4(qa[e], qa[e + 1], qa[e + 2], qa[e + 3], g.idx);
-          const float d2 = (g.ft && j == 1) ? d4(-w2.v[e], w1.v[e], w2.v[e], w3.v[e], g.idz)
-                                            : d4(w0.v[e], w1.v[e], w2.v[e], w3.v[e], g.idz);
-          const bool on = i <= g.nx;
-          float d1c = d1, d2c = d2;
-          if (xstrip && on) {
-            int colC = 0;
-            const int kC = cpml_full(i, g.nx, g.halo, colC);
-            if (kC) d1c = cpml_upd(A.px[1] + (long long)s * A.xs + (long long)(j - 1) * g.W + colC, cx[kC - 1],
-                                   cx[na + nh + kC - 1], d1);
-          }
-          if (kD && on)
-            d2c = cpml_upd(A.pz[0] + (long long)s * A.zs + (long long)colD * P + (i - 1), cz[na + kD - 1],
-                           cz[2 * na + nh + kD - 1], d2);
-          Dz[e] = Rj.v[e] * (d1c + d2c);
-          ndv[e] = DV.v[e] + Dz[e];
-          nv[e] = V.v[e] + ndv[e];
+          Dz[e] = __fmul_rn(Rj.v[e], __fadd_rn(d1[e], d2[e]));
+          ndv[e] = __fadd_rn(DV.v[e], Dz[e]);
+          nv[e] = __fadd_rn(V.v[e], ndv[e]);
         }
         if (uz_all) {
           if (slots) {
@@ -1266,13 +1378,13 @@ struct sw_elastic {
   DevMem ck;                       // [M][4][cap][F] then [M][8][cap][strip]
   DevMem acc;                      // [groups][10][F]
   // tables
-  DevMem d_desc, d_ll, d_int, d_flt, d_tf, d_tr, d_obs, d_ic, d_mask, d_adj, d_mt, d_cp;
+  DevMem d_desc, d_ll, d_int, d_flt, d_tf, d_tr, d_obs, d_ic, d_mask, d_adj, d_mt, d_cp, d_cx4;
   DevMem d_partial, d_amax, d_balls, d_ball_ptr, d_cs;
   DevMem d_icd, d_dres;  // dense inverse covariances; residuals and C^-1 r of those shots
   DevMem d_snap;                     // snapshot stage (one block per shot)
   int snapevery = 0;                 // snapshots requested by the current forward call
   float* const* snap_out = nullptr;  // per caller shot: nt/snapevery blocks [ux, uz, sxx, szz, sxz]
-  int tz = 8;  // rows per block of the stencil kernels (8, 16 or 32; 8 measured fastest)
+  int tz = 0;  // rows per block of the stencil kernels (0: band_rows; 8, 16 or 32)
   bool vec = true;  // four x points per thread (k_el_*4) instead of one
   bool split_disp = true;  // the displacement update as two launches, ux then uz (tz + 128: one launch)
   DevMem d_scales;        // [0] the forward sources' common scale, [1] the adjoint source's scale
@@ -1645,6 +1757,28 @@ void build_tables(sw_elastic* es, const sw_elastic_shot* shots, const std::vecto
     std::copy(s.cpml, s.cpml + es->cps, cps.begin() + (size_t)k * es->cps);
   }
   upload(es, es->d_cp, cps, "C-PML coefficients");
+  {  // axis x by storage column: [a, b] of the full maps, [a_h, b_h] of the half maps
+    const Geo& g = es->g;
+    std::vector<float> cx4((size_t)S * 4 * g.W, 0.0f);
+    const int na = 2 * g.halo + 2, nh = 2 * g.halo;
+    for (int k = 0; k < S; ++k) {
+      const float* cx = &cps[(size_t)k * es->cps];
+      float* o = &cx4[(size_t)k * 4 * g.W];
+      for (int i = 1; i <= g.nx; ++i) {
+        int col = 0;
+        const int kf = cpml_full(i, g.nx, g.halo, col), kh = cpml_half(i, g.nx, g.halo, col);
+        if (kf) {
+          o[g.xcol(i)] = cx[kf - 1];
+          o[g.W + g.xcol(i)] = cx[na + nh + kf - 1];
+        }
+        if (kh && i <= g.nx - 1) {
+          o[2 * g.W + g.xcol(i)] = cx[na + kh - 1];
+          o[3 * g.W + g.xcol(i)] = cx[2 * na + nh + kh - 1];
+        }
+      }
+    }
+    upload(es, es->d_cx4, cx4, "C-PML coefficients by column");
+  }
   check_cuda(cudaMemsetAsync(es->d_tr.p, 0, (size_t)tr_total * sizeof(float), st), "traces clear");
   const long long* LL = es->d_ll.as<long long>();
   const int* IN = es->d_int.as<int>();
@@ -1774,6 +1908,7 @@ struct Run {
     a.dtr_i = es->dtr_i.as<float>(); a.dtr_j = es->dtr_j.as<float>(); a.mu_ij = es->mu_ij.as<float>();
     a.cp = es->d_cp.as<float>();
     a.cps = es->cps;
+    a.cx4 = es->d_cx4.as<float>();
     return a;
   }
   // algorithmic bytes of one step (stress + displacement kernels): per point and
@@ -1829,34 +1964,53 @@ void zero_state(sw_elastic* es, int S, bool adjoint) {
   }
 }
 
+// Rows per block of the vector kernels.  A warp's rows run one after the other
+// and a band re-reads the 3 rows of its z windows: 4 rows are fastest where
+// the launch fills the GPU (8 x 1200 x 600 gradient: 79.3 ms with 2 rows, 77.3
+// with 4, 79.7 with 8); a launch of fewer than 16 warps per SM takes shorter
+// bands (one shot of 333 x 217, gradient: 41.1 ms with 8 rows, 28.4 with 4,
+// 18.7 with 1).
+int band_rows(const sw_elastic* es, int S) {
+  if (es->tz > 0) return es->tz;
+  const int sms = es->ctx->num_sms > 0 ? es->ctx->num_sms : 148;
+  const long long wx = (es->g.nx + 127) / 128;
+  int tz = 4;
+  while (tz > 1 && S * wx * ((es->g.nz + tz - 1) / tz) < 16LL * sms) tz /= 2;
+  return tz;
+}
+
+// the one-point kernels (set_tuning + 64)
 template <int TZ>
+void launch_scalar(const sw_elastic* es, cudaStream_t st, const Args& a, int S, bool stress) {
+  const dim3 grid((es->g.nx + BX - 1) / BX, (es->g.nz + TZ - 1) / TZ, S);
+  if (stress) k_el_stress<TZ><<<grid, BX, 0, st>>>(a);
+  else k_el_disp<TZ><<<grid, BX, 0, st>>>(a);
+}
+
 // returns the number of kernels launched
-int launch_stencil_tz(const sw_elastic* es, cudaStream_t st, const Args& a, int S, bool stress) {
+int launch_stencil(const sw_elastic* es, cudaStream_t st, Args a, int S, bool stress) {
   int nk = 1;
   if (es->vec) {  // four points per thread: 512 per block
-    const dim3 grid((es->g.nx + 511) / 512, (es->g.nz + TZ - 1) / TZ, S);
+    a.tz = band_rows(es, S);
+    const dim3 grid((unsigned)((es->g.nx + 511) / 512 * S), (unsigned)((es->g.nz + a.tz - 1) / a.tz));
     if (stress) {
-      k_el_stress4<TZ><<<grid, BX, 0, st>>>(a);
+      k_el_stress4<<<grid, BX, 0, st>>>(a);
     } else if (es->split_disp) {  // ux and uz updates as two launches
-      k_el_disp4<TZ, 0><<<grid, BX, 0, st>>>(a);
-      k_el_disp4<TZ, 1><<<grid, BX, 0, st>>>(a);
+      k_el_disp4<0><<<grid, BX, 0, st>>>(a);
+      k_el_disp4<1><<<grid, BX, 0, st>>>(a);
       nk = 2;
     } else {
-      k_el_disp4<TZ><<<grid, BX, 0, st>>>(a);
+      k_el_disp4<2><<<grid, BX, 0, st>>>(a);
     }
+  } else if (es->tz == 16) {
+    launch_scalar<16>(es, st, a, S, stress);
+  } else if (es->tz == 32) {
+    launch_scalar<32>(es, st, a, S, stress);
   } else {
-    const dim3 grid((es->g.nx + BX - 1) / BX, (es->g.nz + TZ - 1) / TZ, S);
-    if (stress) k_el_stress<TZ><<<grid, BX, 0, st>>>(a);
-    else k_el_disp<TZ><<<grid, BX, 0, st>>>(a);
+    launch_scalar<8>(es, st, a, S, stress);
   }
   check_cuda(cudaGetLastError(), stress ? "stress launch" : "displacement launch");
   return nk;
-}
-
-int launch_stencil(const sw_elastic* es, cudaStream_t st, const Args& a, int S, bool stress) {
-  if (es->tz == 16) return launch_stencil_tz<16>(es, st, a, S, stress);
-  if (es->tz == 32) return launch_stencil_tz<32>(es, st, a, S, stress);
-  return launch_stencil_tz<8>(es, st, a, S, stress);
 }
 
 // stress, [sigma sources], displacement, [force sources], [recording]
@@ -2014,7 +2168,9 @@ void elastic_init(sw_elastic* es, sw_ctx* ctx, const sw_elastic_params* p, int g
   g.ft = p->freetop ? 1 : 0;
   g.P = (int)round_up(g.nx + XPAD + 8, 32);  // the vector kernels read up to column nx + 36
   g.F = (long long)g.P * (g.nz + 2 * ZPAD);
-  g.W = (int)round_up(2 * g.halo + 3, 4);
+  g.WL = (int)round_up(g.halo + 1, 4);
+  g.xr = std::max(g.WL, (g.nx - 2 - g.halo) / 4 * 4);
+  g.W = g.WL + std::max((int)round_up(g.nx, 4) - g.xr, 0);
   g.idx = (float)(1.0 / p->h[0]);
   g.idz = (float)(1.0 / p->h[1]);
   es->na = 2 * g.halo + 2;
@@ -2421,12 +2577,12 @@ void elastic_gradient(sw_elastic* es, int nshots, const sw_elastic_shot* shots, 
 }
 
 void elastic_set_tuning(sw_elastic* es, int tz) {
-  // tz = rows per block (8, 16, 32; 0 = 8); + 64 selects the one-point-per-thread kernels;
+  // tz = rows per block (8, 16, 32; 0 = band_rows); + 64 selects the one-point-per-thread kernels;
   // + 128 runs the four-point displacement update as one launch instead of two (ux, uz)
   const int rows = tz % 64;
   if (tz < 0 || tz >= 256 || (rows != 0 && rows != 8 && rows != 16 && rows != 32))
     fail(SW_ERR_ARG, "tz must be 0, 8, 16 or 32, optionally + 64 and + 128");
-  es->tz = rows == 0 ? 8 : rows;
+  es->tz = rows;
   es->vec = (tz & 64) == 0;
   es->split_disp = (tz & 128) == 0;
 }

@@ -1,10 +1,11 @@
-"""The x strips' memory variables of the variable-density kernels move in whole
+"""The x strips' memory variables of the variable-density and elastic kernels move in whole
 groups of four columns: grids whose strips end inside a group, meet in one
 group (nx = 2 halo + 3), or leave a partial last group, and band heights from
 one row (the default on small grids) to more rows than the grid has."""
 import numpy as np
 import pytest
 
+import elastic_cases as E
 import vd_cases as V
 from vd_cases import rel_l2, sw
 
@@ -42,3 +43,24 @@ def test_vd_groups_and_bands(ctx, nx, nz, halo, freetop):
     assert rel_l2(out[0][2], tref) < TOL
     assert rel_l2(out[0][0], gref["vp"]) < TOL and rel_l2(out[0][1], gref["rho"]) < TOL
     assert _same(out[8], out[0]) and _same(out[32], out[0])
+
+
+@pytest.mark.parametrize("nx,nz,halo", GRIDS)
+@pytest.mark.parametrize("kind,freetop", [("mt", False), ("force", True)])
+def test_elastic_groups_and_bands(ctx, nx, nz, halo, kind, freetop):
+    case = E.small_case(kind, nt=160, nx=nx, nz=nz, halo=halo, freetop=freetop)
+    shot = case.shots[0]
+    obs = 0.5 * E.oracle_forward(case, shot).astype(np.float32).astype(np.float64)
+    gref, _, tref = E.oracle_gradient(case, shot, obs, check_freq=7)
+    out = {}
+    for tz in (0, 8, 32, 128):
+        run = E.GpuElastic(ctx, case, gradient=True, check_freq=7)
+        ctx.check(ctx.lib.sw_elastic_set_tuning(run.h, tz), "set_tuning")
+        g, m, t = run.gradient([shot], [obs])
+        run.close()
+        out[tz] = [g["rho"], g["lambda"], g["mu"], t[0], np.array(m)]
+    assert rel_l2(out[0][3], tref) < TOL
+    for q, k in enumerate(("rho", "lambda", "mu")):
+        assert rel_l2(out[0][q], gref[k]) < TOL, k
+    for tz in (8, 32, 128):
+        assert _same(out[tz], out[0]), tz
