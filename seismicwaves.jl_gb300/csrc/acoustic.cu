@@ -529,7 +529,6 @@ struct sw_wavesim {
                                           // receiver -> stash index, first-step pressure of receiver rows
   bool pair_on = false;                   // 2D: two time steps per launch where possible (tuning variant)
   bool split3d = true;                    // 3D: inner rows and strip rows as two launches (variant bit 16: one)
-  bool inner_np = false;                  // 3D: the three launches without the software pipeline (variant bit 17)
   bool xsplit = true;                     // 2D 4-warp stencil: x strips as extra blocks (variant bit 18: not)
   int pair_tz = 0;                        // rows per block of the two-step kernel (0 = heuristic)
   int pair_occ = 0;                       // resident-block bound of the two-step kernel (0 = default, 1, 2)
@@ -652,7 +651,7 @@ std::vector<long long> group_key(const sw_wavesim* ws, const std::vector<HostSho
   std::vector<long long> k = {grad ? 1 : 0, ws->grp, ws->variant, ws->tile_tz, ws->pf, ws->adjw ? 1 : 0,
                               ws->cpa ? 1 : 0, ws->pair_ok ? 1 : 0, ws->pair_adj_ok ? 1 : 0, ws->pair_tz,
                               ws->pair_occ, ws->kind_tz[0], ws->kind_tz[1], ws->kind_tz[2], ws->precision,
-                              ws->split3d ? 1 : 0, ws->inner_np ? 1 : 0, ws->xsplit ? 1 : 0,
+                              ws->split3d ? 1 : 0, ws->xsplit ? 1 : 0,
                               (long long)group.size()};
   for (const auto& h : group) k.push_back(h.nt);
   return k;
@@ -1169,9 +1168,21 @@ StepCtx make_step_ctx(sw_wavesim* ws, int S, int kind = TZ_FORWARD) {
     if (ws->N == 2 && (ws->variant & 3) != 1) {
       // register-pipelined 2D stencil: short bands keep every SM at full
       // occupancy with a negligible tail (8 rows measured best on GB300 for
-      // 64 shots of 2001 x 801: 55.6 Gpts/s against 48.4 at 64 rows); small
-      // batches take 4-row bands to fill the GPU
-      TZ = (long long)S * c.tiles_x * ((nint + 7) / 8) < 4LL * sms ? 4 : 8;
+      // 64 shots of 2001 x 801: 55.6 Gpts/s against 48.4 at 64 rows).  A
+      // warp's rows run one after the other, so smaller launches take
+      // shorter bands: 4 rows below 256 warps per SM (16 shots of 2001 x 801,
+      // gradient: 109.8 against 111.1 ms; one of 801 x 801: 35.2 against 43.6
+      // with 8 and 37.2 with 2), 2 below 8 (one of 201 x 201: 8.5 us per step
+      // against 9.2 with 4 and 12.8 with 8; single rows run 8.6)
+      const long long wx = (ws->P + 127) / 128;
+      TZ = 8;
+      if (S * wx * ((nint + 7) / 8) < 256LL * sms) TZ = 4;
+      if (S * wx * ((nint + 3) / 4) < 8LL * sms) TZ = 2;
+    } else if (ws->N == 3 && ws->split3d) {
+      // 16 planes, 8 or 4 while the inner rows make fewer than 8 blocks per SM
+      // (2 x 183 x 157 x 141: 35.2 ms per 300 steps with 16 planes, 45 with 32)
+      TZ = 16;
+      while (TZ > 4 && (long long)S * c.tiles_x * c.tiles_y * ((nint + TZ - 1) / TZ) < 8LL * sms) TZ /= 2;
     } else {
       // aim for >= ~8 blocks per SM in total, with TZ in [tz_min, 64]
       TZ = 64;
@@ -1459,38 +1470,24 @@ struct Launcher {
       a1.tiles_y = sp.tiles_y1;
       a1.tiles_z = sp.tiles_z1;
       const long long b1 = (long long)a.nshots * c.tiles_x * sp.tiles_y1 * sp.tiles_z1;
-      // the slabs are thin: shorter bands while a slab launch would fill less
-      // than two waves of 4 blocks per SM (small batches), 4 rows at least
-      const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
-      int tzs = c.TZ;
-      Split3d ss = sp;
-      while (tzs > 4 && (long long)a.nshots * c.tiles_x * std::min(ss.zslab_units, ss.yslab_units) < 8LL * sms) {
-        tzs /= 2;
-        ss = split3d(ws, tzs, nw);
-      }
+      // the slabs are a halo deep (z) or a halo wide (y): 4-plane bands
+      // (2 x 400^3, gradient: 212.0 ms against 220.0 with the 16 of the inner rows)
+      const int tzs = std::min(c.TZ, 4);
+      const Split3d ss = split3d(ws, tzs, nw);
       StepArgs a2 = a;
       a2.TZ = tzs;
       const long long b2 = (long long)a.nshots * c.tiles_x * ss.zslab_units;
       const long long b3 = (long long)a.nshots * c.tiles_x * ss.yslab_units;
       nk = (b1 > 0) + (b2 > 0) + (b3 > 0);
-      if (b1 > 0 && ws->inner_np) {
-        if (nw == 8) k_ac3d_inner_np<MODE, 8><<<(unsigned)b1, 256, 0, st>>>(a1);
-        else k_ac3d_inner_np<MODE><<<(unsigned)b1, 128, 0, st>>>(a1);
-      } else if (b1 > 0) {
+      if (b1 > 0) {
         if (nw == 8) k_ac3d_inner<MODE, 8><<<(unsigned)b1, 256, 0, st>>>(a1);
         else k_ac3d_inner<MODE><<<(unsigned)b1, 128, 0, st>>>(a1);
       }
-      if (b2 > 0 && ws->inner_np) {
-        if (nw == 8) k_ac3d_zslab<MODE, 8, false><<<(unsigned)b2, 256, 0, st>>>(a2);
-        else k_ac3d_zslab<MODE, 4, false><<<(unsigned)b2, 128, 0, st>>>(a2);
-      } else if (b2 > 0) {
+      if (b2 > 0) {
         if (nw == 8) k_ac3d_zslab<MODE, 8><<<(unsigned)b2, 256, 0, st>>>(a2);
         else k_ac3d_zslab<MODE><<<(unsigned)b2, 128, 0, st>>>(a2);
       }
-      if (b3 > 0 && ws->inner_np) {
-        if (nw == 8) k_ac3d_yslab<MODE, 8, false><<<(unsigned)b3, 256, 0, st>>>(a2);
-        else k_ac3d_yslab<MODE, 4, false><<<(unsigned)b3, 128, 0, st>>>(a2);
-      } else if (b3 > 0) {
+      if (b3 > 0) {
         if (nw == 8) k_ac3d_yslab<MODE, 8><<<(unsigned)b3, 256, 0, st>>>(a2);
         else k_ac3d_yslab<MODE><<<(unsigned)b3, 128, 0, st>>>(a2);
       }
@@ -2379,7 +2376,6 @@ void wavesim_set_tuning(sw_wavesim* ws, int tz, int variant) {
   ws->pair_tz = pair_tz[(variant >> 11) & 7];
   ws->pair_occ = (variant >> 14) & 3;
   ws->split3d = (variant & 65536) == 0;
-  ws->inner_np = (variant & 131072) != 0;
   ws->xsplit = (variant & 262144) == 0;
 }
 void wavesim_set_band_heights(sw_wavesim* ws, int tz_forward, int tz_recompute, int tz_adjoint) {

@@ -329,6 +329,86 @@ __device__ __forceinline__ void cpml_axis_term4(float (&t)[4], const float (&pl)
   st4(s.xi_out + iq, xn);
 }
 
+// The cells of four consecutive points x0 .. x0 + 3 along x: `in` has a bit per
+// interior point inside a strip, the cell right of point e (its qr) is qb + e
+// (n >= 2 H + 3, so no group meets both strips).
+struct XCells {
+  unsigned in;
+  int qb;
+};
+__device__ __forceinline__ XCells xcells(int x0, int n, int H, bool inb) {
+  XCells c;
+  c.qb = x0 < H ? x0 : x0 + 1 - n + 2 * H;
+  c.in = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int x = x0 + e;
+    if (inb && x >= 1 && x <= n - 2 && (x < H || x >= n - H)) c.in |= 1u << e;
+  }
+  return c;
+}
+
+// cpml_axis_term for four consecutive points along the strip axis itself (x):
+// the same arithmetic per point, every memory variable and coefficient loaded
+// before the first is stored.  Point by point these were four dependent trips
+// to L2 per row, which set the time of the rows (and of the blocks) that hold
+// strip points (gradient of 2 shots of 400^3, 60 steps: 282 -> 245 ms with the
+// launches as they were; one shot of 201 x 201: 10.7 -> 9.2 us per step).
+__device__ __forceinline__ void cpml_axis_x4(float (&t)[4], const float (&p0)[4], float left, float right, int x0,
+                                             int n, int H, float ih, const XCells& xc, const StripIO& s) {
+  // cells qb - 1 .. qb + 3 are the half nodes around the points; those next to a strip point are read
+  const unsigned cells = xc.in | xc.in << 1;
+  const float* pi = s.psi_in + s.psi_base + (xc.qb - 1);
+  const float* ah = s.ah + (xc.qb - 1);
+  const float* bh = s.bh + (xc.qb - 1);
+  const float* xi = s.xi_in + s.xi_base + xc.qb;
+  const float* a = s.a + xc.qb;
+  const float* b = s.b + xc.qb;
+  float old[5], xo[4], nw[5], A[5], B[5], an[4], bn[4];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const bool on = cells >> k & 1;
+    old[k] = on ? pi[k] : 0.f;
+    A[k] = on ? ah[k] : 0.f;
+    B[k] = on ? bh[k] : 0.f;
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const bool on = xc.in >> e & 1;
+    xo[e] = on ? xi[e] : 0.f;
+    an[e] = on ? a[e] : 0.f;
+    bn[e] = on ? b[e] : 0.f;
+  }
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const float pl = k == 0 ? left : p0[k - 1], pr = k == 4 ? right : p0[k == 4 ? 3 : k];
+    nw[k] = radd(rmul(B[k], old[k]), rmul(A[k], rmul(rsub(pr, pl), ih)));
+  }
+  float* po = s.psi_out + s.psi_base + (xc.qb - 1);
+  float* xw = s.xi_out + s.xi_base + xc.qb;
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (xc.in >> e & 1) {
+      const float tt = radd(t[e], rmul(rsub(nw[e + 1], nw[e]), ih));
+      const float xn = radd(rmul(bn[e], xo[e]), rmul(an[e], tt));
+      t[e] = radd(tt, xn);
+      po[e + 1] = nw[e + 1];
+      xw[e] = xn;
+      if (x0 + e == 1 || x0 + e == n - H) po[e] = nw[e];  // the strip's first cell
+    }
+  if (s.ck_psi) {
+    float* cp = s.ck_psi + s.psi_base + (xc.qb - 1);
+    float* cx = s.ck_xi + s.xi_base + xc.qb;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (xc.in >> e & 1) {
+        cp[e + 1] = old[e + 1];
+        cx[e] = xo[e];
+        if (x0 + e == 1 || x0 + e == n - H) cp[e] = old[e];
+      }
+  }
+}
+
 // TMA prefetch of a contiguous global range into L2 (no registers, no
 // completion to wait for).  Address 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void l2_prefetch(const void* p, unsigned bytes) {
@@ -355,6 +435,7 @@ template <int MODE>
 struct Ac2dRow {
   int nx, nz, P, H, x0, dbf16;
   bool inb, xstrip, vec_interior, fastx;
+  XCells xc;
   float ihx, ihz, ih2x, ih2z;
   StripIO sx, sz;
   float *pn, *dn, *ckp, *ckd, *Dw, *gg, *gcp;
@@ -376,6 +457,7 @@ struct Ac2dRow {
     sz.a = cp + L; sz.ah = cp + L + na; sz.b = cp + L + na + nh; sz.bh = cp + L + 2 * na + nh;
     sz.psi_step = P; sz.xi_step = P;
     xstrip = inb && (x0 < H || x0 + 3 >= nx - H);
+    xc = xcells(x0, nx, H, inb);
     vec_interior = (x0 >= 1) && (x0 + 3 <= nx - 2);
     // the warp's 128 points all interior and outside the x strips (warp-uniform)
     const int wx = x0 - 4 * (int)(threadIdx.x & 31);
@@ -407,42 +489,25 @@ struct Ac2dRow {
     float outp[4], outd[4], outD[4];
     if ((XS || fastx) && z >= plain_lo(H) && z <= plain_hi(nz, H)) {
       row4_interior(rm, r0, rp, left, right, o, f, ih2x, ih2z, outp, outd, outD);
-    } else if (XS) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float c = r0[e];
-        const float tx = d2term(e == 0 ? left : r0[e - 1], c, e == 3 ? right : r0[e + 1], ih2x);
-        float tz = d2term(rm[e], c, rp[e], ih2z);
-        if (zstrip && inb && !xstrip) {
-          sz.psi_base = x0 + e;
-          sz.xi_base = x0 + e;
-          tz = cpml_axis_term(tz, rm[e], c, rp[e], z, nz, H, ihz, sz);
-        }
-        const float lap = radd(tx, tz);
-        outD[e] = rmul(f[e], lap);
-        outd[e] = radd(o[e], outD[e]);
-        outp[e] = radd(c, outd[e]);
-      }
     } else {
+      float tx[4], tz[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float xm = e == 0 ? left : r0[e - 1];
-        const float xp = e == 3 ? right : r0[e + 1];
-        const float c = r0[e];
-        float tx = d2term(xm, c, xp, ih2x);
-        float tz = d2term(rm[e], c, rp[e], ih2z);
-        const int x = x0 + e;
-        const bool pin = inb && x >= 1 && x <= nx - 2;
-        if (xstrip && pin) tx = cpml_axis_term(tx, xm, c, xp, x, nx, H, ihx, sx);
-        if (zstrip && pin) {
-          sz.psi_base = x;
-          sz.xi_base = x;
-          tz = cpml_axis_term(tz, rm[e], c, rp[e], z, nz, H, ihz, sz);
-        }
-        const float lap = radd(tx, tz);
+        tx[e] = d2term(e == 0 ? left : r0[e - 1], r0[e], e == 3 ? right : r0[e + 1], ih2x);
+        tz[e] = d2term(rm[e], r0[e], rp[e], ih2z);
+      }
+      if (!XS && xc.in) cpml_axis_x4(tx, r0, left, right, x0, nx, H, ihx, xc, sx);
+      if (zstrip && inb && !(XS && xstrip)) {
+        sz.psi_base = x0;
+        sz.xi_base = x0;
+        cpml_axis_term4(tz, rm, r0, rp, z, nz, H, ihz, sz);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float lap = radd(tx[e], tz[e]);
         outD[e] = rmul(f[e], lap);
         outd[e] = radd(o[e], outD[e]);
-        outp[e] = radd(c, outd[e]);
+        outp[e] = radd(r0[e], outd[e]);
       }
     }
     if (!inb || (XS && xstrip)) return;
@@ -1524,7 +1589,7 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
   const float* __restrict__ fa = A.fact;
   const int na = 2 * H + 2, nh = 2 * H;
 
-  const bool xstrip = inb && (x0 < H || x0 + 3 >= nx - H);
+  const XCells xc = xcells(x0, nx, H, inb);
   // region 1: never in a y strip; region 3: always
   const bool ystrip = REGION == 3 || (REGION != 1 && ((y < H) || (y >= ny - H)));
   // the warp's 128 x points and its y row interior and outside the strips
@@ -1605,13 +1670,12 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
         tx[e] = d2term(xm, c, xp, A.ih2[0]);
         ty[e] = d2term(ym[e], c, yp[e], A.ih2[1]);
         tz[e] = d2term(rm[e], c, rp[e], A.ih2[2]);
-        const int x = x0 + e;
-        if (xstrip && inb && x >= 1 && x <= nx - 2) {
-          StripIO s0 = strip_io(A, 0, shot, 1);
-          s0.psi_base = ((long long)z * ny + y) * nh;
-          s0.xi_base = ((long long)z * ny + y) * na;
-          tx[e] = cpml_axis_term(tx[e], xm, c, xp, x, nx, H, A.ih[0], s0);
-        }
+      }
+      if (xc.in) {
+        StripIO s0 = strip_io(A, 0, shot, 1);
+        s0.psi_base = ((long long)z * ny + y) * nh;
+        s0.xi_base = ((long long)z * ny + y) * na;
+        cpml_axis_x4(tx, r0, left, right, x0, nx, H, A.ih[0], xc, s0);
       }
       // the y and z strips: the strip cell is the same for the four points
       // (it depends on y or z only), so their memory variables move as float4
@@ -1711,24 +1775,21 @@ __global__ void __launch_bounds__(32 * NW) k_ac3d_fwd(const StepArgs A) {
 // Three-launch 3D step: rows outside the y and z strips (no y / z C-PML code,
 // fewer registers), the z slabs (z strip code only where it applies), the y
 // slabs.  Every point is computed by exactly one launch with the arithmetic
-// of ac3d_body.
+// of ac3d_body.  No software pipeline: 6 resident blocks per SM of the inner
+// rows and 5 of the slabs beat the pipelined form at 6 and 4 (gradient of 2
+// shots of 400^3, 60 steps: 212 against 244 ms); 8 / 6 / 6 run 216 ms
+// (spills), 5 / 4 / 4 230 ms.
 template <int MODE, int NW = 4>
 __global__ void __launch_bounds__(32 * NW, 24 / NW) k_ac3d_inner(const StepArgs A) {
-  ac3d_body<MODE, NW, false, 1>(A);
-}
-// the same without the software pipeline, at 8 resident blocks of 4 warps
-template <int MODE, int NW = 4>
-__global__ void __launch_bounds__(32 * NW, 32 / NW) k_ac3d_inner_np(const StepArgs A) {
   ac3d_body<MODE, NW, false, 1, false>(A);
 }
-// (the z slabs fit 6 blocks per SM without the software pipeline, 4 with it)
-template <int MODE, int NW = 4, bool PIPE = true>
-__global__ void __launch_bounds__(32 * NW, PIPE ? 16 / NW : 24 / NW) k_ac3d_zslab(const StepArgs A) {
-  ac3d_body<MODE, NW, false, 2, PIPE>(A);
+template <int MODE, int NW = 4>
+__global__ void __launch_bounds__(32 * NW, 20 / NW) k_ac3d_zslab(const StepArgs A) {
+  ac3d_body<MODE, NW, false, 2, false>(A);
 }
-template <int MODE, int NW = 4, bool PIPE = true>
-__global__ void __launch_bounds__(32 * NW, 16 / NW) k_ac3d_yslab(const StepArgs A) {
-  ac3d_body<MODE, NW, false, 3, PIPE>(A);
+template <int MODE, int NW = 4>
+__global__ void __launch_bounds__(32 * NW, 20 / NW) k_ac3d_yslab(const StepArgs A) {
+  ac3d_body<MODE, NW, false, 3, false>(A);
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,49 @@
+// Launches of the time loop as a chain of programmatic dependent launches.
+//
+// A time step is a chain of two to five short kernels, each reading what the
+// one before it wrote.  As plain stream work every link costs the drain of one
+// kernel, the launch of the next and its first instructions, one after the
+// other (about 1.5 us per link on a GB300 in a CUDA graph, as much as a
+// small grid's kernel itself).  Here every kernel of the loop lets its
+// successor be scheduled as soon as all its blocks have started (chain_next)
+// and waits, as its first action on data that the loop writes, until its
+// predecessor has completed and its writes are visible (chain_wait); what lies
+// before chain_wait - index arithmetic, shot tables - overlaps with the
+// predecessor.
+//
+// Rules that keep the chain safe: a kernel launched with launch_chain calls
+// chain_wait in every thread before it returns or touches anything that an
+// earlier kernel of the chain reads or writes (so a kernel completes after its
+// predecessor, and its successor's wait covers the whole chain); the tables
+// read before the wait are uploaded by copies or memsets, which the first
+// kernel of a chain waits for in full.  A kernel launched plainly, a copy or
+// a memset waits for everything before it as always, and chain_wait in a
+// plainly launched kernel returns at once.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <utility>
+
+#include "internal.h"
+
+namespace swgb {
+
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... Q>
+void launch_chain(const char* what, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, Q&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<Q>(args))...), what);
+}
+
+}  // namespace swgb

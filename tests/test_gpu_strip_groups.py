@@ -5,6 +5,7 @@ one row (the default on small grids) to more rows than the grid has."""
 import numpy as np
 import pytest
 
+import cases as C
 import elastic_cases as E
 import vd_cases as V
 from vd_cases import rel_l2, sw
@@ -64,3 +65,23 @@ def test_elastic_groups_and_bands(ctx, nx, nz, halo, kind, freetop):
         assert rel_l2(out[0][q], gref[k]) < TOL, k
     for tz in (8, 32, 128):
         assert _same(out[tz], out[0]), tz
+
+
+@pytest.mark.parametrize("shape,halo", [((23, 26), 10), ((131, 40), 13), ((517, 33), 6), ((60, 50), 1), ((64, 40), 0),
+                                        ((23, 25, 24), 10), ((133, 20, 18), 3), ((30, 28, 19), 0)])
+@pytest.mark.parametrize("freetop", [False, True])
+def test_acoustic_groups(oracle, shape, halo, freetop):
+    """Constant density, 2D and 3D: four points of an x strip at once, at the strips' ends inside a group and on
+    the narrowest grid of a halo; gradient with checkpoints (the copies of the memory variables included)."""
+    h = (9.0, 8.0, 7.0)[:len(shape)]
+    vp = C.smooth_model(shape, 1700.0, 3100.0, 5)
+    case = C.Case(vp=vp, h=h, dt=C.stable_dt(vp, h), halo=halo, freetop=freetop)
+    ex = [hh * (n - 1) for n, hh in zip(shape, h)]
+    rec = [[x] + [0.4 * e for e in ex[1:-1]] + [0.3 * ex[-1]] for x in np.linspace(0.1, 0.9, 7) * ex[0]]
+    shot = C.make_shot(h, ex, 90, case.dt, 25.0, [[0.45 * e for e in ex]], rec)
+    shot.observed = 0.5 * C.oracle_forward(oracle, sw, case, shot).astype(np.float32).astype(np.float64)
+    gref, _, tref = C.oracle_gradient(oracle, sw, case, shot, check_freq=7)
+    run = C.GpuRun(sw, case, gradient=True, check_freq=7)
+    g, _, t = run.gradient([shot])
+    run.close()
+    assert rel_l2(t[0], tref) < TOL and rel_l2(g, gref) < TOL
