@@ -40,6 +40,7 @@
 #include <cuda_bf16.h>
 
 #include "acoustic_kernels.cuh"
+#include "graph.cuh"
 #include "internal.h"
 #include "ccts.cuh"
 
@@ -119,7 +120,17 @@ __global__ void k_inject_record(const ShotDesc* __restrict__ desc, const long lo
                                 FieldArg plo, FieldArg dlo, FieldArgE dexp, int P) {
   const int shot = blockIdx.x;
   const ShotDesc D = desc[shot];
-  if (it > D.nt) return;
+  // this thread's first source point and receiver: the tables are read while the stencil still runs
+  const bool on = it <= D.nt;
+  const int t0 = threadIdx.x;
+  const bool src0 = on && t0 < D.nsp, rec0 = on && record && t0 < D.nrec;
+  const long long slin0 = src0 ? pts[D.sp_off + t0] : 0, rlin0 = rec0 ? rec_lin[D.rec_off + t0] : 0;
+  const int sk0 = src0 ? ptr[D.sp_ptr + t0] : 0, sk1 = src0 ? ptr[D.sp_ptr + t0 + 1] : 0;
+  const int slot0 = src0 ? bslot[D.sp_off + t0] : -1;
+  const float sv0 = sk1 > sk0 ? D.tf[(long long)(it - 1) + (long long)ids[sk0] * D.nt] : 0.f;
+  chain_wait();
+  chain_next();
+  if (!on) return;
   if (it_stash > 0) {
     const float* sp = stash.p + (long long)shot * stash.s;
     for (int r = threadIdx.x; r < D.nrec; r += blockDim.x)
@@ -133,11 +144,12 @@ __global__ void k_inject_record(const ShotDesc* __restrict__ desc, const long lo
     dd16 = dd;
     dd = nullptr;
   }
-  for (int u = threadIdx.x; u < D.nsp; u += blockDim.x) {
-    const long long lin = pts[D.sp_off + u];
+  for (int u = t0; u < D.nsp; u += blockDim.x) {
+    const bool first = u == t0;
+    const long long lin = first ? slin0 : pts[D.sp_off + u];
     float add = 0.f;
-    const int k0 = ptr[D.sp_ptr + u], k1 = ptr[D.sp_ptr + u + 1];
-    const int slot = bslot[D.sp_off + u];
+    const int k0 = first ? sk0 : ptr[D.sp_ptr + u], k1 = first ? sk1 : ptr[D.sp_ptr + u + 1];
+    const int slot = first ? slot0 : bslot[D.sp_off + u];
     if (slot >= 0) {
       for (int k = k0; k < k1; ++k) add += D.tf[(long long)(it - 1) + (long long)ids[k] * D.nt];
       float sd;
@@ -161,7 +173,7 @@ __global__ void k_inject_record(const ShotDesc* __restrict__ desc, const long lo
     } else {
       float acc = pn[lin];
       for (int k = k0; k < k1; ++k) {
-        const float v = D.tf[(long long)(it - 1) + (long long)ids[k] * D.nt];
+        const float v = first && k == k0 ? sv0 : D.tf[(long long)(it - 1) + (long long)ids[k] * D.nt];
         acc += v;
         add += v;
       }
@@ -189,8 +201,8 @@ __global__ void k_inject_record(const ShotDesc* __restrict__ desc, const long lo
   if (!record) return;
   __syncthreads();
   const float* pnl = plo.p ? plo.p + (long long)shot * plo.s : nullptr;
-  for (int r = threadIdx.x; r < D.nrec; r += blockDim.x) {
-    const long long q = rec_lin[D.rec_off + r];
+  for (int r = t0; r < D.nrec; r += blockDim.x) {
+    const long long q = r == t0 ? rlin0 : rec_lin[D.rec_off + r];
     D.tr[(long long)(it - 1) + (long long)r * D.nt] = pnl ? __fadd_rn(pn[q], pnl[q]) : pn[q];
   }
 }
@@ -204,6 +216,8 @@ __device__ void adj_inject_shot(const ShotDesc& D, const long long* __restrict__
                                 const float* dp, int dbf16, float* gp, float* cp, int it, const signed char* ex,
                                 int P);
 
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // One block per accumulator group (grp consecutive shots share one gradient
 // pair); the group's shots are handled one after the other, so receivers of
 // different shots on the same grid point never update the pair concurrently.
@@ -211,6 +225,18 @@ __global__ void k_adj_inject(const ShotDesc* __restrict__ desc, const long long*
                              const int* __restrict__ ptr, const int* __restrict__ ids,
                              const int* __restrict__ bslot, FieldArg lam, FieldArg lamd, FieldArg dcorr, FieldArg g,
                              FieldArg gc, int it, int nshots, int grp, int dbf16, FieldArgE dexp, int P) {
+  // the shot's table entries of this thread are in L1 when the stencil completes
+  if ((int)blockIdx.x * grp < nshots) {
+    const ShotDesc& D = desc[blockIdx.x * grp];
+    if (it <= D.nt && (int)threadIdx.x < D.nrp) {
+      const int k0 = ptr[D.rp_ptr + threadIdx.x];
+      prefetch_l1(pts + D.rp_off + threadIdx.x);
+      prefetch_l1(bslot + D.rp_off + threadIdx.x);
+      prefetch_l1(D.adj + (it - 1) + (long long)ids[k0] * D.nt);
+    }
+  }
+  chain_wait();
+  chain_next();
   float* gp = g.p + (long long)blockIdx.x * g.s;
   float* cp = gc.p ? gc.p + (long long)blockIdx.x * gc.s : nullptr;  // null: plain FP32 sums
   for (int j = 0; j < grp; ++j) {
@@ -568,21 +594,12 @@ struct sw_wavesim {
                            // false: the grouped Kahan adjoint (k_ac2d_adj_grp) for 4+ shots
   bool adjw = false;       // the current gradient call uses MODE_ADJW
   DevMem tot64;            // MODE_ADJW: FP64 gradient total (padded layout)
-  // CUDA graphs of a group's whole time loop, keyed by what the captured launches depend on
-  long long gen = 0;  // bumped whenever a device buffer the kernels see is (re)allocated
+  GraphCache cache;  // a group's whole time loop
   bool use_graphs = true;
-  std::map<std::vector<long long>, cudaGraphExec_t> graphs;
-  std::map<std::vector<long long>, int> graph_uses;  // calls per key (a key is captured on its second call)
   DevMem d_gout, d_mout;  // gradient / misfit of the host-buffer path (stable addresses for the graphs)
   // snapshots requested by the current forward call (snapevery = 0: none)
   int snapevery = 0;
   float* const* snap_out = nullptr;  // per caller shot: host buffer of nt/snapevery fields
-  void drop_graphs() {
-    for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
-    graphs.clear();
-    graph_uses.clear();
-  }
-  ~sw_wavesim() { drop_graphs(); }
 };
 
 namespace {
@@ -598,53 +615,14 @@ void ensure(sw_wavesim* ws, DevMem& m, size_t bytes, const char* what) {
   if (m.bytes >= bytes && m.p) return;
   m.release();
   dev_alloc(m, bytes, what, ws->ctx->stream);
-  ++ws->gen;
+  ++ws->cache.gen;
 }
 
-// Runs `work` (the device work of one group: launches, memsets, no host
-// synchronisation and no allocation) through a CUDA graph: captured on the
-// second call with `key` (one-off calls run directly), replayed afterwards;
-// at most 32 graphs are kept per simulation, later keys run directly.  Launch-bound cases (small grids, single
-// shots) gain the most.  Work runs directly instead when profiling (the
-// per-kernel events belong to single launches), when the caller's stream is
-// itself being captured (the launches then join the caller's graph), for the
-// TMA stencil variant, or when graphs are switched off.
+// GraphCache::run, or directly for the TMA stencil variant or when graphs are switched off.
 template <typename Work>
 void run_graph(sw_wavesim* ws, std::vector<long long> key, Work&& work) {
-  cudaStream_t st = ws->ctx->stream;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  check_cuda(cudaStreamIsCapturing(st, &cs), "cudaStreamIsCapturing");
-  if (!ws->use_graphs || ws->ctx->prof.on || cs != cudaStreamCaptureStatusNone || (ws->variant & 3) == 1) {
-    work();
-    return;
-  }
-  key.push_back(ws->gen);
-  auto it = ws->graphs.find(key);
-  if (it == ws->graphs.end()) {
-    if (ws->graph_uses.size() > 4096) ws->graph_uses.clear();
-    if (++ws->graph_uses[key] < 2 || ws->graphs.size() >= 32) {
-      work();
-      return;
-    }
-    check_cuda(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin stream capture");
-    try {
-      work();
-    } catch (...) {
-      cudaGraph_t g = nullptr;
-      cudaStreamEndCapture(st, &g);
-      if (g) cudaGraphDestroy(g);
-      cudaGetLastError();
-      throw;
-    }
-    cudaGraph_t g = nullptr;
-    check_cuda(cudaStreamEndCapture(st, &g), "end stream capture");
-    cudaGraphExec_t ex = nullptr;
-    const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
-    cudaGraphDestroy(g);
-    check_cuda(e, "graph instantiate");
-    it = ws->graphs.emplace(key, ex).first;
-  }
-  check_cuda(cudaGraphLaunch(it->second, st), "graph launch");
+  if (!ws->use_graphs || (ws->variant & 3) == 1) work();
+  else ws->cache.run(ws->ctx, std::move(key), work);
 }
 
 std::vector<long long> group_key(const sw_wavesim* ws, const std::vector<HostShot>& group, bool grad) {
@@ -1062,7 +1040,7 @@ void ensure_state(sw_wavesim* ws, int S, bool grad, int max_nt) {
     ws->cap = S;
     ws->d_slots = 0;
     ws->ck_slots = 0;
-    ++ws->gen;
+    ++ws->cache.gen;
   }
   if (ws->precision == 1 && ws->hp_cap < ws->cap) {
     for (int b = 0; b < 2; ++b) dev_alloc(ws->plo[b], (size_t)ws->cap * F * sizeof(float), "pressure low part", st);
@@ -1073,7 +1051,7 @@ void ensure_state(sw_wavesim* ws, int S, bool grad, int max_nt) {
       dev_alloc(ws->xi64[d], (size_t)ws->cap * ws->xsz[d] * sizeof(double), "xi (FP64)", st);
     }
     ws->hp_cap = ws->cap;
-    ++ws->gen;
+    ++ws->cache.gen;
   }
   if (grad) {
     const int K = ws->gp.check_freq;
@@ -1087,7 +1065,7 @@ void ensure_state(sw_wavesim* ws, int S, bool grad, int max_nt) {
         check_cuda(cudaMemsetAsync(ws->dexp.p, 0, ws->dexp.bytes, st), "D exponents");
       }
       ws->d_slots = dslots;
-      ++ws->gen;
+      ++ws->cache.gen;
     }
     const long long cks = K == 1 ? 0 : max_nt / K;
     if (cks > ws->ck_slots) {
@@ -1103,11 +1081,11 @@ void ensure_state(sw_wavesim* ws, int S, bool grad, int max_nt) {
         dev_alloc(ws->ck_stage, (size_t)ws->cap * 2 * F * sizeof(float), "checkpoint stage", st);
       }
       ws->ck_slots = cks;
-      ++ws->gen;
+      ++ws->cache.gen;
     }
     if (!ws->zero.p) {
       dev_alloc(ws->zero, (size_t)(2 * F + ws->strip_total) * sizeof(float), "zero state", st);
-      ++ws->gen;
+      ++ws->cache.gen;
     }
   }
 }
@@ -1358,7 +1336,8 @@ int launch_2d_xsplit(long long blocks, cudaStream_t st, const StepArgs& a) {
   int nl, xr, ng;
   xstrip_groups(a.n0, a.halo, a.P, nl, xr, ng);
   const long long items = (long long)ng * (a.n1 - 2) * a.nshots;
-  k_ac2d_step<MODE, 4, 1, true><<<(unsigned)(blocks + (items + 127) / 128), 128, 0, st>>>(a);
+  launch_chain("stencil launch", k_ac2d_step<MODE, 4, 1, true>, dim3((unsigned)(blocks + (items + 127) / 128)), dim3(128),
+               st, a);
   return 1;
 }
 
@@ -1415,10 +1394,9 @@ struct Launcher {
     if constexpr (MODE == MODE_FWD || MODE == MODE_FWD_D) {
       if (ws->precision == 1 && !recompute) {  // compensated forward (context from make_hp_ctx)
         if (ws->N == 2)
-          k_ac_hp<MODE, 2><<<(unsigned)blocks, 128, 0, st>>>(a);
+          launch_chain("compensated stencil launch", k_ac_hp<MODE, 2>, dim3((unsigned)blocks), dim3(128), st, a);
         else
-          k_ac_hp<MODE, 3><<<(unsigned)blocks, 128, 0, st>>>(a);
-        check_cuda(cudaGetLastError(), "compensated stencil launch");
+          launch_chain("compensated stencil launch", k_ac_hp<MODE, 3>, dim3((unsigned)blocks), dim3(128), st, a);
         ws->ctx->prof.end(st, kind, ev);
         return;
       }
@@ -1480,16 +1458,16 @@ struct Launcher {
       const long long b3 = (long long)a.nshots * c.tiles_x * ss.yslab_units;
       nk = (b1 > 0) + (b2 > 0) + (b3 > 0);
       if (b1 > 0) {
-        if (nw == 8) k_ac3d_inner<MODE, 8><<<(unsigned)b1, 256, 0, st>>>(a1);
-        else k_ac3d_inner<MODE><<<(unsigned)b1, 128, 0, st>>>(a1);
+        if (nw == 8) launch_chain("stencil launch", k_ac3d_inner<MODE, 8>, dim3((unsigned)b1), dim3(256), st, a1);
+        else launch_chain("stencil launch", k_ac3d_inner<MODE, 4>, dim3((unsigned)b1), dim3(128), st, a1);
       }
       if (b2 > 0) {
-        if (nw == 8) k_ac3d_zslab<MODE, 8><<<(unsigned)b2, 256, 0, st>>>(a2);
-        else k_ac3d_zslab<MODE><<<(unsigned)b2, 128, 0, st>>>(a2);
+        if (nw == 8) launch_chain("stencil launch", k_ac3d_zslab<MODE, 8>, dim3((unsigned)b2), dim3(256), st, a2);
+        else launch_chain("stencil launch", k_ac3d_zslab<MODE, 4>, dim3((unsigned)b2), dim3(128), st, a2);
       }
       if (b3 > 0) {
-        if (nw == 8) k_ac3d_yslab<MODE, 8><<<(unsigned)b3, 256, 0, st>>>(a2);
-        else k_ac3d_yslab<MODE><<<(unsigned)b3, 128, 0, st>>>(a2);
+        if (nw == 8) launch_chain("stencil launch", k_ac3d_yslab<MODE, 8>, dim3((unsigned)b3), dim3(256), st, a2);
+        else launch_chain("stencil launch", k_ac3d_yslab<MODE, 4>, dim3((unsigned)b3), dim3(128), st, a2);
       }
     } else {
       const int nw = block_rows3d(ws);
@@ -1646,12 +1624,11 @@ void launch_inject(sw_wavesim* ws, int Sa, const FieldArg& pnew, const FieldArg&
   cudaEvent_t ev = nullptr;
   ws->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
   const FieldArg stash{ws->d_stash.as<float>(), (long long)PAIR_MAXRR * ws->P};
-  k_inject_record<<<Sa, 128, 0, st>>>(ws->d_desc.as<ShotDesc>(), ws->d_pts.as<long long>(), ws->d_ptr.as<int>(),
-                                      ws->d_ids.as<int>(), ws->d_bslot.as<int>(), ws->d_rec.as<long long>(), pnew,
-                                      dnew, Dw, d_first, it, record,
-                                      (ws->gradient && ws->gp.snapshot_bf16 >= 1) ? (ws->gp.snapshot_bf16 == 3 ? 2 : 1) : 0,
-                                      ws->d_recstash.as<int>(), stash, it_stash, plo, dlo, dexp_for(ws, Dw), ws->P);
-  check_cuda(cudaGetLastError(), "inject/record launch");
+  launch_chain("inject/record launch", k_inject_record, dim3((unsigned)Sa), dim3(128), st, ws->d_desc.as<ShotDesc>(),
+               ws->d_pts.as<long long>(), ws->d_ptr.as<int>(), ws->d_ids.as<int>(), ws->d_bslot.as<int>(),
+               ws->d_rec.as<long long>(), pnew, dnew, Dw, d_first, it, record,
+               (ws->gradient && ws->gp.snapshot_bf16 >= 1) ? (ws->gp.snapshot_bf16 == 3 ? 2 : 1) : 0,
+               ws->d_recstash.as<int>(), stash, it_stash, plo, dlo, dexp_for(ws, Dw), ws->P);
   ws->ctx->prof.end(st, KK_SRCREC, ev);
 }
 
@@ -1961,11 +1938,10 @@ void adjoint_group(sw_wavesim* ws, const std::vector<HostShot>& group) {
     const int it_last = two ? it - 1 : it;  // the step whose adjoint sources are injected now
     cudaEvent_t ev = nullptr;
     ws->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    k_adj_inject<<<(Sa + ws->grp - 1) / ws->grp, 128, 0, st>>>(
-        ws->d_desc.as<ShotDesc>(), ws->d_pts.as<long long>(), ws->d_ptr.as<int>(), ws->d_ids.as<int>(),
-        ws->d_bslot.as<int>(), a.pnew, a.dout, dcorr_last, a.g, a.gc, it_last, Sa, ws->grp, a.dbf16,
-        dexp_for(ws, dcorr_last), ws->P);
-    check_cuda(cudaGetLastError(), "adjoint inject launch");
+    launch_chain("adjoint inject launch", k_adj_inject, dim3((unsigned)((Sa + ws->grp - 1) / ws->grp)), dim3(128), st,
+                 ws->d_desc.as<ShotDesc>(), ws->d_pts.as<long long>(), ws->d_ptr.as<int>(), ws->d_ids.as<int>(),
+                 ws->d_bslot.as<int>(), a.pnew, a.dout, dcorr_last, a.g, a.gc, it_last, Sa, ws->grp, a.dbf16,
+                 dexp_for(ws, dcorr_last), ws->P);
     ws->ctx->prof.end(st, KK_SRCREC, ev);
     if (ws->adjw && (it_last - 1) % 32 == 0) {  // at most 32 terms per FP32 sum
       ws->ctx->prof.begin(st, KK_OTHER, 0.0, &ev);
@@ -2386,7 +2362,7 @@ void wavesim_set_band_heights(sw_wavesim* ws, int tz_forward, int tz_recompute, 
 void wavesim_set_precision(sw_wavesim* ws, int mode) {
   if (mode == ws->precision) return;
   ws->precision = mode;
-  ws->drop_graphs();
+  ws->cache.drop();
   if (mode == 1 && !ws->fact_lo.p) {
     cudaStream_t st = ws->ctx->stream;
     dev_alloc(ws->fact_lo, (size_t)ws->F * sizeof(float), "fact low part", st);
@@ -2408,7 +2384,7 @@ void wavesim_set_wait_test(sw_wavesim* ws, long long wait_cycles, int withhold) 
 }
 void wavesim_use_graphs(sw_wavesim* ws, bool on) {
   ws->use_graphs = on;
-  if (!on) ws->drop_graphs();
+  if (!on) ws->cache.drop();
 }
 sw_ctx* wavesim_ctx(sw_wavesim* ws) { return ws->ctx; }
 sw_wavesim* wavesim_new() { return new sw_wavesim(); }

@@ -40,6 +40,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "chain.cuh"
 #include "internal.h"
 #include "ff.cuh"
 
@@ -627,6 +628,8 @@ struct Ac2dBounds {
 template <int MODE, int NW, int DP = 1, bool XS = false>
 __global__ void __launch_bounds__(32 * NW, (Ac2dBounds<MODE, NW>::MINB - (DP - 1))) k_ac2d_step(const StepArgs A) {
   constexpr unsigned FULL = 0xffffffffu;
+  chain_next();
+  chain_wait();
   if constexpr (XS) {
     const long long nb_main = (long long)A.nshots * A.tiles_x * A.tiles_y * A.tiles_z;
     if ((long long)blockIdx.x >= nb_main) {
@@ -1567,6 +1570,8 @@ __device__ __forceinline__ bool ac3d_work(const StepArgs& A, int tile, int warp,
 template <int MODE, int NW, bool FAST = false, int REGION = 0, bool PIPE = true>
 __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
   constexpr unsigned FULL = 0xffffffffu;
+  chain_next();
+  chain_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int S = A.nshots;
   const int shot = blockIdx.x % S;
@@ -2172,6 +2177,8 @@ template <int MODE, int NDIM>
 __global__ void __launch_bounds__(128, NDIM == 2 ? 6 : 1) k_ac_hp(const StepArgs A) {
   static_assert(MODE == MODE_FWD || MODE == MODE_FWD_D, "compensated step: forward modes only");
   constexpr unsigned FULL = 0xffffffffu;
+  chain_next();
+  chain_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int S = A.nshots;
   const int shot = blockIdx.x % S;

@@ -5,11 +5,18 @@
 // kernel, the launch of the next and its first instructions, one after the
 // other (about 1.5 us per link on a GB300 in a CUDA graph, as much as a
 // small grid's kernel itself).  Here every kernel of the loop lets its
-// successor be scheduled as soon as all its blocks have started (chain_next)
-// and waits, as its first action on data that the loop writes, until its
+// successor be scheduled early (chain_next, once all its blocks have called
+// it) and waits, as its first action on data that the loop writes, until its
 // predecessor has completed and its writes are visible (chain_wait); what lies
 // before chain_wait - index arithmetic, shot tables - overlaps with the
-// predecessor.
+// predecessor.  The stencils call chain_next first thing; the source and
+// receiver kernels call it after their chain_wait, since their few blocks
+// would otherwise let the next stencil in while the previous one still runs,
+// and its blocks would crowd on the SMs that became free first (one shot of
+// 801 x 801, gradient: 30.4 ms against 36.0; compensated forward of 4 shots of
+// 901 x 455: 34.8 against 45.7).  Without any chain_next: 35.3 ms; two shots of
+// 601 x 397 elastic, 500 steps: 9.9 ms with, 10.9 without, 16.4 as plain
+// launches outside a graph.
 //
 // Rules that keep the chain safe: a kernel launched with launch_chain calls
 // chain_wait in every thread before it returns or touches anything that an

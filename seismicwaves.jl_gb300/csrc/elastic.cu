@@ -51,6 +51,8 @@
 #include <sstream>
 #include <vector>
 
+#include "chain.cuh"
+#include "graph.cuh"
 #include "internal.h"
 #include "ccts.cuh"
 
@@ -440,6 +442,8 @@ __device__ __forceinline__ unsigned xmask_half(const Geo& g, int i0) {
 // kernels spill (80.2 against 77.3 ms), with 4 / 5 too few rows are in flight
 // (79.4 ms).
 __global__ void __launch_bounds__(BX, 5) k_el_stress4(const Args A) {
+  chain_next();
+  chain_wait();
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
@@ -592,6 +596,8 @@ struct ElDispBounds {
 };
 template <int COMP>
 __global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const Args A) {
+  chain_next();
+  chain_wait();
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
@@ -833,32 +839,35 @@ __global__ void k_el_inject_sigma(const ShotDesc* __restrict__ desc, int it, lon
                                   float* sxz) {
   const int s = blockIdx.y;
   const ShotDesc& D = desc[s];
-  if (it > D.nt || D.kind != 0) return;
+  const bool on = it <= D.nt && D.kind == 0;
   const float scale = D.sf;
-  const long long so = (long long)s * F;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;  // the grid covers the largest table
+  // what the point gets needs the tables only: formed while the stress update still runs
+  float a[2] = {0.0f, 0.0f}, b = 0.0f;
+  long long c[2] = {0, 0};
+#pragma unroll
   for (int t = 0; t < 2; ++t) {
     const Inj J = D.src[t];
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < J.np; p += gridDim.x * blockDim.x) {
-      float a = 0.0f, b = 0.0f;
-      for (int e = J.ptr[p]; e < J.ptr[p + 1]; ++e) {
-        const int k = J.item[e];
-        const float v = J.coef[e] * (D.tf[(long long)(it - 1) + (long long)k * D.nt] * scale);
-        if (t == 0) {
-          a += D.mtp[3 * k] * v;
-          b += D.mtp[3 * k + 1] * v;
-        } else {
-          a += D.mtp[3 * k + 2] * v;
-        }
-      }
-      const long long c = so + J.lin[p];
+    if (!on || p >= J.np) continue;
+    c[t] = (long long)s * F + J.lin[p];
+    for (int e = J.ptr[p]; e < J.ptr[p + 1]; ++e) {
+      const int k = J.item[e];
+      const float v = J.coef[e] * (D.tf[(long long)(it - 1) + (long long)k * D.nt] * scale);
       if (t == 0) {
-        sxx[c] += a;
-        szz[c] += b;
+        a[0] += D.mtp[3 * k] * v;
+        b += D.mtp[3 * k + 1] * v;
       } else {
-        sxz[c] += a;
+        a[1] += D.mtp[3 * k + 2] * v;
       }
     }
   }
+  chain_wait();
+  chain_next();
+  if (on && p < D.src[0].np) {
+    sxx[c[0]] += a[0];
+    szz[c[0]] += b;
+  }
+  if (on && p < D.src[1].np) sxz[c[1]] += a[1];
 }
 
 // u += w tf / rho dt^2 on the ux (table 0) and uz (table 1) grids; adjoint = 1
@@ -872,29 +881,36 @@ __global__ void k_el_inject_force(const ShotDesc* __restrict__ desc, int it, int
                                   const float* __restrict__ dtr_i, const float* __restrict__ dtr_j) {
   const int s = blockIdx.y;
   const ShotDesc& D = desc[s];
-  if (it > D.nt) return;
-  if (!adjoint && D.kind != 1) return;
+  const bool on = it <= D.nt && (adjoint || D.kind == 1);
   const long long so = (long long)s * F;
   const float* tf = adjoint ? D.adjsrc : D.tf;
   const float scale = adjoint ? *adj_scale : D.sf;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;  // the grid covers the largest table
+  // the forces need the tables only: formed while the displacement update still runs
+  float acc[2] = {0.0f, 0.0f}, r[2] = {0.0f, 0.0f};
+  long long c[2] = {-1, -1};
+#pragma unroll
   for (int t = 0; t < 2; ++t) {
     const Inj J = adjoint ? D.adj[t] : D.src[t];
-    float* u = t == 0 ? ux : uz;
-    float* du = t == 0 ? dux : duz;
-    float* Dd = t == 0 ? Dx : Dz;
-    const float* dtr = t == 0 ? dtr_i : dtr_j;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < J.np; p += gridDim.x * blockDim.x) {
-      float acc = 0.0f;
-      for (int e = J.ptr[p]; e < J.ptr[p + 1]; ++e) {
-        const int k = J.item[e];
-        acc += J.coef[e] * (tf[(long long)(it - 1) + (long long)D.nt * (t + 2LL * k)] * scale);
-      }
-      const long long c = J.lin[p];
-      const float v = acc * dtr[c];
-      u[so + c] += v;
-      du[so + c] += v;
-      if (Dd) Dd[so + c] += v;
+    if (!on || p >= J.np) continue;
+    c[t] = J.lin[p];
+    r[t] = (t == 0 ? dtr_i : dtr_j)[c[t]];
+    for (int e = J.ptr[p]; e < J.ptr[p + 1]; ++e) {
+      const int k = J.item[e];
+      acc[t] += J.coef[e] * (tf[(long long)(it - 1) + (long long)D.nt * (t + 2LL * k)] * scale);
     }
+  }
+  chain_wait();
+  chain_next();
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    if (c[t] < 0) continue;
+    float* u = (t == 0 ? ux : uz) + so + c[t];
+    float* du = (t == 0 ? dux : duz) + so + c[t];
+    float* Dd = t == 0 ? Dx : Dz;
+    *u = __fmaf_rn(acc[t], r[t], *u);
+    *du = __fmaf_rn(acc[t], r[t], *du);
+    if (Dd) Dd[so + c[t]] = __fmaf_rn(acc[t], r[t], Dd[so + c[t]]);
   }
 }
 
@@ -903,16 +919,23 @@ __global__ void k_el_record(const ShotDesc* __restrict__ desc, int it, long long
                             const float* __restrict__ uz) {
   const int s = blockIdx.y;
   const ShotDesc& D = desc[s];
-  if (it > D.nt) return;
+  const bool on = it <= D.nt;
   const float inv_scale = 1.0f / D.sf;
   const long long so = (long long)s * F;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < 2 * D.nrec; q += gridDim.x * blockDim.x) {
-    const int t = q & 1, r = q >> 1;
-    const float* u = (t == 0 ? ux : uz) + so;
-    float acc = 0.0f;
-    for (int e = D.rptr[t][r]; e < D.rptr[t][r + 1]; ++e) acc += D.rcoef[t][e] * u[D.rlin[t][e]];
-    D.tr[(long long)(it - 1) + (long long)D.nt * (t + 2LL * r)] = acc * inv_scale;
-  }
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;  // the grid covers every receiver component
+  const int t = q & 1, r = q >> 1;
+  const bool mine = on && q < 2 * D.nrec;
+  const float* u = (t == 0 ? ux : uz) + so;
+  const long long* lin = D.rlin[t];
+  const float* coef = D.rcoef[t];
+  const int e0 = mine ? D.rptr[t][r] : 0, e1 = mine ? D.rptr[t][r + 1] : 0;
+  chain_wait();
+  chain_next();
+  if (!mine) return;
+  float acc = 0.0f;
+#pragma unroll 8
+  for (int e = e0; e < e1; ++e) acc = __fmaf_rn(coef[e], u[lin[e]], acc);
+  D.tr[(long long)(it - 1) + (long long)D.nt * (t + 2LL * r)] = acc * inv_scale;
 }
 
 // The power of two 2^e with 2^e * max|C^-1 r| close to 2^20 (1 for a zero or
@@ -1112,6 +1135,8 @@ __global__ void __launch_bounds__(BX) k_el_corr(const CorrArgs A) {
 // D of row j) and takes the x neighbours from the adjacent lanes (loaded at
 // the warp edges); the z re-reads of neighbouring rows hit L1/L2.
 __global__ void __launch_bounds__(BX) k_el_corr4(const CorrArgs A) {
+  chain_next();
+  chain_wait();
   const Geo g = A.g;
   const int grp = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1390,17 +1415,7 @@ struct sw_elastic {
   DevMem d_scales;        // [0] the forward sources' common scale, [1] the adjoint source's scale
   DevMem d_ccts, d_partial2;  // CCTS descriptors and per-trace misfit terms
   DevMem d_gout, d_mout;  // gradient / misfit of the host-buffer path (stable addresses for the graphs)
-  // CUDA graphs of a group's whole gradient (forward, misfit, adjoint,
-  // reduction), keyed by what the captured launches depend on
-  long long gen = 0;  // bumped whenever a device buffer the kernels see is (re)allocated
-  std::map<std::vector<long long>, cudaGraphExec_t> graphs;
-  std::map<std::vector<long long>, int> graph_uses;
-  void drop_graphs() {
-    for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
-    graphs.clear();
-    graph_uses.clear();
-  }
-  ~sw_elastic() { drop_graphs(); }
+  GraphCache cache;  // a group's whole forward or gradient
 };
 
 namespace {
@@ -1410,50 +1425,7 @@ inline long long round_up(long long v, long long m) { return (v + m - 1) / m * m
 void ensure(sw_elastic* es, DevMem& m, size_t bytes, const char* what) {
   if (m.bytes >= bytes && m.p) return;
   dev_alloc(m, bytes, what, es->ctx->stream);
-  ++es->gen;
-}
-
-// Runs `work` (the device work of one group's gradient: launches, memsets and
-// device copies, no host synchronisation, no allocation) through a CUDA
-// graph: captured on the second call with `key`, replayed afterwards (at most
-// 32 graphs per simulation); directly while profiling or when the caller's
-// stream is itself being captured (the launches then join the caller's graph).
-template <typename Work>
-void el_run_graph(sw_elastic* es, std::vector<long long> key, Work&& work) {
-  cudaStream_t st = es->ctx->stream;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  check_cuda(cudaStreamIsCapturing(st, &cs), "cudaStreamIsCapturing");
-  if (es->ctx->prof.on || cs != cudaStreamCaptureStatusNone) {
-    work();
-    return;
-  }
-  key.push_back(es->gen);
-  auto it = es->graphs.find(key);
-  if (it == es->graphs.end()) {
-    if (es->graph_uses.size() > 4096) es->graph_uses.clear();
-    if (++es->graph_uses[key] < 2 || es->graphs.size() >= 32) {
-      work();
-      return;
-    }
-    check_cuda(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin stream capture");
-    try {
-      work();
-    } catch (...) {
-      cudaGraph_t g = nullptr;
-      cudaStreamEndCapture(st, &g);
-      if (g) cudaGraphDestroy(g);
-      cudaGetLastError();
-      throw;
-    }
-    cudaGraph_t g = nullptr;
-    check_cuda(cudaStreamEndCapture(st, &g), "end stream capture");
-    cudaGraphExec_t ex = nullptr;
-    const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
-    cudaGraphDestroy(g);
-    check_cuda(e, "graph instantiate");
-    it = es->graphs.emplace(key, ex).first;
-  }
-  check_cuda(cudaGraphLaunch(it->second, st), "graph launch");
+  ++es->cache.gen;
 }
 
 template <typename T>
@@ -1582,19 +1554,19 @@ void ensure_state(sw_elastic* es, int S, bool grad, int max_nt, int ngroups) {
     es->cap = S;
     es->cap_slots = 0;
     es->cap_ck = 0;
-    ++es->gen;
+    ++es->cache.gen;
   }
   if (grad) {
     const int K = es->gp.check_freq;
     const int M = (max_nt + K - 1) / K;
     const size_t slot_b = (size_t)K * 4 * es->cap * F * sizeof(float);
-    if (es->slots.bytes < slot_b) { dev_alloc(es->slots, slot_b, "gradient slots", es->ctx->stream); ++es->gen; }
+    if (es->slots.bytes < slot_b) { dev_alloc(es->slots, slot_b, "gradient slots", es->ctx->stream); ++es->cache.gen; }
     // per checkpoint: u, du (4 fields) and the 8 memory-variable strips of every shot
     const size_t ck_b = (size_t)std::max(M - 1, 1) * (4 * (size_t)es->cap * F + 4 * (size_t)es->cap * (es->xs + es->zs)) *
                         sizeof(float);
-    if (es->ck.bytes < ck_b) { dev_alloc(es->ck, ck_b, "checkpoints", es->ctx->stream); ++es->gen; }
+    if (es->ck.bytes < ck_b) { dev_alloc(es->ck, ck_b, "checkpoints", es->ctx->stream); ++es->cache.gen; }
     const size_t acc_b = (size_t)ngroups * 10 * F * sizeof(float);
-    if (es->acc.bytes < acc_b) { dev_alloc(es->acc, acc_b, "gradient accumulators", es->ctx->stream); ++es->gen; }
+    if (es->acc.bytes < acc_b) { dev_alloc(es->acc, acc_b, "gradient accumulators", es->ctx->stream); ++es->cache.gen; }
   }
 }
 
@@ -1889,7 +1861,7 @@ struct Run {
     }
     gx_src = (ns + 127) / 128;
     gx_adj = (na + 127) / 128;
-    gx_rec = (nr + 255) / 256;
+    gx_rec = (nr + 63) / 64;
   }
 
   Args args(bool adjoint) const {
@@ -1924,9 +1896,8 @@ struct Run {
     DevMem* f = es->st;
     cudaEvent_t ev = nullptr;
     es->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    k_el_inject_sigma<<<dim3(gx_src, S), 128, 0, st>>>(ddesc, it, es->g.F, f[4].as<float>(), f[5].as<float>(),
-                                                  f[6].as<float>());
-    check_cuda(cudaGetLastError(), "stress injection launch");
+    launch_chain("stress injection launch", k_el_inject_sigma, dim3(gx_src, S), dim3(128), st, ddesc, it, es->g.F,
+                 f[4].as<float>(), f[5].as<float>(), f[6].as<float>());
     es->ctx->prof.end(st, KK_SRCREC, ev);
   }
   void inject_force(int S, int it, bool adjoint, const float* adj_scale, float* sD[2]) {
@@ -1934,21 +1905,18 @@ struct Run {
     DevMem* f = adjoint ? es->ast : es->st;
     cudaEvent_t ev = nullptr;
     es->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    k_el_inject_force<<<dim3(adjoint ? gx_adj : gx_src, S), 128, 0, st>>>(ddesc, it, adjoint ? 1 : 0, adj_scale,
-                                                                         es->g.F,
-                                                                         f[0].as<float>(),
-                                                  f[1].as<float>(), f[2].as<float>(), f[3].as<float>(),
-                                                  sD ? sD[0] : nullptr, sD ? sD[1] : nullptr, es->dtr_i.as<float>(),
-                                                  es->dtr_j.as<float>());
-    check_cuda(cudaGetLastError(), "force injection launch");
+    launch_chain("force injection launch", k_el_inject_force, dim3(adjoint ? gx_adj : gx_src, S), dim3(128), st, ddesc, it,
+                 adjoint ? 1 : 0, adj_scale, es->g.F, f[0].as<float>(), f[1].as<float>(), f[2].as<float>(),
+                 f[3].as<float>(), sD ? sD[0] : nullptr, sD ? sD[1] : nullptr, es->dtr_i.as<float>(),
+                 es->dtr_j.as<float>());
     es->ctx->prof.end(st, KK_SRCREC, ev);
   }
   void record(int S, int it) {
     if (S <= 0) return;
     cudaEvent_t ev = nullptr;
     es->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    k_el_record<<<dim3(gx_rec, S), 256, 0, st>>>(ddesc, it, es->g.F, es->st[0].as<float>(), es->st[1].as<float>());
-    check_cuda(cudaGetLastError(), "record launch");
+    launch_chain("record launch", k_el_record, dim3(gx_rec, S), dim3(64), st, ddesc, it, es->g.F, es->st[0].as<float>(),
+                 es->st[1].as<float>());
     es->ctx->prof.end(st, KK_SRCREC, ev);
   }
 };
@@ -1994,13 +1962,13 @@ int launch_stencil(const sw_elastic* es, cudaStream_t st, Args a, int S, bool st
     a.tz = band_rows(es, S);
     const dim3 grid((unsigned)((es->g.nx + 511) / 512 * S), (unsigned)((es->g.nz + a.tz - 1) / a.tz));
     if (stress) {
-      k_el_stress4<<<grid, BX, 0, st>>>(a);
+      launch_chain("stress launch", k_el_stress4, grid, dim3(BX), st, a);
     } else if (es->split_disp) {  // ux and uz updates as two launches
-      k_el_disp4<0><<<grid, BX, 0, st>>>(a);
-      k_el_disp4<1><<<grid, BX, 0, st>>>(a);
+      launch_chain("displacement launch", k_el_disp4<0>, grid, dim3(BX), st, a);
+      launch_chain("displacement launch", k_el_disp4<1>, grid, dim3(BX), st, a);
       nk = 2;
     } else {
-      k_el_disp4<2><<<grid, BX, 0, st>>>(a);
+      launch_chain("displacement launch", k_el_disp4<2>, grid, dim3(BX), st, a);
     }
   } else if (es->tz == 16) {
     launch_scalar<16>(es, st, a, S, stress);
@@ -2255,11 +2223,21 @@ void elastic_forward(sw_elastic* es, int nshots, const sw_elastic_shot* shots, b
     R.size_grids(desc);
     R.any_mt = R.any_force = false;
     for (const auto& h : group) (shots[h.orig].kind == 0 ? R.any_mt : R.any_force) = true;
-    zero_state(es, S, false);
-    for (int it = 1; it <= group.front().nt; ++it) {
-      const int A = active_count(group, it);
-      full_step(R, A, it, true, KK_STENCIL, nullptr, nullptr);
-      if (es->snapevery > 0 && it % es->snapevery == 0) save_snapshots(es, group, A, it);
+    auto body = [&] {
+      zero_state(es, S, false);
+      for (int it = 1; it <= group.front().nt; ++it) {
+        const int A = active_count(group, it);
+        full_step(R, A, it, true, KK_STENCIL, nullptr, nullptr);
+        if (es->snapevery > 0 && it % es->snapevery == 0) save_snapshots(es, group, A, it);
+      }
+    };
+    if (es->snapevery > 0) {  // host copies inside the loop: no graph
+      body();
+    } else {
+      std::vector<long long> key = {0, S, es->tz, es->vec ? 1 : 0, es->split_disp ? 1 : 0, R.any_mt ? 1 : 0,
+                                    R.any_force ? 1 : 0, R.gx_src, R.gx_rec};
+      for (const auto& h : group) key.push_back(h.nt);
+      es->cache.run(es->ctx, key, body);
     }
     download_traces(es, shots, group, desc, on_device);
   }
@@ -2441,7 +2419,7 @@ void elastic_gradient(sw_elastic* es, int nshots, const sw_elastic_shot* shots, 
       const std::vector<float> sc = {sf_ref, 1.0f};
       upload(es, es->d_scales, sc, "source scales");
     }
-    std::vector<long long> key = {S, ntmax, es->tz, es->vec ? 1 : 0, es->split_disp ? 1 : 0, first_group ? 1 : 0,
+    std::vector<long long> key = {1, S, ntmax, es->tz, es->vec ? 1 : 0, es->split_disp ? 1 : 0, first_group ? 1 : 0,
                                   mute ? 1 : 0,
                                   R.gx_src, R.gx_adj, R.gx_rec, (long long)(uintptr_t)out[0],
                                   (long long)(uintptr_t)out[1], (long long)(uintptr_t)out[2],
@@ -2534,7 +2512,7 @@ void elastic_gradient(sw_elastic* es, int nshots, const sw_elastic_shot* shots, 
           es->ctx->prof.begin(st, KK_CORR, pts * (A * 24.0 + ng * 80.0), &ev);
           if (es->vec) {
             const dim3 grid4((g.nx + 511) / 512, g.nz, ng);
-            k_el_corr4<<<grid4, BX, 0, st>>>(c);
+            launch_chain("correlation launch", k_el_corr4, grid4, dim3(BX), st, c);
           } else {
             k_el_corr<<<grid, BX, 0, st>>>(c);
           }
@@ -2559,7 +2537,7 @@ void elastic_gradient(sw_elastic* es, int nshots, const sw_elastic_shot* shots, 
         es->ctx->prof.end(st, KK_OTHER, ev);
       }
     };
-    el_run_graph(es, key, body);
+    es->cache.run(es->ctx, key, body);
     download_traces(es, shots, group, desc, on_device);
     check_cuda(cudaStreamSynchronize(st), "elastic gradient group");
     first_group = false;

@@ -46,6 +46,8 @@
 #include <sstream>
 #include <vector>
 
+#include "chain.cuh"
+#include "graph.cuh"
 #include "internal.h"
 #include "ccts.cuh"
 #include "ff.cuh"
@@ -231,6 +233,8 @@ struct VdPBounds {
 
 template <bool CORR>
 __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs A) {
+  chain_next();
+  chain_wait();
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
@@ -357,6 +361,8 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
 // 1:nx x 1:nz-1); p rows j-1 .. j+2 in registers, the same split and the same
 // handling of the memory variables as k_vd_p.
 __global__ void __launch_bounds__(BX, 7) k_vd_v(const VArgs A) {
+  chain_next();
+  chain_wait();
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
@@ -485,6 +491,8 @@ __device__ __forceinline__ ff cpml_upd64(double* psi, double a, double b, ff dv)
 
 template <int TZ>
 __global__ void __launch_bounds__(BX) k_vd_p_hp(const HArgs A) {
+  chain_next();
+  chain_wait();
   const Geo g = A.g;
   const int s = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -579,6 +587,8 @@ __global__ void __launch_bounds__(BX) k_vd_p_hp(const HArgs A) {
 
 template <int TZ>
 __global__ void __launch_bounds__(BX) k_vd_v_hp(const HArgs A) {
+  chain_next();
+  chain_wait();
   const Geo g = A.g;
   const int s = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -703,11 +713,20 @@ struct ShotDesc {
 __global__ void k_vd_srcrec(const ShotDesc* __restrict__ desc, int it, long long F, float* p, int record,
                             float* plo) {
   const ShotDesc D = desc[blockIdx.x];
-  if (it > D.nt) return;  // block uniform
+  // this thread's first source point and receiver: the tables are read while the stencil still runs
+  const bool on = it <= D.nt;  // block uniform
+  const int t0 = threadIdx.x;
+  const bool src0 = on && t0 < D.nsp;
+  const long long slin0 = src0 ? D.sp_lin[t0] : 0, rlin0 = on && record && t0 < D.nrec ? D.rec_lin[t0] : 0;
+  const int sk0 = src0 ? D.sp_ptr[t0] : 0, sk1 = src0 ? D.sp_ptr[t0 + 1] : 0;
+  const float sv0 = sk1 > sk0 ? D.tf[(long long)(it - 1) + (long long)D.sp_ids[sk0] * D.nt] : 0.f;
+  chain_wait();
+  chain_next();
+  if (!on) return;
   float* pp = p + (long long)blockIdx.x * F;
   float* pl = plo ? plo + (long long)blockIdx.x * F : nullptr;  // compensated forward: low parts
-  for (int u = threadIdx.x; u < D.nsp; u += blockDim.x) {
-    const long long c = D.sp_lin[u];
+  for (int u = t0; u < D.nsp; u += blockDim.x) {
+    const long long c = u == t0 ? slin0 : D.sp_lin[u];
     if (pl) {
       ff v{pp[c], pl[c]};
       for (int k = D.sp_ptr[u]; k < D.sp_ptr[u + 1]; ++k)
@@ -717,13 +736,15 @@ __global__ void k_vd_srcrec(const ShotDesc* __restrict__ desc, int it, long long
       continue;
     }
     float v = pp[c];
-    for (int k = D.sp_ptr[u]; k < D.sp_ptr[u + 1]; ++k) v += D.tf[(long long)(it - 1) + (long long)D.sp_ids[k] * D.nt];
+    const int k0 = u == t0 ? sk0 : D.sp_ptr[u], k1 = u == t0 ? sk1 : D.sp_ptr[u + 1];
+    for (int k = k0; k < k1; ++k)
+      v += u == t0 && k == k0 ? sv0 : D.tf[(long long)(it - 1) + (long long)D.sp_ids[k] * D.nt];
     pp[c] = v;
   }
   if (!record) return;
   __syncthreads();
-  for (int r = threadIdx.x; r < D.nrec; r += blockDim.x) {
-    const long long q = D.rec_lin[r];
+  for (int r = t0; r < D.nrec; r += blockDim.x) {
+    const long long q = r == t0 ? rlin0 : D.rec_lin[r];
     D.tr[(long long)(it - 1) + (long long)r * D.nt] = pl ? __fadd_rn(pp[q], pl[q]) : pp[q];
   }
 }
@@ -734,15 +755,24 @@ __global__ void k_vd_srcrec(const ShotDesc* __restrict__ desc, int it, long long
 __global__ void k_vd_adjinj(const ShotDesc* __restrict__ desc, int it, long long F, float* ap, const float* pc,
                             const float* po, float* acc, float idt) {
   const ShotDesc D = desc[blockIdx.x];
-  if (it > D.nt) return;
+  const bool on = it <= D.nt;
+  const int t0 = threadIdx.x;
+  const bool rec0 = on && t0 < D.nrp;
+  const long long lin0 = rec0 ? D.rp_lin[t0] : 0;
+  const int rk0 = rec0 ? D.rp_ptr[t0] : 0, rk1 = rec0 ? D.rp_ptr[t0 + 1] : 0;
+  const float rv0 = rk1 > rk0 ? D.adj[(long long)(it - 1) + (long long)D.rp_ids[rk0] * D.nt] : 0.f;
+  chain_wait();
+  chain_next();
+  if (!on) return;
   const long long so = (long long)blockIdx.x * F;
   float* a = ap + so;
   float* g0 = acc + 3 * so;
-  for (int u = threadIdx.x; u < D.nrp; u += blockDim.x) {
-    const long long c = D.rp_lin[u];
+  for (int u = t0; u < D.nrp; u += blockDim.x) {
+    const long long c = u == t0 ? lin0 : D.rp_lin[u];
     float v = a[c], add = 0.0f;
-    for (int k = D.rp_ptr[u]; k < D.rp_ptr[u + 1]; ++k) {
-      const float s = D.adj[(long long)(it - 1) + (long long)D.rp_ids[k] * D.nt];
+    const int k0 = u == t0 ? rk0 : D.rp_ptr[u], k1 = u == t0 ? rk1 : D.rp_ptr[u + 1];
+    for (int k = k0; k < k1; ++k) {
+      const float s = u == t0 && k == k0 ? rv0 : D.adj[(long long)(it - 1) + (long long)D.rp_ids[k] * D.nt];
       v += s;
       add += s;
     }
@@ -965,6 +995,8 @@ struct sw_acoustic_vd {
   int hp_cap = 0;
   DevMem plo, vxl, vzl, xi64[2], psi64[2], m0l, m1xl, m1zl, d_cp64;
   std::vector<float> m0l_h, m1xl_h, m1zl_h;
+  DevMem d_gout, d_mout;  // gradient / misfit of the host-buffer path (stable addresses for the graphs)
+  GraphCache cache;       // a group's whole forward or gradient
 };
 
 namespace {
@@ -974,6 +1006,7 @@ inline long long round_up(long long v, long long m) { return (v + m - 1) / m * m
 void ensure(sw_acoustic_vd* vd, DevMem& m, size_t bytes, const char* what) {
   if (m.bytes >= bytes && m.p) return;
   dev_alloc(m, bytes, what, vd->ctx->stream);
+  ++vd->cache.gen;
 }
 
 template <typename T>
@@ -1062,6 +1095,7 @@ void ensure_state(sw_acoustic_vd* vd, int S, bool grad, int max_nt, int ngroups)
       vd->acc.release();
     }
     vd->cap = S;
+    ++vd->cache.gen;
   }
   if (vd->precision == 1 && vd->hp_cap < vd->cap) {
     for (DevMem* m : {&vd->plo, &vd->vxl, &vd->vzl})
@@ -1072,20 +1106,21 @@ void ensure_state(sw_acoustic_vd* vd, int S, bool grad, int max_nt, int ngroups)
       dev_alloc(vd->psi64[d], (size_t)vd->cap * w * sizeof(double), "VD memory variables (FP64)", st);
     }
     vd->hp_cap = vd->cap;
+    ++vd->cache.gen;
   }
   if (grad) {
     const int K = vd->gp.check_freq;
     const size_t cap = (size_t)vd->cap;
     // the slots' padding must stay zero: allocated zeroed, and no kernel writes outside the nodes
     const size_t slot_b = (size_t)(K + 1) * cap * F * sizeof(float);
-    if (vd->slots.bytes < slot_b) dev_alloc(vd->slots, slot_b, "VD pressure slots", st);
+    ensure(vd, vd->slots, slot_b, "VD pressure slots");
     const size_t ck_b = (size_t)std::max(checkpoints_needed(vd, max_nt), 1) *
                         (3 * cap * F + 2 * cap * (vd->xs + vd->zs)) * sizeof(float);
-    if (vd->ck.bytes < ck_b) dev_alloc(vd->ck, ck_b, "VD checkpoints", st);
+    ensure(vd, vd->ck, ck_b, "VD checkpoints");
     const size_t acc_b = cap * 3 * F * sizeof(float);
-    if (vd->acc.bytes < acc_b) dev_alloc(vd->acc, acc_b, "VD window sums", st);
+    ensure(vd, vd->acc, acc_b, "VD window sums");
     const size_t tot_b = (size_t)ngroups * 3 * F * sizeof(double);
-    if (vd->tot.bytes < tot_b) dev_alloc(vd->tot, tot_b, "VD gradient totals", st);
+    ensure(vd, vd->tot, tot_b, "VD gradient totals");
   }
 }
 
@@ -1412,14 +1447,11 @@ struct Run {
   }
   void launch_p(PArgs a, int S, bool corr) const {
     a.tz = band_rows(vd, S);
-    if (corr) k_vd_p<true><<<grid(S, a.tz), BX, 0, st>>>(a);
-    else k_vd_p<false><<<grid(S, a.tz), BX, 0, st>>>(a);
-    check_cuda(cudaGetLastError(), "pressure update launch");
+    launch_chain("pressure update launch", corr ? k_vd_p<true> : k_vd_p<false>, grid(S, a.tz), dim3(BX), st, a);
   }
   void launch_v(VArgs a, int S) const {
     a.tz = band_rows(vd, S);
-    k_vd_v<<<grid(S, a.tz), BX, 0, st>>>(a);
-    check_cuda(cudaGetLastError(), "velocity update launch");
+    launch_chain("velocity update launch", k_vd_v, grid(S, a.tz), dim3(BX), st, a);
   }
   // algorithmic bytes per node and shot: pressure R vx vz p, W p (16); velocity
   // R p vx vz, W vx vz (20); shared by the shots: fact_m0, fact_m1 x2 (12)
@@ -1464,16 +1496,14 @@ struct Run {
     const dim3 grid((vd->g.nx + 511) / 512, (vd->g.nz + TZ - 1) / TZ, S);
     cudaEvent_t ev = nullptr;
     vd->ctx->prof.begin(st, kind, fwd_bytes(S) + hp_extra_bytes(S), &ev);
-    k_vd_p_hp<TZ><<<grid, BX, 0, st>>>(a);
-    check_cuda(cudaGetLastError(), "compensated pressure update launch");
+    launch_chain("compensated pressure update launch", k_vd_p_hp<TZ>, grid, dim3(BX), st, a);
     vd->ctx->prof.end(st, kind, ev);
     vd->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    k_vd_srcrec<<<S, 128, 0, st>>>(ddesc, it, vd->g.F, pout, record ? 1 : 0, vd->plo.as<float>());
-    check_cuda(cudaGetLastError(), "injection launch");
+    launch_chain("injection launch", k_vd_srcrec, dim3(S), dim3(128), st, ddesc, it, vd->g.F, pout, record ? 1 : 0,
+                 vd->plo.as<float>());
     vd->ctx->prof.end(st, KK_SRCREC, ev);
     vd->ctx->prof.begin(st, kind, 0.0, &ev);
-    k_vd_v_hp<TZ><<<grid, BX, 0, st>>>(a);
-    check_cuda(cudaGetLastError(), "compensated velocity update launch");
+    launch_chain("compensated velocity update launch", k_vd_v_hp<TZ>, grid, dim3(BX), st, a);
     vd->ctx->prof.end(st, kind, ev);
   }
   // extra bytes of the compensated step per node and shot: R/W the low parts of p, vx, vz (24),
@@ -1491,8 +1521,8 @@ struct Run {
     launch_p(pargs(false, pin, pout), S, false);
     vd->ctx->prof.end(st, kind, ev);
     vd->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    k_vd_srcrec<<<S, 128, 0, st>>>(ddesc, it, vd->g.F, pout, record ? 1 : 0, nullptr);
-    check_cuda(cudaGetLastError(), "injection launch");
+    launch_chain("injection launch", k_vd_srcrec, dim3(S), dim3(128), st, ddesc, it, vd->g.F, pout, record ? 1 : 0,
+                 nullptr);
     vd->ctx->prof.end(st, KK_SRCREC, ev);
     vd->ctx->prof.begin(st, kind, 0.0, &ev);
     launch_v(vargs(false, pout), S);
@@ -1513,8 +1543,8 @@ struct Run {
     launch_p(a, S, true);
     vd->ctx->prof.end(st, KK_ADJOINT, ev, 2);
     vd->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    k_vd_adjinj<<<S, 128, 0, st>>>(ddesc, it, vd->g.F, ap, pc, po, vd->acc.as<float>(), a.idt);
-    check_cuda(cudaGetLastError(), "adjoint injection launch");
+    launch_chain("adjoint injection launch", k_vd_adjinj, dim3(S), dim3(128), st, ddesc, it, vd->g.F, ap, pc, po,
+                 vd->acc.as<float>(), a.idt);
     vd->ctx->prof.end(st, KK_SRCREC, ev);
   }
 };
@@ -1685,12 +1715,21 @@ void vd_forward(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, b
     std::vector<ShotDesc> desc;
     build_tables(vd, shots, group, on_device, false, desc);
     Run R{vd, vd->ctx->stream, vd->d_desc.as<ShotDesc>()};
-    zero_state(vd, S, false);
-    float* p = vd->st[0].as<float>();
-    for (int it = 1; it <= group.front().nt; ++it) {
-      const int A = active_count(group, it);
-      R.forward_step(A, it, p, p, true, KK_STENCIL);
-      if (vd->snapevery > 0 && it % vd->snapevery == 0) save_snapshots(vd, group, A, it);
+    auto body = [&] {
+      zero_state(vd, S, false);
+      float* p = vd->st[0].as<float>();
+      for (int it = 1; it <= group.front().nt; ++it) {
+        const int A = active_count(group, it);
+        R.forward_step(A, it, p, p, true, KK_STENCIL);
+        if (vd->snapevery > 0 && it % vd->snapevery == 0) save_snapshots(vd, group, A, it);
+      }
+    };
+    if (vd->snapevery > 0) {  // host copies inside the loop: no graph
+      body();
+    } else {
+      std::vector<long long> key = {0, S, vd->tz, vd->precision};
+      for (const auto& h : group) key.push_back(h.nt);
+      vd->cache.run(vd->ctx, key, body);
     }
     download_traces(vd, shots, group, desc, on_device);
   }
@@ -1739,16 +1778,15 @@ void vd_gradient(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, 
   const long long np = (long long)g.nx * g.nz;
   const long long F = g.F;
   const int K = vd->gp.check_freq;
-  DevMem dout, dmis;
   double* out[2] = {g_vp, g_rho};
   double* mout = misfit;
   if (!on_device) {
-    dev_alloc(dout, (size_t)2 * np * sizeof(double), "gradient output", st);
-    for (int q = 0; q < 2; ++q) out[q] = dout.as<double>() + q * np;
+    ensure(vd, vd->d_gout, (size_t)2 * np * sizeof(double), "gradient output");
+    for (int q = 0; q < 2; ++q) out[q] = vd->d_gout.as<double>() + q * np;
   }
   if (!on_device || !mout) {
-    dev_alloc(dmis, sizeof(double), "misfit output", st);
-    mout = dmis.as<double>();
+    ensure(vd, vd->d_mout, sizeof(double), "misfit output");
+    mout = vd->d_mout.as<double>();
   }
   const std::vector<HostShot> order = sorted_order(nshots, shots);
   bool first_group = true;
@@ -1813,36 +1851,11 @@ void vd_gradient(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, 
       copy(vd->xi[1].p, sp[2], (size_t)S * vd->zs * sizeof(float), "checkpoint load");
       copy(vd->psi[1].p, sp[3], (size_t)S * vd->zs * sizeof(float), "checkpoint load");
     };
-    // forward: in place up to the last window, then p of each step into the slots
-    zero_state(vd, S, false);
-    const int last_start = (M - 1) * K;
-    float* p = vd->st[0].as<float>();
-    for (int it = 1; it <= ntmax; ++it) {
-      const int A = active_count(group, it);
-      if (it < last_start) R.forward_step(A, it, p, p, true, KK_STENCIL);
-      else if (it == last_start) R.forward_step(A, it, p, slot(0), true, KK_STENCIL);
-      else R.forward_step(A, it, slot(it - last_start - 1), slot(it - last_start), true, KK_STENCIL);
-      if (it % K == 0 && it / K <= M - 2) save_ck(it / K);
-    }
-    download_traces(vd, shots, group, desc, on_device);
-    // misfit and prescaled adjoint sources
     const int nblk = 64;
     ensure(vd, vd->d_partial, (size_t)nblk * S * sizeof(double), "misfit partials");
+    size_t smem = 0;
+    int crec = 0;
     {
-      bool any_dense = false;
-      for (const auto& d : desc) any_dense = any_dense || d.icd;
-      cudaEvent_t ev = nullptr;
-      vd->ctx->prof.begin(st, KK_OTHER, 0.0, &ev);
-      if (any_dense) {
-        k_vd_residual_dense<<<dim3(nblk, S), 256, 0, st>>>(R.ddesc);
-        check_cuda(cudaGetLastError(), "residual launch");
-        for (const auto& d : desc)
-          if (d.icd) dense_invcov(vd->ctx, d.nt, d.nrec, d.icd, d.resid, const_cast<float*>(d.cres));
-      }
-      k_vd_misfit<<<dim3(nblk, S), 256, 0, st>>>(R.ddesc, vd->m0.as<float>(), vd->d_partial.as<double>());
-      check_cuda(cudaGetLastError(), "misfit launch");
-      k_vd_misfit_sum<<<1, 256, 0, st>>>(vd->d_partial.as<double>(), nblk * S, mout, first_group ? 0 : 1);
-      check_cuda(cudaGetLastError(), "misfit sum launch");
       // CCTS shots: misfit and adjoint source from the cross-correlation time shift
       std::vector<int> kind(S), ntv(S), nrec(S);
       std::vector<double> mdt(S);
@@ -1861,40 +1874,8 @@ void vd_gradient(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, 
         rl[k] = desc[k].rec_lin;
       }
       ensure(vd, vd->d_ccts, (size_t)S * sizeof(CctsShot), "CCTS table");
-      size_t smem = 0;
-      const int crec = upload_ccts(vd->ctx, vd->d_ccts.as<CctsShot>(), kind, mdt, ntv, nrec, tr, obs, adj, rl, &smem);
-      if (crec) {
-        ensure(vd, vd->d_partial2, (size_t)crec * S * sizeof(double), "CCTS partials");
-        k_ccts<<<dim3(crec, S), CCTS_THREADS, smem, st>>>(vd->d_ccts.as<CctsShot>(), vd->m0.as<float>(),
-                                                          vd->d_partial2.as<double>());
-        check_cuda(cudaGetLastError(), "CCTS misfit launch");
-        k_vd_misfit_sum<<<1, 256, 0, st>>>(vd->d_partial2.as<double>(), crec * S, mout, 1);
-        check_cuda(cudaGetLastError(), "CCTS misfit sum launch");
-      }
-      vd->ctx->prof.end(st, KK_OTHER, ev);
-    }
-    // adjoint with recompute, fused correlation and window flushes
-    zero_state(vd, S, true);
-    check_cuda(cudaMemsetAsync(vd->acc.p, 0, (size_t)S * 3 * F * sizeof(float), st), "window sums clear");
-    check_cuda(cudaMemsetAsync(vd->tot.p, 0, (size_t)ngroups * 3 * F * sizeof(double), st), "totals clear");
-    const int fblocks = (int)std::min<long long>((3 * (F / 4) + 255) / 256, 8192);
-    for (int m = M - 1; m >= 0; --m) {
-      const int t0 = m * K + 1, t1 = std::min((m + 1) * K, ntmax);
-      if (m < M - 1) {
-        load_ck(m);
-        for (int t = t0; t <= t1; ++t)
-          R.forward_step(active_count(group, t), t, slot(t - t0), slot(t - t0 + 1), false, KK_RECOMPUTE);
-      }
-      for (int it = t1; it >= t0; --it) R.adjoint_step(active_count(group, it), it, slot(it - t0 + 1), slot(it - t0));
-      const int Aw = active_count(group, t0);
-      if (Aw > 0) {
-        cudaEvent_t ev = nullptr;
-        vd->ctx->prof.begin(st, KK_OTHER, 0.0, &ev);
-        k_vd_flush<<<fblocks, 256, 0, st>>>(g, Aw, gsize, vd->acc.as<float>(), vd->tot.as<double>());
-        check_cuda(cudaGetLastError(), "window flush launch");
-        check_cuda(cudaMemsetAsync(vd->acc.p, 0, (size_t)Aw * 3 * F * sizeof(float), st), "window sums clear");
-        vd->ctx->prof.end(st, KK_OTHER, ev);
-      }
+      crec = upload_ccts(vd->ctx, vd->d_ccts.as<CctsShot>(), kind, mdt, ntv, nrec, tr, obs, adj, rl, &smem);
+      if (crec) ensure(vd, vd->d_partial2, (size_t)crec * S * sizeof(double), "CCTS partials");
     }
     // mute balls per group (= per shot when muting)
     std::vector<MuteBall> balls;
@@ -1926,18 +1907,89 @@ void vd_gradient(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, 
       upload(vd, vd->d_balls, balls, "mute balls");
       upload(vd, vd->d_ball_ptr, bptr, "mute balls");
     }
-    {
-      cudaEvent_t ev = nullptr;
-      vd->ctx->prof.begin(st, KK_OTHER, 0.0, &ev);
-      const int blocks = (int)std::min<long long>((np + 255) / 256, 8192);
-      k_vd_reduce<<<blocks, 256, 0, st>>>(g, ngroups, vd->tot.as<double>(), vd->vp_d.as<double>(), vd->rho_d.as<double>(),
-                                          vd->interp, vd->prm.h[0], vd->prm.h[1],
-                                          mute ? vd->d_balls.as<MuteBall>() : nullptr,
-                                          mute ? vd->d_ball_ptr.as<int>() : nullptr, out[0], out[1],
-                                          first_group ? 0 : 1);
-      check_cuda(cudaGetLastError(), "gradient reduction launch");
-      vd->ctx->prof.end(st, KK_OTHER, ev);
-    }
+    // the group's device work -- forward, misfit, adjoint with recompute and
+    // correlation, reduction -- as one CUDA graph
+    auto body = [&] {
+      // forward: in place up to the last window, then p of each step into the slots
+      zero_state(vd, S, false);
+      const int last_start = (M - 1) * K;
+      float* p = vd->st[0].as<float>();
+      for (int it = 1; it <= ntmax; ++it) {
+        const int A = active_count(group, it);
+        if (it < last_start) R.forward_step(A, it, p, p, true, KK_STENCIL);
+        else if (it == last_start) R.forward_step(A, it, p, slot(0), true, KK_STENCIL);
+        else R.forward_step(A, it, slot(it - last_start - 1), slot(it - last_start), true, KK_STENCIL);
+        if (it % K == 0 && it / K <= M - 2) save_ck(it / K);
+      }
+      // misfit and prescaled adjoint sources
+      {
+        bool any_dense = false;
+        for (const auto& d : desc) any_dense = any_dense || d.icd;
+        cudaEvent_t ev = nullptr;
+        vd->ctx->prof.begin(st, KK_OTHER, 0.0, &ev);
+        if (any_dense) {
+          k_vd_residual_dense<<<dim3(nblk, S), 256, 0, st>>>(R.ddesc);
+          check_cuda(cudaGetLastError(), "residual launch");
+          for (const auto& d : desc)
+            if (d.icd) dense_invcov(vd->ctx, d.nt, d.nrec, d.icd, d.resid, const_cast<float*>(d.cres));
+        }
+        k_vd_misfit<<<dim3(nblk, S), 256, 0, st>>>(R.ddesc, vd->m0.as<float>(), vd->d_partial.as<double>());
+        check_cuda(cudaGetLastError(), "misfit launch");
+        k_vd_misfit_sum<<<1, 256, 0, st>>>(vd->d_partial.as<double>(), nblk * S, mout, first_group ? 0 : 1);
+        check_cuda(cudaGetLastError(), "misfit sum launch");
+        if (crec) {
+          k_ccts<<<dim3(crec, S), CCTS_THREADS, smem, st>>>(vd->d_ccts.as<CctsShot>(), vd->m0.as<float>(),
+                                                            vd->d_partial2.as<double>());
+          check_cuda(cudaGetLastError(), "CCTS misfit launch");
+          k_vd_misfit_sum<<<1, 256, 0, st>>>(vd->d_partial2.as<double>(), crec * S, mout, 1);
+          check_cuda(cudaGetLastError(), "CCTS misfit sum launch");
+        }
+        vd->ctx->prof.end(st, KK_OTHER, ev);
+      }
+      // adjoint with recompute, fused correlation and window flushes
+      zero_state(vd, S, true);
+      check_cuda(cudaMemsetAsync(vd->acc.p, 0, (size_t)S * 3 * F * sizeof(float), st), "window sums clear");
+      check_cuda(cudaMemsetAsync(vd->tot.p, 0, (size_t)ngroups * 3 * F * sizeof(double), st), "totals clear");
+      const int fblocks = (int)std::min<long long>((3 * (F / 4) + 255) / 256, 8192);
+      for (int m = M - 1; m >= 0; --m) {
+        const int t0 = m * K + 1, t1 = std::min((m + 1) * K, ntmax);
+        if (m < M - 1) {
+          load_ck(m);
+          for (int t = t0; t <= t1; ++t)
+            R.forward_step(active_count(group, t), t, slot(t - t0), slot(t - t0 + 1), false, KK_RECOMPUTE);
+        }
+        for (int it = t1; it >= t0; --it) R.adjoint_step(active_count(group, it), it, slot(it - t0 + 1), slot(it - t0));
+        const int Aw = active_count(group, t0);
+        if (Aw > 0) {
+          cudaEvent_t ev = nullptr;
+          vd->ctx->prof.begin(st, KK_OTHER, 0.0, &ev);
+          k_vd_flush<<<fblocks, 256, 0, st>>>(g, Aw, gsize, vd->acc.as<float>(), vd->tot.as<double>());
+          check_cuda(cudaGetLastError(), "window flush launch");
+          check_cuda(cudaMemsetAsync(vd->acc.p, 0, (size_t)Aw * 3 * F * sizeof(float), st), "window sums clear");
+          vd->ctx->prof.end(st, KK_OTHER, ev);
+        }
+      }
+      {
+        cudaEvent_t ev = nullptr;
+        vd->ctx->prof.begin(st, KK_OTHER, 0.0, &ev);
+        const int blocks = (int)std::min<long long>((np + 255) / 256, 8192);
+        k_vd_reduce<<<blocks, 256, 0, st>>>(g, ngroups, vd->tot.as<double>(), vd->vp_d.as<double>(), vd->rho_d.as<double>(),
+                                            vd->interp, vd->prm.h[0], vd->prm.h[1],
+                                            mute ? vd->d_balls.as<MuteBall>() : nullptr,
+                                            mute ? vd->d_ball_ptr.as<int>() : nullptr, out[0], out[1],
+                                            first_group ? 0 : 1);
+        check_cuda(cudaGetLastError(), "gradient reduction launch");
+        vd->ctx->prof.end(st, KK_OTHER, ev);
+      }
+    };
+    std::vector<long long> key = {1, S, ntmax, vd->tz, vd->precision, first_group ? 1 : 0, mute ? 1 : 0, crec,
+                                  (long long)smem, (long long)(uintptr_t)out[0], (long long)(uintptr_t)out[1],
+                                  (long long)(uintptr_t)mout};
+    for (const auto& h : group) key.push_back(h.nt);
+    for (int k = 0; k < S; ++k)  // the dense products' operands are launch arguments
+      if (desc[k].icd) key.insert(key.end(), {k, desc[k].nrec, (long long)(uintptr_t)desc[k].icd});
+    vd->cache.run(vd->ctx, key, body);
+    download_traces(vd, shots, group, desc, on_device);
     check_cuda(cudaStreamSynchronize(st), "VD gradient group");
     first_group = false;
   }
