@@ -1129,6 +1129,18 @@ int block_rows3d(const sw_wavesim* ws) { return (ws->variant & 3) == 2 ? 8 : 4; 
 
 enum { TZ_FORWARD = 0, TZ_RECOMPUTE = 1, TZ_ADJOINT = 2 };
 
+// 2D launches with fewer than 16 rows (of 128 points) per SM in all: one row
+// per warp, 3 resident blocks per SM (168 registers, nothing spilled) and no
+// separate x-strip blocks, whose threads take longer than a row.  Latency of
+// one row is all there is to win (one shot of 201 x 201: 5.2 us per step
+// against 7.0 with the strips split off in 2-row bands, 5.6 at 4 blocks per
+// SM; 2 shots of 301 x 187, gradient: 6.3 against 8.3 ms; one of 801 x 801, 37
+// rows per SM: 38.2 against 31.1).
+bool small_2d(const sw_wavesim* ws, int S) {
+  const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
+  return ws->N == 2 && (long long)S * ((ws->P + 127) / 128) * (ws->n[1] - 2) < 16LL * sms;
+}
+
 StepCtx make_step_ctx(sw_wavesim* ws, int S, int kind = TZ_FORWARD) {
   StepCtx c{ws, 0, 0, 1, 0};
   const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
@@ -1150,12 +1162,12 @@ StepCtx make_step_ctx(sw_wavesim* ws, int S, int kind = TZ_FORWARD) {
       // warp's rows run one after the other, so smaller launches take
       // shorter bands: 4 rows below 256 warps per SM (16 shots of 2001 x 801,
       // gradient: 109.8 against 111.1 ms; one of 801 x 801: 35.2 against 43.6
-      // with 8 and 37.2 with 2), 2 below 8 (one of 201 x 201: 8.5 us per step
-      // against 9.2 with 4 and 12.8 with 8; single rows run 8.6)
+      // with 8 and 37.2 with 2), 2 below 8, single rows for small_2d
       const long long wx = (ws->P + 127) / 128;
       TZ = 8;
       if (S * wx * ((nint + 7) / 8) < 256LL * sms) TZ = 4;
       if (S * wx * ((nint + 3) / 4) < 8LL * sms) TZ = 2;
+      if (small_2d(ws, S)) TZ = 1;
     } else if (ws->N == 3 && ws->split3d) {
       // 16 planes, 8 or 4 while the inner rows make fewer than 8 blocks per SM
       // (2 x 183 x 157 x 141: 35.2 ms per 300 steps with 16 planes, 45 with 32)
@@ -1326,18 +1338,28 @@ void enable_pair_carveout() {
   done_for_device = dev;
 }
 
+// Blocks of 128 lane groups of the x strips (xstrip_item).
+long long xstrip_blocks(const StepArgs& a) {
+  int nl, xr, ng;
+  xstrip_groups(a.n0, a.halo, a.P, nl, xr, ng);
+  return ((long long)ng * (a.n1 - 2) * a.nshots + 127) / 128;
+}
+
 // The 2D one-step stencil of 4-warp blocks with the x strips split off:
 // `blocks` main blocks for the lanes outside the x strips, then one block
 // per 128 lane groups of the x strips (rows x shots), which run in the tail
 // of the launch (79.5 against 78.4 Gpts/s as a second launch on the 64-shot
-// headline).  Returns the number of kernels launched.
+// headline).  A small launch (small_2d) takes the one-kernel form with
+// registers for every load of a row to be in flight.  Returns the number of
+// kernels launched.
 template <int MODE>
-int launch_2d_xsplit(long long blocks, cudaStream_t st, const StepArgs& a) {
-  int nl, xr, ng;
-  xstrip_groups(a.n0, a.halo, a.P, nl, xr, ng);
-  const long long items = (long long)ng * (a.n1 - 2) * a.nshots;
-  launch_chain("stencil launch", k_ac2d_step<MODE, 4, 1, true>, dim3((unsigned)(blocks + (items + 127) / 128)), dim3(128),
-               st, a);
+int launch_2d_xsplit(long long blocks, bool small, cudaStream_t st, const StepArgs& a) {
+  if (small) {
+    launch_chain("stencil launch", k_ac2d_step<MODE, 4, 1, false, 3>, dim3((unsigned)blocks), dim3(128), st, a);
+    return 1;
+  }
+  launch_chain("stencil launch", k_ac2d_step<MODE, 4, 1, true>, dim3((unsigned)(blocks + xstrip_blocks(a))), dim3(128), st,
+               a);
   return 1;
 }
 
@@ -1407,7 +1429,7 @@ struct Launcher {
         enable_cpa_carveout<MODE>();
         k_ac2d_cpa<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       } else if (nw == 4 && ws->xsplit)
-        nk = launch_2d_xsplit<MODE>(blocks, st, a);
+        nk = launch_2d_xsplit<MODE>(blocks, small_2d(ws, a.nshots), st, a);
       else if (nw == 4)
         k_ac2d_step<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       else if (nw == 8)
@@ -1433,7 +1455,7 @@ struct Launcher {
       }
       if (launched) {
       } else if (nw == 4 && ws->xsplit)
-        nk = launch_2d_xsplit<MODE>(blocks, st, a);
+        nk = launch_2d_xsplit<MODE>(blocks, small_2d(ws, a.nshots), st, a);
       else if (nw == 4)
         k_ac2d_step<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       else if (nw == 8)

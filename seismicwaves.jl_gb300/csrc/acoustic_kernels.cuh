@@ -624,9 +624,9 @@ struct Ac2dBounds {
 // XS: the lanes that meet an x strip store nothing in the main blocks (the
 // first nshots x tiles_x x tiles_z); the blocks after them take the lane
 // groups of the x strips, one per thread (xstrip_item), so that this work
-// fills the tail of the launch.
-template <int MODE, int NW, int DP = 1, bool XS = false>
-__global__ void __launch_bounds__(32 * NW, (Ac2dBounds<MODE, NW>::MINB - (DP - 1))) k_ac2d_step(const StepArgs A) {
+// fills the tail of the launch.  MB: resident blocks per SM.
+template <int MODE, int NW, int DP = 1, bool XS = false, int MB = Ac2dBounds<MODE, NW>::MINB - (DP - 1)>
+__global__ void __launch_bounds__(32 * NW, MB) k_ac2d_step(const StepArgs A) {
   constexpr unsigned FULL = 0xffffffffu;
   chain_next();
   chain_wait();

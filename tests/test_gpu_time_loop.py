@@ -5,6 +5,7 @@ chained launches) gives, bit for bit; shots of different length in a batch
 import numpy as np
 import pytest
 
+import cases as C
 import elastic_cases as E
 import vd_cases as V
 from vd_cases import sw
@@ -55,3 +56,29 @@ def test_replayed_time_loop_is_bitwise_a_first_call(ctx, kind, grad):
     got = _run(ctx, kind, grad, [1.0, 1.0, 1.1, 0.9])
     assert all(np.abs(w).max() > 0 for w in want)
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("nx,nz,shots", [(45, 45, 1), (130, 90, 2), (700, 400, 1), (700, 410, 2), (257, 190, 9)])
+def test_small_2d_launches_are_bitwise_the_split_ones(nx, nz, shots):
+    """Constant density: one-row launches of small batches (below 16 rows of 128 points per SM; the sizes lie on
+    both sides) against explicit 8-row bands with the x strips in the main blocks (variant bit 18)."""
+    h = (9.0, 8.0)
+    vp = C.smooth_model((nx, nz), 1700.0, 3200.0, nx)
+    case = C.Case(vp=vp, h=h, dt=C.stable_dt(vp, h), halo=9, freetop=bool(nx % 2))
+    ex = [hh * (n - 1) for n, hh in zip(vp.shape, h)]
+    sh = []
+    for k in range(shots):  # receivers a few points off the source: 70 steps carry a wave about 25 points
+        x, z = (0.2 + 0.06 * k) * ex[0], 0.3 * ex[1]
+        sh.append(C.make_shot(h, ex, 70 - 5 * k, case.dt, 25.0, [[x, z]], [[x + 9.0 * q, z + 16.0] for q in range(9)]))
+    for s in sh:
+        s.observed = 1e-3 * np.cos(np.arange(s.nt * 9.0)).reshape(s.nt, 9)
+    out = []
+    for variant, bands in ((0, None), (262144, (8, 8, 8))):
+        run = C.GpuRun(sw, case, gradient=True, check_freq=8, variant=variant)
+        if bands:
+            run.ctx.check(run.ctx.lib.sw_wavesim_set_band_heights(run.h, *bands), "band heights")
+        g, m, t = run.gradient(sh)
+        run.close()
+        out.append([g, np.array(m)] + list(t))
+    assert np.abs(out[0][0]).max() > 0
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
