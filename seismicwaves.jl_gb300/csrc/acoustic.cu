@@ -1190,8 +1190,12 @@ StepCtx make_step_ctx(sw_wavesim* ws, int S, int kind = TZ_FORWARD) {
 }
 
 // Compensated forward step (k_ac_hp): 2D blocks of 512 x points, 3D blocks of
-// 128 x points and 4 y rows; bands of 32 rows, shorter while the launch would
-// have fewer than 8 blocks per SM, 4 rows at least.
+// 128 x points and 4 y rows.  2D bands of 4 rows, single rows while the launch
+// would have fewer than 24 blocks per SM (the strip rows, FP64-bound, then
+// spread over the SMs: 2 shots of 801 x 801 37.8 us per step against 47.3 with
+// 4-row bands; 32 of 901 x 455 212 with 4 rows, 244 with 1, 226 with 8).  3D
+// bands of 32 rows, shorter while the launch would have fewer than 8 blocks
+// per SM, 4 rows at least.
 StepCtx make_hp_ctx(sw_wavesim* ws, int S) {
   StepCtx c{ws, 0, 0, 1, 0};
   const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
@@ -1203,7 +1207,9 @@ StepCtx make_hp_ctx(sw_wavesim* ws, int S) {
   }
   const int nint = ws->n[ws->N - 1] - 2;
   int TZ = 32;
-  while (TZ > 4 && (long long)S * c.tiles_x * c.tiles_y * ((nint + TZ - 1) / TZ) < 8LL * sms) TZ /= 2;
+  if (ws->N == 2) TZ = (long long)S * c.tiles_x * ((nint + 3) / 4) < 24LL * sms ? 1 : 4;
+  else
+    while (TZ > 4 && (long long)S * c.tiles_x * c.tiles_y * ((nint + TZ - 1) / TZ) < 8LL * sms) TZ /= 2;
   c.TZ = TZ;
   c.tiles_z = (nint + TZ - 1) / TZ;
   return c;
@@ -1338,7 +1344,7 @@ void enable_pair_carveout() {
   done_for_device = dev;
 }
 
-// Blocks of 128 lane groups of the x strips (xstrip_item).
+// Blocks of 128 lane groups of the x strips (xstrip_item, hp_xstrip_item).
 long long xstrip_blocks(const StepArgs& a) {
   int nl, xr, ng;
   xstrip_groups(a.n0, a.halo, a.P, nl, xr, ng);
@@ -1416,7 +1422,8 @@ struct Launcher {
     if constexpr (MODE == MODE_FWD || MODE == MODE_FWD_D) {
       if (ws->precision == 1 && !recompute) {  // compensated forward (context from make_hp_ctx)
         if (ws->N == 2)
-          launch_chain("compensated stencil launch", k_ac_hp<MODE, 2>, dim3((unsigned)blocks), dim3(128), st, a);
+          launch_chain("compensated stencil launch", k_ac_hp<MODE, 2>, dim3((unsigned)(blocks + xstrip_blocks(a))), dim3(128),
+                       st, a);
         else
           launch_chain("compensated stencil launch", k_ac_hp<MODE, 3>, dim3((unsigned)blocks), dim3(128), st, a);
         ws->ctx->prof.end(st, kind, ev);

@@ -2129,77 +2129,158 @@ __device__ __forceinline__ Strip64 strip64_io(const StepArgs& A, int d, int shot
   return s;
 }
 __device__ __forceinline__ double ff_d(ff a) { return (double)a.hi + (double)a.lo; }
-__device__ __forceinline__ ff cpml_axis_corr64(ff d2, ff pl, ff p0, ff pr, int x, int n, int halo, double ih,
-                                               const Strip64& s) {
-  int qr;
-  bool first;
-  if (x < halo) {
-    qr = x;
-    first = (x == 1);
-  } else if (x >= n - halo) {
-    qr = x + 1 - n + 2 * halo;
-    first = (x == n - halo);
-  } else {
-    return ff{0.f, 0.f};
-  }
-  const int ql = qr - 1;
-  const long long il = s.psi_base + (long long)ql * s.psi_step;
-  const long long ir = s.psi_base + (long long)qr * s.psi_step;
+// one point: psi left and right of it (new values back through them) and xi,
+// loaded by the caller with the row
+__device__ __forceinline__ ff cpml_corr64(ff d2, ff pl, ff p0, ff pr, double& psil, double& psir, double& xi, double al,
+                                          double bl, double ar, double br, double a, double b, double ih) {
   const double P0 = ff_d(p0);
-  const double oldl = s.psi_in[il];
-  const double oldr = s.psi_in[ir];
-  const double newl = s.bh[ql] * oldl + s.ah[ql] * ((P0 - ff_d(pl)) * ih);
-  const double newr = s.bh[qr] * oldr + s.ah[qr] * ((ff_d(pr) - P0) * ih);
-  s.psi_out[ir] = newr;
-  if (s.ck_psi) s.ck_psi[ir] = (float)oldr;
-  if (first) {
-    s.psi_out[il] = newl;
-    if (s.ck_psi) s.ck_psi[il] = (float)oldl;
-  }
-  const double dpsi = (newr - newl) * ih;
-  const long long iq = s.xi_base + (long long)qr * s.xi_step;
-  const double xo = s.xi_in[iq];
-  if (s.ck_xi) s.ck_xi[iq] = (float)xo;
-  const double xn = s.b[qr] * xo + s.a[qr] * (ff_d(d2) + dpsi);
-  s.xi_out[iq] = xn;
-  const double corr = dpsi + xn;
+  psil = bl * psil + al * ((P0 - ff_d(pl)) * ih);
+  psir = br * psir + ar * ((ff_d(pr) - P0) * ih);
+  const double dpsi = (psir - psil) * ih;
+  xi = b * xi + a * (ff_d(d2) + dpsi);
+  const double corr = dpsi + xi;
   const float hi = (float)corr;
   return ff{hi, (float)(corr - (double)hi)};
+}
+// One axis whose strip cell is the same for the thread's four points (y, z).
+__device__ __forceinline__ bool strip_cell(int v, int n, int H, int& qr, bool& first) {
+  if (v < H) {
+    qr = v;
+    first = v == 1;
+    return true;
+  }
+  if (v >= n - H) {
+    qr = v + 1 - n + 2 * H;
+    first = v == n - H;
+    return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void ld4d(double (&v)[4], const double* p) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void st4d(double* p, const double (&v)[4]) {
+  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+  *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
+}
+__device__ __forceinline__ void st4f(float* p, const double (&v)[4]) {
+  const float w[4] = {(float)v[0], (float)v[1], (float)v[2], (float)v[3]};
+  st4(p, w);
+}
+// The correction of the four points of a row in the strip of axis y or z
+// (cell qr), added to t; base = the row's offset in the strip arrays.
+__device__ __forceinline__ void cpml_corr64_4(ff (&t)[4], const float (&lh)[4], const float (&ll)[4],
+                                              const float (&ch)[4], const float (&cl)[4], const float (&rh)[4],
+                                              const float (&rl)[4], int qr, bool first, double ih, const Strip64& s) {
+  const long long il = s.psi_base + (long long)(qr - 1) * s.psi_step, ir = s.psi_base + (long long)qr * s.psi_step;
+  const long long iq = s.xi_base + (long long)qr * s.xi_step;
+  double pl[4], pr[4], xi[4];
+  ld4d(pl, s.psi_in + il);
+  ld4d(pr, s.psi_in + ir);
+  ld4d(xi, s.xi_in + iq);
+  if (s.ck_psi) {
+    st4f(s.ck_psi + ir, pr);
+    if (first) st4f(s.ck_psi + il, pl);
+  }
+  if (s.ck_xi) st4f(s.ck_xi + iq, xi);
+  const double al = s.ah[qr - 1], bl = s.bh[qr - 1], ar = s.ah[qr], br = s.bh[qr], a = s.a[qr], b = s.b[qr];
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    t[e] = ff_add(t[e], cpml_corr64(t[e], ff{lh[e], ll[e]}, ff{ch[e], cl[e]}, ff{rh[e], rl[e]}, pl[e], pr[e], xi[e], al,
+                                    bl, ar, br, a, b, ih));
+  st4d(s.psi_out + ir, pr);
+  if (first) st4d(s.psi_out + il, pl);
+  st4d(s.xi_out + iq, xi);
+}
+// The correction of four consecutive points along x (see cpml_axis_x4).
+__device__ __forceinline__ void cpml_corr64_x4(ff (&t)[4], const float (&ch)[4], const float (&cl)[4], ff left, ff right,
+                                               int x0, int n, int H, double ih, const XCells& xc, const Strip64& s) {
+  double psi[5], xi[4];
+  int q[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) q[e] = x0 + e < H ? x0 + e : x0 + e + 1 - n + 2 * H;
+  // psi[k] is the half node left of point k (k = 4: right of point 3)
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const bool l = k < 4 && (xc.in >> (k < 4 ? k : 0) & 1), r = k > 0 && (xc.in >> (k > 0 ? k - 1 : 0) & 1);
+    psi[k] = r ? s.psi_in[s.psi_base + q[k > 0 ? k - 1 : 0]] : l ? s.psi_in[s.psi_base + q[k < 4 ? k : 0] - 1] : 0.0;
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) xi[e] = (xc.in >> e & 1) ? s.xi_in[s.xi_base + q[e]] : 0.0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (xc.in >> e & 1) {
+      const bool first = x0 + e == 1 || x0 + e == n - H;
+      const int qr = q[e];
+      double pl = psi[e], pr = psi[e + 1], x = xi[e];
+      if (s.ck_psi) {
+        s.ck_psi[s.psi_base + qr] = (float)pr;
+        if (first) s.ck_psi[s.psi_base + qr - 1] = (float)pl;
+      }
+      if (s.ck_xi) s.ck_xi[s.xi_base + qr] = (float)x;
+      const ff c{ch[e], cl[e]};
+      const ff l = e == 0 ? left : ff{ch[e > 0 ? e - 1 : 0], cl[e > 0 ? e - 1 : 0]};
+      const ff r = e == 3 ? right : ff{ch[e < 3 ? e + 1 : 3], cl[e < 3 ? e + 1 : 3]};
+      t[e] = ff_add(t[e], cpml_corr64(t[e], l, c, r, pl, pr, x, s.ah[qr - 1], s.bh[qr - 1], s.ah[qr], s.bh[qr], s.a[qr],
+                                      s.b[qr], ih));
+      s.psi_out[s.psi_base + qr] = pr;
+      if (first) s.psi_out[s.psi_base + qr - 1] = pl;
+      s.xi_out[s.xi_base + qr] = x;
+    }
 }
 
 // One warp = 128 x points (4 per thread) of one row (2D) or of one y row
 // (3D), marching a band of TZ rows of the last axis; 4 warps per block (2D:
 // 512 x points; 3D: 4 y rows).  Forward modes only (MODE_FWD, MODE_FWD_D).
-// The 2D kernel is bounded for six blocks per SM (80 registers, a few bytes
-// of spills, faster than the unbounded allocation); a bound spills heavily in
-// 3D.
-template <int MODE, int NDIM>
-__global__ void __launch_bounds__(128, NDIM == 2 ? 6 : 1) k_ac_hp(const StepArgs A) {
-  static_assert(MODE == MODE_FWD || MODE == MODE_FWD_D, "compensated step: forward modes only");
+// The 2D kernel is bounded for six blocks per SM: bound by the latency of a
+// row and by FP64 issue in the strips (16 shots of 2001 x 801: 273 us per step;
+// 287 at four blocks, 307 at three, which spill nothing); a bound spills
+// heavily in 3D.
+// 2D: the lanes that meet an x strip store nothing in the main blocks; ITEM
+// blocks at the end of the launch take those groups of four points, one
+// (group, row, shot) per thread.  GB300 executes FP64 at 2 lanes per clock and
+// SM whatever lanes are active, so a warp with 5 strip lanes paid as much as
+// one with 32 (about 1 us of the SM per row): 16 shots of 2001 x 801 760 -> 273
+// us per step with this split and the strips' memory variables loaded with
+// the row, 4 shots of 901 x 455 87 -> 44.
+template <int MODE, int NDIM, bool ITEM>
+__device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
   constexpr unsigned FULL = 0xffffffffu;
-  chain_next();
-  chain_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int S = A.nshots;
-  const int shot = blockIdx.x % S;
-  int tile = blockIdx.x / S;
   const int nx = A.n0, P = A.P, H = A.halo;
   const int nm = NDIM == 2 ? A.n1 : A.n2;  // marching axis
   const int ny = NDIM == 3 ? A.n1 : 1;
-  int wx0, y = 0;
-  if (NDIM == 2) {
-    wx0 = (tile % A.tiles_x) * 512 + warp * 128;
-    tile /= A.tiles_x;
+  int shot, x0, y = 0, z_begin, z_end;
+  if (ITEM) {
+    int nl, xr, ng;
+    xstrip_groups(nx, H, P, nl, xr, ng);
+    const int g = (int)(item % ng);
+    const long long rest = item / ng;
+    z_begin = 1 + (int)(rest % (nm - 2));
+    z_end = z_begin + 1;
+    shot = (int)(rest / (nm - 2));
+    if (shot >= S) return;
+    x0 = g < nl ? 4 * g : xr + 4 * (g - nl);
   } else {
-    wx0 = (tile % A.tiles_x) * 128;
-    tile /= A.tiles_x;
-    y = 1 + (tile % A.tiles_y) * 4 + warp;
-    tile /= A.tiles_y;
+    shot = blockIdx.x % S;
+    int tile = blockIdx.x / S;
+    int wx0;
+    if (NDIM == 2) {
+      wx0 = (tile % A.tiles_x) * 512 + warp * 128;
+      tile /= A.tiles_x;
+    } else {
+      wx0 = (tile % A.tiles_x) * 128;
+      tile /= A.tiles_x;
+      y = 1 + (tile % A.tiles_y) * 4 + warp;
+      tile /= A.tiles_y;
+    }
+    z_begin = 1 + tile * A.TZ;
+    z_end = min(z_begin + A.TZ, nm - 1);
+    if (z_begin >= z_end || wx0 >= P || (NDIM == 3 && y > ny - 2)) return;  // warp-uniform
+    x0 = wx0 + lane * 4;
   }
-  const int z_begin = 1 + tile * A.TZ;
-  const int z_end = min(z_begin + A.TZ, nm - 1);
-  if (z_begin >= z_end || wx0 >= P || (NDIM == 3 && y > ny - 2)) return;  // warp-uniform
-  const int x0 = wx0 + lane * 4;
   const bool inb = x0 < P;
   const int xa = inb ? x0 : P - 4;
   const long long plane = NDIM == 2 ? (long long)P : (long long)P * ny;  // stride of the marching axis
@@ -2218,8 +2299,12 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? 6 : 1) k_ac_hp(const StepArgs
   float* ckd = fptr(A.ck_d, shot);
   float* Dw = nullptr;
   if (MODE == MODE_FWD_D && shot >= A.d_first) Dw = dptr(A.Dout, shot, A.dbf16);
-  const bool xstrip = inb && (x0 < H || x0 + 3 >= nx - H);
-  const bool ystrip = NDIM == 3 && ((y < H) || (y >= ny - H));
+  XCells xc = xcells(x0, nx, H, inb);
+  if (NDIM == 2 && !ITEM) xc.in = 0;
+  const bool own = inb && !(NDIM == 2 && !ITEM && (x0 < H || x0 + 3 >= nx - H));  // points this thread stores
+  int yq = 0;
+  bool yfirst = false;
+  const bool ystrip = NDIM == 3 && strip_cell(y, ny, H, yq, yfirst);
   const int ax_m = NDIM - 1;  // index of the marching axis in ih / ih2
   const ff ih2x{A.ih2[0], A.ih2_lo[0]}, ih2m{A.ih2[ax_m], A.ih2_lo[ax_m]};
   const ff ih2y{A.ih2[1], A.ih2_lo[1]};
@@ -2248,66 +2333,66 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? 6 : 1) k_ac_hp(const StepArgs
       ld4(yph, pc + idx + P);
       ld4(ypl, pcl + idx + P);
     }
-    float lh = __shfl_up_sync(FULL, r0h[3], 1), ll = __shfl_up_sync(FULL, r0l[3], 1);
-    float rh = __shfl_down_sync(FULL, r0h[0], 1), rl = __shfl_down_sync(FULL, r0l[0], 1);
-    if (lane == 0) {
+    float lh, ll, rh, rl;
+    if (!ITEM) {
+      lh = __shfl_up_sync(FULL, r0h[3], 1);
+      ll = __shfl_up_sync(FULL, r0l[3], 1);
+      rh = __shfl_down_sync(FULL, r0h[0], 1);
+      rl = __shfl_down_sync(FULL, r0l[0], 1);
+    }
+    if (ITEM || lane == 0) {
       lh = xa > 0 ? pc[idx - 1] : 0.f;
       ll = xa > 0 ? pcl[idx - 1] : 0.f;
     }
-    if (lane == 31) {
+    if (ITEM || lane == 31) {
       rh = xa + 4 < P ? pc[idx + 4] : 0.f;
       rl = xa + 4 < P ? pcl[idx + 4] : 0.f;
     }
-    const bool mstrip = (z < H) || (z >= nm - H);
+    int mq = 0;
+    bool mfirst = false;
+    const bool mstrip = strip_cell(z, nm, H, mq, mfirst);
     float outph[4], outpl[4], outdh[4], outdl[4], outD[4];
+    ff tx[4], tm[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float xmh = e == 0 ? lh : r0h[e - 1], xml = e == 0 ? ll : r0l[e - 1];
       const float xph = e == 3 ? rh : r0h[e + 1], xpl = e == 3 ? rl : r0l[e + 1];
-      const float ch = r0h[e], cl = r0l[e];
-      const int x = x0 + e;
-      const bool pin = inb && x >= 1 && x <= nx - 2;
-      ff dx = ff_d2(xmh, xml, ch, cl, xph, xpl);
-      ff dm = ff_d2(rmh[e], rml[e], ch, cl, rph[e], rpl[e]);
-      ff tx = ff_mul(dx, ih2x), tm = ff_mul(dm, ih2m);
-      if (xstrip && pin) {
-        Strip64 s0 = strip64_io(A, 0, shot, 1);
-        if (NDIM == 2) {
-          s0.psi_base = (long long)z * nh;
-          s0.xi_base = (long long)z * na;
-        } else {
-          s0.psi_base = ((long long)z * ny + y) * nh;
-          s0.xi_base = ((long long)z * ny + y) * na;
-        }
-        tx = ff_add(tx, cpml_axis_corr64(tx, ff{xmh, xml}, ff{ch, cl}, ff{xph, xpl}, x, nx, H, A.ihd[0], s0));
+      tx[e] = ff_mul(ff_d2(xmh, xml, r0h[e], r0l[e], xph, xpl), ih2x);
+      tm[e] = ff_mul(ff_d2(rmh[e], rml[e], r0h[e], r0l[e], rph[e], rpl[e]), ih2m);
+    }
+    if (xc.in) {
+      Strip64 s0 = strip64_io(A, 0, shot, 1);
+      s0.psi_base = NDIM == 2 ? (long long)z * nh : ((long long)z * ny + y) * nh;
+      s0.xi_base = NDIM == 2 ? (long long)z * na : ((long long)z * ny + y) * na;
+      cpml_corr64_x4(tx, r0h, r0l, ff{lh, ll}, ff{rh, rl}, x0, nx, H, A.ihd[0], xc, s0);
+    }
+    if (mstrip && own) {
+      Strip64 sm = strip64_io(A, ax_m, shot, plane);
+      sm.psi_base = sm.xi_base = rowoff;
+      if (NDIM == 2) sm.psi_base = sm.xi_base = xa;
+      cpml_corr64_4(tm, rmh, rml, r0h, r0l, rph, rpl, mq, mfirst, A.ihd[ax_m], sm);
+    }
+    ff lap[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) lap[e] = ff_add(tx[e], tm[e]);
+    if (NDIM == 3) {
+      ff ty[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ty[e] = ff_mul(ff_d2(ymh[e], yml[e], r0h[e], r0l[e], yph[e], ypl[e]), ih2y);
+      if (ystrip && inb) {
+        Strip64 s1 = strip64_io(A, 1, shot, P);
+        s1.psi_base = (long long)z * nh * P + xa;
+        s1.xi_base = (long long)z * na * P + xa;
+        cpml_corr64_4(ty, ymh, yml, r0h, r0l, yph, ypl, yq, yfirst, A.ihd[1], s1);
       }
-      if (mstrip && pin) {
-        Strip64 sm = strip64_io(A, ax_m, shot, plane);
-        if (NDIM == 2) {
-          sm.psi_base = x;
-          sm.xi_base = x;
-        } else {
-          sm.psi_base = (long long)y * P + x;
-          sm.xi_base = (long long)y * P + x;
-        }
-        tm = ff_add(tm, cpml_axis_corr64(tm, ff{rmh[e], rml[e]}, ff{ch, cl}, ff{rph[e], rpl[e]}, z, nm, H,
-                                         A.ihd[ax_m], sm));
-      }
-      ff lap = ff_add(tx, tm);
-      if (NDIM == 3) {
-        ff ty = ff_mul(ff_d2(ymh[e], yml[e], ch, cl, yph[e], ypl[e]), ih2y);
-        if (ystrip && pin) {
-          Strip64 s1 = strip64_io(A, 1, shot, P);
-          s1.psi_base = (long long)z * nh * P + x;
-          s1.xi_base = (long long)z * na * P + x;
-          ty = ff_add(ty, cpml_axis_corr64(ty, ff{ymh[e], yml[e]}, ff{ch, cl}, ff{yph[e], ypl[e]}, y, ny, H, A.ihd[1],
-                                           s1));
-        }
-        lap = ff_add(lap, ty);
-      }
-      const ff D = ff_mul(ff{fa[e], fb[e]}, lap);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) lap[e] = ff_add(lap[e], ty[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const ff D = ff_mul(ff{fa[e], fb[e]}, lap[e]);
       const ff dn = ff_add(ff{oh[e], ol[e]}, D);
-      const ff pnw = ff_add(ff{ch, cl}, dn);
+      const ff pnw = ff_add(ff{r0h[e], r0l[e]}, dn);
       outD[e] = ff_round(D);
       outdh[e] = dn.hi;
       outdl[e] = dn.lo;
@@ -2315,12 +2400,12 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? 6 : 1) k_ac_hp(const StepArgs
       outpl[e] = pnw.lo;
     }
     int de = 0;  // FP16 D slots (3D): the exponent of this warp's tile
-    if (MODE == MODE_FWD_D && A.dbf16 == 2 && Dw) {
+    if (NDIM == 3 && MODE == MODE_FWD_D && A.dbf16 == 2 && Dw) {
       de = warp_dexp(outD, inb);
-      const long long erow = ((long long)z * ny + y) * A.ntx + (wx0 >> 7);
+      const long long erow = ((long long)z * ny + y) * A.ntx + (x0 >> 7);  // the warp's tile
       if (lane == 0) A.Dexp.p[(long long)shot * A.Dexp.s + erow] = (signed char)de;
     }
-    if (inb) {
+    if (own) {
       if (ckp) {
         float cp4[4], cd4[4];
 #pragma unroll
@@ -2359,6 +2444,26 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? 6 : 1) k_ac_hp(const StepArgs
       r0l[e] = rpl[e];
     }
   }
+}
+
+template <int MODE>
+__device__ __noinline__ void hp_xstrip_item(const StepArgs& A, long long item) {
+  hp_body<MODE, 2, true>(A, item);
+}
+
+template <int MODE, int NDIM>
+__global__ void __launch_bounds__(128, NDIM == 2 ? 6 : 1) k_ac_hp(const StepArgs A) {
+  static_assert(MODE == MODE_FWD || MODE == MODE_FWD_D, "compensated step: forward modes only");
+  chain_next();
+  chain_wait();
+  if constexpr (NDIM == 2) {
+    const long long nb_main = (long long)A.nshots * A.tiles_x * A.tiles_z;
+    if ((long long)blockIdx.x >= nb_main) {
+      hp_xstrip_item<MODE>(A, ((long long)blockIdx.x - nb_main) * 128 + threadIdx.x);
+      return;
+    }
+  }
+  hp_body<MODE, NDIM, false>(A, 0);
 }
 
 }  // namespace swgb
