@@ -1348,7 +1348,7 @@ void enable_pair_carveout() {
 long long xstrip_blocks(const StepArgs& a) {
   int nl, xr, ng;
   xstrip_groups(a.n0, a.halo, a.P, nl, xr, ng);
-  return ((long long)ng * (a.n1 - 2) * a.nshots + 127) / 128;
+  return ((long long)ng * (a.n1 - 2) * (a.n2 > 1 ? a.n2 - 2 : 1) * a.nshots + 127) / 128;
 }
 
 // The 2D one-step stencil of 4-warp blocks with the x strips split off:
@@ -1421,11 +1421,13 @@ struct Launcher {
     int nk = 1;  // kernels launched for this step
     if constexpr (MODE == MODE_FWD || MODE == MODE_FWD_D) {
       if (ws->precision == 1 && !recompute) {  // compensated forward (context from make_hp_ctx)
+        const char* what = "compensated stencil launch";
         if (ws->N == 2)
-          launch_chain("compensated stencil launch", k_ac_hp<MODE, 2>, dim3((unsigned)(blocks + xstrip_blocks(a))), dim3(128),
-                       st, a);
+          launch_chain(what, k_ac_hp<MODE, 2, true>, dim3((unsigned)(blocks + xstrip_blocks(a))), dim3(128), st, a);
+        else if (a.dbf16 == 2)
+          launch_chain(what, k_ac_hp<MODE, 3, false>, dim3((unsigned)blocks), dim3(128), st, a);
         else
-          launch_chain("compensated stencil launch", k_ac_hp<MODE, 3>, dim3((unsigned)blocks), dim3(128), st, a);
+          launch_chain(what, k_ac_hp<MODE, 3, true>, dim3((unsigned)(blocks + xstrip_blocks(a))), dim3(128), st, a);
         ws->ctx->prof.end(st, kind, ev);
         return;
       }

@@ -2235,16 +2235,16 @@ __device__ __forceinline__ void cpml_corr64_x4(ff (&t)[4], const float (&ch)[4],
 // 512 x points; 3D: 4 y rows).  Forward modes only (MODE_FWD, MODE_FWD_D).
 // The 2D kernel is bounded for six blocks per SM: bound by the latency of a
 // row and by FP64 issue in the strips (16 shots of 2001 x 801: 273 us per step;
-// 287 at four blocks, 307 at three, which spill nothing); a bound spills
-// heavily in 3D.
-// 2D: the lanes that meet an x strip store nothing in the main blocks; ITEM
+// 287 at four blocks, 307 at three, which spill nothing), the 3D one with the
+// x strips split off for four (400^3: 1674 us per step against 2053 unbounded).
+// XS: the lanes that meet an x strip store nothing in the main blocks; ITEM
 // blocks at the end of the launch take those groups of four points, one
 // (group, row, shot) per thread.  GB300 executes FP64 at 2 lanes per clock and
 // SM whatever lanes are active, so a warp with 5 strip lanes paid as much as
 // one with 32 (about 1 us of the SM per row): 16 shots of 2001 x 801 760 -> 273
 // us per step with this split and the strips' memory variables loaded with
-// the row, 4 shots of 901 x 455 87 -> 44.
-template <int MODE, int NDIM, bool ITEM>
+// the row, 4 shots of 901 x 455 87 -> 44, 2 of 183 x 157 x 141 1170 -> 556.
+template <int MODE, int NDIM, bool XS, bool ITEM>
 __device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2257,11 +2257,15 @@ __device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
     int nl, xr, ng;
     xstrip_groups(nx, H, P, nl, xr, ng);
     const int g = (int)(item % ng);
-    const long long rest = item / ng;
+    long long rest = item / ng;
+    if (NDIM == 3) {
+      y = 1 + (int)(rest % (ny - 2));
+      rest /= ny - 2;
+    }
     z_begin = 1 + (int)(rest % (nm - 2));
     z_end = z_begin + 1;
+    if (rest / (nm - 2) >= S) return;
     shot = (int)(rest / (nm - 2));
-    if (shot >= S) return;
     x0 = g < nl ? 4 * g : xr + 4 * (g - nl);
   } else {
     shot = blockIdx.x % S;
@@ -2300,8 +2304,8 @@ __device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
   float* Dw = nullptr;
   if (MODE == MODE_FWD_D && shot >= A.d_first) Dw = dptr(A.Dout, shot, A.dbf16);
   XCells xc = xcells(x0, nx, H, inb);
-  if (NDIM == 2 && !ITEM) xc.in = 0;
-  const bool own = inb && !(NDIM == 2 && !ITEM && (x0 < H || x0 + 3 >= nx - H));  // points this thread stores
+  if (XS && !ITEM) xc.in = 0;
+  const bool own = inb && !(XS && !ITEM && (x0 < H || x0 + 3 >= nx - H));  // points this thread stores
   int yq = 0;
   bool yfirst = false;
   const bool ystrip = NDIM == 3 && strip_cell(y, ny, H, yq, yfirst);
@@ -2379,7 +2383,7 @@ __device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
       ff ty[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) ty[e] = ff_mul(ff_d2(ymh[e], yml[e], r0h[e], r0l[e], yph[e], ypl[e]), ih2y);
-      if (ystrip && inb) {
+      if (ystrip && own) {
         Strip64 s1 = strip64_io(A, 1, shot, P);
         s1.psi_base = (long long)z * nh * P + xa;
         s1.xi_base = (long long)z * na * P + xa;
@@ -2400,7 +2404,7 @@ __device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
       outpl[e] = pnw.lo;
     }
     int de = 0;  // FP16 D slots (3D): the exponent of this warp's tile
-    if (NDIM == 3 && MODE == MODE_FWD_D && A.dbf16 == 2 && Dw) {
+    if (NDIM == 3 && !XS && MODE == MODE_FWD_D && A.dbf16 == 2 && Dw) {
       de = warp_dexp(outD, inb);
       const long long erow = ((long long)z * ny + y) * A.ntx + (x0 >> 7);  // the warp's tile
       if (lane == 0) A.Dexp.p[(long long)shot * A.Dexp.s + erow] = (signed char)de;
@@ -2446,24 +2450,26 @@ __device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
   }
 }
 
-template <int MODE>
+template <int MODE, int NDIM>
 __device__ __noinline__ void hp_xstrip_item(const StepArgs& A, long long item) {
-  hp_body<MODE, 2, true>(A, item);
+  hp_body<MODE, NDIM, true, true>(A, item);
 }
 
-template <int MODE, int NDIM>
-__global__ void __launch_bounds__(128, NDIM == 2 ? 6 : 1) k_ac_hp(const StepArgs A) {
+// XS: the x strips in blocks of their own (always in 2D; in 3D unless the FP16
+// D slots need the maximum over each warp's whole tile).
+template <int MODE, int NDIM, bool XS>
+__global__ void __launch_bounds__(128, NDIM == 2 ? 6 : XS ? 4 : 1) k_ac_hp(const StepArgs A) {
   static_assert(MODE == MODE_FWD || MODE == MODE_FWD_D, "compensated step: forward modes only");
   chain_next();
   chain_wait();
-  if constexpr (NDIM == 2) {
-    const long long nb_main = (long long)A.nshots * A.tiles_x * A.tiles_z;
+  if constexpr (XS) {
+    const long long nb_main = (long long)A.nshots * A.tiles_x * A.tiles_y * A.tiles_z;
     if ((long long)blockIdx.x >= nb_main) {
-      hp_xstrip_item<MODE>(A, ((long long)blockIdx.x - nb_main) * 128 + threadIdx.x);
+      hp_xstrip_item<MODE, NDIM>(A, ((long long)blockIdx.x - nb_main) * 128 + threadIdx.x);
       return;
     }
   }
-  hp_body<MODE, NDIM, false>(A, 0);
+  hp_body<MODE, NDIM, XS, false>(A, 0);
 }
 
 }  // namespace swgb
