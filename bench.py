@@ -824,7 +824,7 @@ def _extra_acoustic3d(a, device):
     clk = clocks.stop()
     pts = float(w.point_steps())
     peak, _ = _peak()
-    k3 = "k_ac3d_inner + k_ac3d_zslab + k_ac3d_yslab"
+    k3 = "k_ac3d_xstrip + k_ac3d_main"
     names = {0: f"{k3} <1> forward", 4: f"{k3} <1> recompute", 1: f"{k3} <2> adjoint + correlation"}
     kern = {names[k]: {"ms": prof[k][0], "GB_per_s": prof[k][2] / (prof[k][0] / 1e3) / 1e9 if prof[k][0] else None,
                        "frac": prof[k][2] / (prof[k][0] / 1e3) / 1e9 / peak if prof[k][0] else None}
@@ -975,7 +975,7 @@ def run_gb300(a):
 
     def kname(m):
         if nd == 3:
-            return f"k_ac3d_inner + k_ac3d_zslab + k_ac3d_yslab<{m}>"
+            return f"k_ac3d_xstrip + k_ac3d_main<{m}>"
         return f"k_ac2d_step<{m}, XS> (x strips as extra blocks)" if xs else f"k_ac2d_step<{m}>"
 
     if nd == 2 and veff >= 0 and (veff & 256) and nshots >= 4:

@@ -227,9 +227,9 @@ int sw_acoustic_forward_snapshots(sw_wavesim* ws, int32_t nshots, const sw_acous
  * block of that kernel (0 = heuristic: 32, fewer for small batches; 1 = 8,
  * 2 = 16, 3 = 32, 4 = 64, 5 = 128, 6 = 4) and bits 14-15 its resident-block
  * bound (0 = 6 forward / 5 adjoint blocks per SM, 1 = 4 / 3, 2 = 7 / 4).
- * 3D: + 65536 runs the step as one launch instead of three (rows outside the
- * y / z strips, the z slabs, the y slabs); + 131072 is accepted and has no
- * effect (the three launches always run without a software pipeline).  2D, 4 warps per block: by default the
+ * 3D: + 65536 runs the step as one launch instead of two (the groups of four
+ * points that meet an x strip; the others, by z slabs, y slabs and inner
+ * rows); + 131072 is accepted and has no effect.  2D, 4 warps per block: by default the
  * 4-point lane groups that meet an x strip are advanced by extra blocks at the
  * end of the stencil launch, one group per thread (the main blocks skip
  * them); + 262144 keeps them in the main blocks' per-point C-PML path.
@@ -282,7 +282,7 @@ int sw_wavesim_use_graphs(sw_wavesim* ws, int32_t on);
 int sw_profile_enable(sw_ctx* ctx, int32_t on);
 int sw_profile_read(sw_ctx* ctx, int32_t kind, double* total_ms, int64_t* launches, double* bytes);
 /* Kernel launches inside the brackets that sw_profile_read counts as
- * `launches` (one bracket per step of a kind; the 3D step as three launches,
+ * `launches` (one bracket per step of a kind; the 3D step as two launches,
  * the variable-density adjoint pair and the elastic displacement pair launch
  * several kernels). */
 int sw_profile_read_kernels(sw_ctx* ctx, int32_t kind, int64_t* kernels);

@@ -566,6 +566,7 @@ struct sw_wavesim {
   DevMem g, gc;
   DevMem dbuf;                         // D slots
   DevMem dexp;                         // FP16 D slots (snapshot_bf16 3): exponent per row and 128-point x tile
+  DevMem dstrip;                       // and the x strips' D of the current step (dstrip_floats per shot)
   long long d_slots = 0;
   DevMem ck;                           // checkpoint slots (with BF16 snapshots: the psi / xi strips only)
   long long ck_slots = 0;
@@ -954,6 +955,12 @@ void build_tables(sw_wavesim* ws, const sw_acoustic_shot* shots, const std::vect
 
 size_t per_shot_bytes(const sw_wavesim* ws, bool grad, int max_nt);
 
+// FP16 D slots: the x strips' D of one step and shot in FP32 (ac3d_body), [z][y][group][4].
+long long dstrip_floats(const sw_wavesim* ws) {
+  int nl, xr, ng;
+  xstrip_groups(ws->n[0], ws->prm.halo, ws->P, nl, xr, ng);
+  return (long long)ws->n[1] * ws->n[2] * std::max(ng, 1) * 4;
+}
 // Exponent array of the FP16 D slots: per slot rows x x-tiles bytes, slots of a shot contiguous.
 long long dexp_slot(const sw_wavesim* ws) {
   long long rows = 1;
@@ -975,7 +982,7 @@ size_t owned_bytes(const sw_wavesim* ws) {
   size_t owned = 0;
   for (int b = 0; b < 2; ++b) owned += ws->pb[b].bytes + ws->ab[b].bytes + ws->plo[b].bytes;
   owned += ws->db.bytes + ws->adb.bytes + ws->g.bytes + ws->gc.bytes + ws->dbuf.bytes + ws->ck.bytes + ws->dlo.bytes;
-  owned += ws->db2.bytes + ws->adb2.bytes + ws->ck16.bytes + ws->ck_stage.bytes;
+  owned += ws->dstrip.bytes + ws->db2.bytes + ws->adb2.bytes + ws->ck16.bytes + ws->ck_stage.bytes;
   for (int d = 0; d < 3; ++d) owned += ws->psi64[0][d].bytes + ws->psi64[1][d].bytes + ws->xi64[d].bytes;
   for (int k = 0; k < 2; ++k)
     for (int d = 0; d < 3; ++d) owned += ws->psi[k][d].bytes + ws->apsi[k][d].bytes;
@@ -1063,6 +1070,7 @@ void ensure_state(sw_wavesim* ws, int S, bool grad, int max_nt) {
       if (ws->gp.snapshot_bf16 == 3) {
         dev_alloc(ws->dexp, (size_t)ws->cap * dslots * dexp_slot(ws), "D exponents", st);
         check_cuda(cudaMemsetAsync(ws->dexp.p, 0, ws->dexp.bytes, st), "D exponents");
+        dev_alloc(ws->dstrip, (size_t)ws->cap * dstrip_floats(ws) * sizeof(float), "D of the x strips", st);
       }
       ws->d_slots = dslots;
       ++ws->cache.gen;
@@ -1106,6 +1114,7 @@ size_t per_shot_bytes(const sw_wavesim* ws, bool grad, int max_nt) {
     const int K = ws->gp.check_freq;
     const long long dsl = (K == 1 ? (long long)max_nt : K) * ws->F;
     floats += ws->gp.snapshot_bf16 >= 1 ? (dsl + 1) / 2 : dsl;  // BF16 D slots take half
+    if (ws->gp.snapshot_bf16 == 3) floats += dstrip_floats(ws);
     if (K > 1) {
       if (ws->gp.snapshot_bf16 == 2)  // BF16 (p, d) = one float's worth per point, plus the FP32 stage
         floats += (long long)(max_nt / K) * (ws->F + ws->strip_total) + 2 * ws->F;
@@ -1472,34 +1481,24 @@ struct Launcher {
       else
         k_ac2d_step<MODE, 16><<<(unsigned)blocks, 512, 0, st>>>(a);
     } else if (ws->split3d) {
-      // rows outside the y / z strips, the z slabs, the y slabs (k_ac3d_inner, k_ac3d_zslab, k_ac3d_yslab)
       const int nw = block_rows3d(ws);
       const Split3d sp = split3d(ws, c.TZ, nw);
-      StepArgs a1 = a;
-      a1.tiles_y = sp.tiles_y1;
-      a1.tiles_z = sp.tiles_z1;
-      const long long b1 = (long long)a.nshots * c.tiles_x * sp.tiles_y1 * sp.tiles_z1;
       // the slabs are a halo deep (z) or a halo wide (y): 4-plane bands
       // (2 x 400^3, gradient: 212.0 ms against 220.0 with the 16 of the inner rows)
-      const int tzs = std::min(c.TZ, 4);
-      const Split3d ss = split3d(ws, tzs, nw);
-      StepArgs a2 = a;
-      a2.TZ = tzs;
-      const long long b2 = (long long)a.nshots * c.tiles_x * ss.zslab_units;
-      const long long b3 = (long long)a.nshots * c.tiles_x * ss.yslab_units;
-      nk = (b1 > 0) + (b2 > 0) + (b3 > 0);
-      if (b1 > 0) {
-        if (nw == 8) launch_chain("stencil launch", k_ac3d_inner<MODE, 8>, dim3((unsigned)b1), dim3(256), st, a1);
-        else launch_chain("stencil launch", k_ac3d_inner<MODE, 4>, dim3((unsigned)b1), dim3(128), st, a1);
-      }
-      if (b2 > 0) {
-        if (nw == 8) launch_chain("stencil launch", k_ac3d_zslab<MODE, 8>, dim3((unsigned)b2), dim3(256), st, a2);
-        else launch_chain("stencil launch", k_ac3d_zslab<MODE, 4>, dim3((unsigned)b2), dim3(128), st, a2);
-      }
-      if (b3 > 0) {
-        if (nw == 8) launch_chain("stencil launch", k_ac3d_yslab<MODE, 8>, dim3((unsigned)b3), dim3(256), st, a2);
-        else launch_chain("stencil launch", k_ac3d_yslab<MODE, 4>, dim3((unsigned)b3), dim3(128), st, a2);
-      }
+      a.TZs = std::min(c.TZ, 4);
+      const Split3d ss = split3d(ws, a.TZs, nw);
+      a.tiles_y = sp.tiles_y1;
+      a.tiles_z = sp.tiles_z1;
+      const long long b1 = (long long)a.nshots * c.tiles_x * sp.tiles_y1 * sp.tiles_z1;
+      a.b_z = (long long)a.nshots * c.tiles_x * ss.zslab_units;
+      a.b_y = (long long)a.nshots * c.tiles_x * ss.yslab_units;
+      if (a.dbf16 == 2) a.Dstrip = FieldArg{ws->dstrip.as<float>(), dstrip_floats(ws)};
+      const long long bx = xstrip_blocks(a);
+      nk = bx > 0 ? 2 : 1;
+      if (bx > 0) launch_chain("stencil launch", k_ac3d_xstrip<MODE>, dim3((unsigned)bx), dim3(128), st, a);
+      const dim3 grid((unsigned)(a.b_z + a.b_y + b1));
+      if (nw == 8) launch_chain("stencil launch", k_ac3d_main<MODE, 8>, grid, dim3(256), st, a);
+      else launch_chain("stencil launch", k_ac3d_main<MODE, 4>, grid, dim3(128), st, a);
     } else {
       const int nw = block_rows3d(ws);
       if constexpr (MODE == MODE_FWD) {

@@ -84,6 +84,9 @@ struct StepArgs {
   int dbf16;  // Dout / dcorr: 0 FP32, 1 BF16, 2 FP16 scaled by 2^e per row and 128-point x tile (3D)
   FieldArgE Dexp, dcorr_exp;  // dbf16 == 2: the exponents e of Dout / dcorr, [row][x tile]
   int ntx;                    // x tiles of 128 points per row of the exponent arrays
+  FieldArg Dstrip;            // dbf16 == 2: D of the x strips' groups, [z][y][group][4] (3D)
+  int TZs;                    // 3D: planes per block of the slabs
+  long long b_z, b_y;         // 3D: blocks of the z and of the y slabs
   // compensated step (k_ac_hp): low parts of p[n], p[n+1] and d (in place), of fact and of 1/h^2;
   // FP64 C-PML coefficients (stride cpml_stride), memory variables and 1/h
   FieldArg plo_cur, plo_new, dlo;
@@ -415,6 +418,8 @@ __device__ __forceinline__ void cpml_axis_x4(float (&t)[4], const float (&p0)[4]
 __device__ __forceinline__ void l2_prefetch(const void* p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
+
+__device__ __forceinline__ void l2_prefetch_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ float* fptr(const FieldArg& f, int shot) {
   return f.p ? f.p + (long long)shot * f.s : nullptr;
@@ -1522,7 +1527,7 @@ __device__ __forceinline__ void split_axis(int n, int H, int& a, int& b) {
 // x tile as (z band, y group) units.
 template <int NW, int REGION>
 __device__ __forceinline__ bool ac3d_work(const StepArgs& A, int tile, int warp, int& y, int& z_begin, int& z_end) {
-  const int ny = A.n1, nz = A.n2, H = A.halo, TZ = A.TZ;
+  const int ny = A.n1, nz = A.n2, H = A.halo, TZ = REGION >= 2 ? A.TZs : A.TZ;
   if (REGION == 0) {
     const int tyi = tile % A.tiles_y, tzi = tile / A.tiles_y;
     y = 1 + tyi * NW + warp;
@@ -1567,22 +1572,41 @@ __device__ __forceinline__ bool ac3d_work(const StepArgs& A, int tile, int warp,
   return z_begin < z_end && y <= ny - 2;
 }
 
-template <int MODE, int NW, bool FAST = false, int REGION = 0, bool PIPE = true>
-__device__ __forceinline__ void ac3d_body(const StepArgs& A) {
+// XS: the lanes that meet an x strip store nothing but their share of an FP16 D
+// tile (XBODY); the groups of four points they hold are advanced one per
+// thread (XITEM, see k_ac3d_xstrip).
+enum XMode { XNONE = 0, XBODY = 1, XITEM = 2 };
+template <int MODE, int NW, bool FAST = false, int REGION = 0, bool PIPE = true, int XS = XNONE>
+__device__ __forceinline__ void ac3d_body(const StepArgs& A, long long block) {
   constexpr unsigned FULL = 0xffffffffu;
-  chain_next();
-  chain_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int S = A.nshots;
-  const int shot = blockIdx.x % S;
-  int tile = blockIdx.x / S;
-  const int txi = tile % A.tiles_x;
-  tile /= A.tiles_x;
   const int nx = A.n0, ny = A.n1, nz = A.n2, P = A.P, H = A.halo;
-  int y, z_begin, z_end;  // one y row per warp, NW rows per block
-  if (!ac3d_work<NW, REGION>(A, tile, warp, y, z_begin, z_end)) return;  // warp-uniform
-  const int wx0 = txi * 128;
-  const int x0 = wx0 + lane * 4;
+  int nl = 0, xr = 0, ng = 0;  // the x strips' groups
+  if (XS != XNONE) xstrip_groups(nx, H, P, nl, xr, ng);
+  int shot, wx0 = 0, x0, y, z_begin, z_end;
+  if (XS == XITEM) {
+    const long long item = block * (32 * NW) + threadIdx.x;
+    const int g = (int)(item % ng);
+    long long rest = item / ng;
+    y = 1 + (int)(rest % (ny - 2));
+    rest /= ny - 2;
+    z_begin = 1 + (int)(rest % (nz - 2));
+    z_end = z_begin + 1;
+    rest /= nz - 2;
+    if (rest >= S) return;
+    shot = (int)rest;
+    x0 = g < nl ? 4 * g : xr + 4 * (g - nl);
+  } else {
+    shot = (int)(block % S);
+    int tile = (int)(block / S);
+    const int txi = tile % A.tiles_x;
+    tile /= A.tiles_x;
+    // one y row per warp, NW rows per block
+    if (!ac3d_work<NW, REGION>(A, tile, warp, y, z_begin, z_end)) return;  // warp-uniform
+    wx0 = txi * 128;
+    x0 = wx0 + lane * 4;
+  }
   const bool inb = x0 < P;
   const int xa = inb ? x0 : P - 4;
   const long long plane = (long long)P * ny;
@@ -1594,7 +1618,10 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
   const float* __restrict__ fa = A.fact;
   const int na = 2 * H + 2, nh = 2 * H;
 
-  const XCells xc = xcells(x0, nx, H, inb);
+  XCells xc = xcells(x0, nx, H, inb);
+  const bool xlane = XS == XBODY && inb && (x0 < 4 * nl || x0 >= xr);  // advanced by an XITEM thread
+  const bool own = inb && !xlane;
+  if (XS == XBODY) xc.in = 0;
   // region 1: never in a y strip; region 3: always
   const bool ystrip = REGION == 3 || (REGION != 1 && ((y < H) || (y >= ny - H)));
   // the warp's 128 x points and its y row interior and outside the strips
@@ -1637,6 +1664,14 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
       ld4(yp, pc + idx + P);
       ld4rw(o, di + idx);
       ld4(f, fa + idx);
+      if (XS == XBODY && z + 1 < z_end) {  // the next plane's DRAM rows on their way into L2, no registers held
+        l2_prefetch_line(pc + idx + 2 * plane);
+        l2_prefetch_line(di + idx + plane);
+        if (MODE == MODE_ADJ) {
+          l2_prefetch_line(gg + idx + plane);
+          l2_prefetch_line(gcp + idx + plane);
+        }
+      }
     } else if (more) {
       const long long nidx = idx + plane;
       ld4(rpn, pc + nidx + plane);
@@ -1645,10 +1680,13 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
       ld4rw(on, di + nidx);
       ld4(fn, fa + nidx);
     }
-    float left = __shfl_up_sync(FULL, r0[3], 1);
-    float right = __shfl_down_sync(FULL, r0[0], 1);
-    if (lane == 0) left = xa > 0 ? pc[idx - 1] : 0.f;
-    if (lane == 31) right = xa + 4 < P ? pc[idx + 4] : 0.f;
+    float left = 0.f, right = 0.f;
+    if (XS != XITEM) {
+      left = __shfl_up_sync(FULL, r0[3], 1);
+      right = __shfl_down_sync(FULL, r0[0], 1);
+    }
+    if (XS == XITEM || lane == 0) left = xa > 0 ? pc[idx - 1] : 0.f;
+    if (XS == XITEM || lane == 31) right = xa + 4 < P ? pc[idx + 4] : 0.f;
     // regions 1 and 3: never in a z strip; region 2: always
     const bool zstrip = REGION == 2 || (REGION != 1 && REGION != 3 && ((z < H) || (z >= nz - H)));
     float outp[4], outd[4], outD[4];
@@ -1684,13 +1722,13 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
       }
       // the y and z strips: the strip cell is the same for the four points
       // (it depends on y or z only), so their memory variables move as float4
-      if (ystrip && inb) {
+      if (ystrip && own) {
         StripIO s1 = strip_io(A, 1, shot, P);
         s1.psi_base = (long long)z * nh * P + xa;
         s1.xi_base = (long long)z * na * P + xa;
         cpml_axis_term4(ty, ym, r0, yp, y, ny, H, A.ih[1], s1);
       }
-      if (zstrip && inb) {
+      if (zstrip && own) {
         StripIO s2 = strip_io(A, 2, shot, (long long)ny * P);
         s2.psi_base = (long long)y * P + xa;
         s2.xi_base = (long long)y * P + xa;
@@ -1704,14 +1742,24 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
         outp[e] = radd(r0[e], outd[e]);
       }
     }
-    // FP16 D slots: the exponent of this warp's tile of row (y, z)
-    const long long erow = ((long long)z * ny + y) * A.ntx + txi;
+    // FP16 D slots: the exponent of the 128-point tile of row (y, z)
+    const long long erow = ((long long)z * ny + y) * A.ntx + (x0 >> 7);
     int de = 0;
-    if (MODE == MODE_FWD_D && A.dbf16 == 2 && Dw) {
-      de = warp_dexp(outD, inb);
-      if (lane == 0) A.Dexp.p[(long long)shot * A.Dexp.s + erow] = (signed char)de;
+    const bool d16 = MODE == MODE_FWD_D && A.dbf16 == 2 && Dw;
+    if (d16) {
+      // the x strips' D comes from (goes to) the scratch row, so that the
+      // exponent is the maximum over the whole tile
+      float* sc = nullptr;
+      if (XS == XITEM || xlane)
+        sc = A.Dstrip.p + (long long)shot * A.Dstrip.s + (((long long)z * ny + y) * ng + (x0 < 4 * nl ? x0 / 4 : nl + (x0 - xr) / 4)) * 4;
+      if (XS == XITEM) st4(sc, outD);
+      if (xlane) ld4rw(outD, sc);
+      if (XS != XITEM) {
+        de = warp_dexp(outD, inb);
+        if (lane == 0) A.Dexp.p[(long long)shot * A.Dexp.s + erow] = (signed char)de;
+      }
     }
-    if (inb) {
+    if (own) {
       if (ckp) {
         st4(ckp + idx, r0);
         st4(ckd + idx, o);
@@ -1736,7 +1784,7 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
       if (vec_interior) {
         st4(pn + idx, outp);
         st4(dn + idx, outd);
-        if (MODE == MODE_FWD_D && Dw) dst4(Dw, idx, outD, A.dbf16, de);
+        if (MODE == MODE_FWD_D && Dw && !(XS == XITEM && d16)) dst4(Dw, idx, outD, A.dbf16, de);
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -1744,9 +1792,17 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
           if (x >= 1 && x <= nx - 2) {
             pn[idx + e] = outp[e];
             dn[idx + e] = outd[e];
-            if (MODE == MODE_FWD_D && Dw) dst1(Dw, idx + e, outD[e], A.dbf16, de);
+            if (MODE == MODE_FWD_D && Dw && !(XS == XITEM && d16)) dst1(Dw, idx + e, outD[e], A.dbf16, de);
           }
         }
+      }
+    } else if (xlane && d16) {
+      if (vec_interior) {
+        dst4(Dw, idx, outD, 2, de);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (x0 + e >= 1 && x0 + e <= nx - 2) dst1(Dw, idx + e, outD[e], 2, de);
       }
     }
 #pragma unroll
@@ -1771,30 +1827,46 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A) {
 // register choice (1.96 against 1.76 TB/s).
 template <int MODE, int NW = 4>
 __global__ void __launch_bounds__(32 * NW, 24 / NW) k_ac3d_step(const StepArgs A) {
-  ac3d_body<MODE, NW>(A);
+  ac3d_body<MODE, NW>(A, blockIdx.x);
 }
 template <int MODE, int NW = 4>
 __global__ void __launch_bounds__(32 * NW) k_ac3d_fwd(const StepArgs A) {
-  ac3d_body<MODE, NW, true>(A);
+  ac3d_body<MODE, NW, true>(A, blockIdx.x);
 }
-// Three-launch 3D step: rows outside the y and z strips (no y / z C-PML code,
-// fewer registers), the z slabs (z strip code only where it applies), the y
-// slabs.  Every point is computed by exactly one launch with the arithmetic
-// of ac3d_body.  No software pipeline: 6 resident blocks per SM of the inner
-// rows and 5 of the slabs beat the pipelined form at 6 and 4 (gradient of 2
-// shots of 400^3, 60 steps: 212 against 244 ms); 8 / 6 / 6 run 216 ms
-// (spills), 5 / 4 / 4 230 ms.
-template <int MODE, int NW = 4>
-__global__ void __launch_bounds__(32 * NW, 24 / NW) k_ac3d_inner(const StepArgs A) {
-  ac3d_body<MODE, NW, false, 1, false>(A);
+// The 3D step in two launches.  k_ac3d_xstrip advances the groups of four
+// points that meet an x strip, one (group, y, z, shot) per thread; k_ac3d_main
+// the others: the z slabs (z strip code only where it applies), the y slabs and
+// the rows outside both strips (no y / z C-PML code), in this order.  Every
+// point is computed once with the arithmetic of ac3d_body.  In the rows' own
+// warps the x strips were 3 of 4 warps of a 400-point row running C-PML code for
+// 1 to 5 lanes (413 instructions per warp row against 183 now).  Bound by the
+// latency of a row's loads: 8 resident blocks per SM (64 registers, some
+// spills) and, for the adjoint, its sums prefetched a plane ahead; gradient of
+// 2 shots of 400^3, 60 steps: 176 ms (three launches with the strips inside:
+// 213; 6 blocks 190, 7 183, 9 186; without the prefetch 180), forward of 2 of
+// 183 x 157 x 141: 25.9 ms per 300 steps (34.8).  5 blocks of the strip kernel
+// (4: 27.9 ms, 6: 28.0).
+template <int MODE>
+__global__ void __launch_bounds__(128, 5) k_ac3d_xstrip(const StepArgs A) {
+  chain_next();
+  chain_wait();
+  ac3d_body<MODE, 4, false, 0, false, XITEM>(A, blockIdx.x);
 }
 template <int MODE, int NW = 4>
-__global__ void __launch_bounds__(32 * NW, 20 / NW) k_ac3d_zslab(const StepArgs A) {
-  ac3d_body<MODE, NW, false, 2, false>(A);
-}
-template <int MODE, int NW = 4>
-__global__ void __launch_bounds__(32 * NW, 20 / NW) k_ac3d_yslab(const StepArgs A) {
-  ac3d_body<MODE, NW, false, 3, false>(A);
+__global__ void __launch_bounds__(32 * NW, 32 / NW) k_ac3d_main(const StepArgs A) {
+  chain_next();
+  chain_wait();
+  long long b = blockIdx.x;
+  if (b < A.b_z) {
+    ac3d_body<MODE, NW, false, 2, false, XBODY>(A, b);
+    return;
+  }
+  b -= A.b_z;
+  if (b < A.b_y) {
+    ac3d_body<MODE, NW, false, 3, false, XBODY>(A, b);
+    return;
+  }
+  ac3d_body<MODE, NW, false, 1, false, XBODY>(A, b - A.b_y);
 }
 
 // ---------------------------------------------------------------------------
