@@ -634,15 +634,15 @@ template <int MODE, int NW, int DP = 1, bool XS = false, int MB = Ac2dBounds<MOD
 __global__ void __launch_bounds__(32 * NW, MB) k_ac2d_step(const StepArgs A) {
   constexpr unsigned FULL = 0xffffffffu;
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   if constexpr (XS) {
     const long long nb_main = (long long)A.nshots * A.tiles_x * A.tiles_y * A.tiles_z;
     if ((long long)blockIdx.x >= nb_main) {
-      xstrip_item<MODE>(A, ((long long)blockIdx.x - nb_main) * (32 * NW) + threadIdx.x);
+      xstrip_item<MODE>(A, ((long long)blockIdx.x - nb_main) * (32 * NW) + tid);
       return;
     }
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   constexpr int nwarps = NW;
   const int S = A.nshots;
   // block order: x tiles fastest (neighbouring CTAs stream one contiguous row
@@ -1577,16 +1577,16 @@ __device__ __forceinline__ bool ac3d_work(const StepArgs& A, int tile, int warp,
 // thread (XITEM, see k_ac3d_xstrip).
 enum XMode { XNONE = 0, XBODY = 1, XITEM = 2 };
 template <int MODE, int NW, bool FAST = false, int REGION = 0, bool PIPE = true, int XS = XNONE>
-__device__ __forceinline__ void ac3d_body(const StepArgs& A, long long block) {
+__device__ __forceinline__ void ac3d_body(const StepArgs& A, long long block, unsigned tid) {
   constexpr unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int S = A.nshots;
   const int nx = A.n0, ny = A.n1, nz = A.n2, P = A.P, H = A.halo;
   int nl = 0, xr = 0, ng = 0;  // the x strips' groups
   if (XS != XNONE) xstrip_groups(nx, H, P, nl, xr, ng);
   int shot, wx0 = 0, x0, y, z_begin, z_end;
   if (XS == XITEM) {
-    const long long item = block * (32 * NW) + threadIdx.x;
+    const long long item = block * (32 * NW) + tid;
     const int g = (int)(item % ng);
     long long rest = item / ng;
     y = 1 + (int)(rest % (ny - 2));
@@ -1827,11 +1827,11 @@ __device__ __forceinline__ void ac3d_body(const StepArgs& A, long long block) {
 // register choice (1.96 against 1.76 TB/s).
 template <int MODE, int NW = 4>
 __global__ void __launch_bounds__(32 * NW, 24 / NW) k_ac3d_step(const StepArgs A) {
-  ac3d_body<MODE, NW>(A, blockIdx.x);
+  ac3d_body<MODE, NW>(A, blockIdx.x, threadIdx.x);
 }
 template <int MODE, int NW = 4>
 __global__ void __launch_bounds__(32 * NW) k_ac3d_fwd(const StepArgs A) {
-  ac3d_body<MODE, NW, true>(A, blockIdx.x);
+  ac3d_body<MODE, NW, true>(A, blockIdx.x, threadIdx.x);
 }
 // The 3D step in two launches.  k_ac3d_xstrip advances the groups of four
 // points that meet an x strip, one (group, y, z, shot) per thread; k_ac3d_main
@@ -1849,24 +1849,23 @@ __global__ void __launch_bounds__(32 * NW) k_ac3d_fwd(const StepArgs A) {
 template <int MODE>
 __global__ void __launch_bounds__(128, 5) k_ac3d_xstrip(const StepArgs A) {
   chain_next();
-  chain_wait();
-  ac3d_body<MODE, 4, false, 0, false, XITEM>(A, blockIdx.x);
+  ac3d_body<MODE, 4, false, 0, false, XITEM>(A, blockIdx.x, chain_wait_tid());
 }
 template <int MODE, int NW = 4>
 __global__ void __launch_bounds__(32 * NW, 32 / NW) k_ac3d_main(const StepArgs A) {
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   long long b = blockIdx.x;
   if (b < A.b_z) {
-    ac3d_body<MODE, NW, false, 2, false, XBODY>(A, b);
+    ac3d_body<MODE, NW, false, 2, false, XBODY>(A, b, tid);
     return;
   }
   b -= A.b_z;
   if (b < A.b_y) {
-    ac3d_body<MODE, NW, false, 3, false, XBODY>(A, b);
+    ac3d_body<MODE, NW, false, 3, false, XBODY>(A, b, tid);
     return;
   }
-  ac3d_body<MODE, NW, false, 1, false, XBODY>(A, b - A.b_y);
+  ac3d_body<MODE, NW, false, 1, false, XBODY>(A, b - A.b_y, tid);
 }
 
 // ---------------------------------------------------------------------------
@@ -2317,9 +2316,9 @@ __device__ __forceinline__ void cpml_corr64_x4(ff (&t)[4], const float (&ch)[4],
 // us per step with this split and the strips' memory variables loaded with
 // the row, 4 shots of 901 x 455 87 -> 44, 2 of 183 x 157 x 141 1170 -> 556.
 template <int MODE, int NDIM, bool XS, bool ITEM>
-__device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
+__device__ __forceinline__ void hp_body(const StepArgs& A, long long item, unsigned tid) {
   constexpr unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int S = A.nshots;
   const int nx = A.n0, P = A.P, H = A.halo;
   const int nm = NDIM == 2 ? A.n1 : A.n2;  // marching axis
@@ -2524,7 +2523,7 @@ __device__ __forceinline__ void hp_body(const StepArgs& A, long long item) {
 
 template <int MODE, int NDIM>
 __device__ __noinline__ void hp_xstrip_item(const StepArgs& A, long long item) {
-  hp_body<MODE, NDIM, true, true>(A, item);
+  hp_body<MODE, NDIM, true, true>(A, item, 0);
 }
 
 // XS: the x strips in blocks of their own (always in 2D; in 3D unless the FP16
@@ -2533,15 +2532,15 @@ template <int MODE, int NDIM, bool XS>
 __global__ void __launch_bounds__(128, NDIM == 2 ? 6 : XS ? 4 : 1) k_ac_hp(const StepArgs A) {
   static_assert(MODE == MODE_FWD || MODE == MODE_FWD_D, "compensated step: forward modes only");
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   if constexpr (XS) {
     const long long nb_main = (long long)A.nshots * A.tiles_x * A.tiles_y * A.tiles_z;
     if ((long long)blockIdx.x >= nb_main) {
-      hp_xstrip_item<MODE, NDIM>(A, ((long long)blockIdx.x - nb_main) * 128 + threadIdx.x);
+      hp_xstrip_item<MODE, NDIM>(A, ((long long)blockIdx.x - nb_main) * 128 + tid);
       return;
     }
   }
-  hp_body<MODE, NDIM, XS, false>(A, 0);
+  hp_body<MODE, NDIM, XS, false>(A, 0, tid);
 }
 
 }  // namespace swgb

@@ -23,7 +23,8 @@
 // earlier kernel of the chain reads or writes (so a kernel completes after its
 // predecessor, and its successor's wait covers the whole chain); the tables
 // read before the wait are uploaded by copies or memsets, which the first
-// kernel of a chain waits for in full.  A kernel launched plainly, a copy or
+// kernel of a chain waits for in full; a kernel that reads what the loop writes
+// through the read-only path takes its thread index from chain_wait_tid.  A kernel launched plainly, a copy or
 // a memset waits for everything before it as always, and chain_wait in a
 // plainly launched kernel returns at once.
 #pragma once
@@ -38,6 +39,15 @@ namespace swgb {
 
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// chain_wait, giving the thread's index in its block.  Loads through the
+// read-only path (__ldg, const __restrict__) are invariant to the compiler, so
+// no memory clobber keeps it from moving them up past the wait; a load whose
+// address is formed with this index cannot move.
+__device__ __forceinline__ unsigned chain_wait_tid() {
+  unsigned t = threadIdx.x;
+  asm volatile("griddepcontrol.wait;" : "+r"(t) : : "memory");
+  return t;
+}
 
 template <typename... P, typename... Q>
 void launch_chain(const char* what, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, Q&&... args) {

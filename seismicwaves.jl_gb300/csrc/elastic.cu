@@ -443,11 +443,11 @@ __device__ __forceinline__ unsigned xmask_half(const Geo& g, int i0) {
 // (79.4 ms).
 __global__ void __launch_bounds__(BX, 5) k_el_stress4(const Args A) {
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
   const int j0 = blockIdx.y * A.tz + 1;
   const int j1 = min(j0 + A.tz - 1, g.nz - 1);
@@ -597,11 +597,11 @@ struct ElDispBounds {
 template <int COMP>
 __global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const Args A) {
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
   const int j0 = blockIdx.y * A.tz + 1;
   const int j1 = min(j0 + A.tz - 1, g.nz);
@@ -921,17 +921,16 @@ __global__ void k_el_record(const ShotDesc* __restrict__ desc, int it, long long
   const ShotDesc& D = desc[s];
   const bool on = it <= D.nt;
   const float inv_scale = 1.0f / D.sf;
-  const long long so = (long long)s * F;
   const int q = blockIdx.x * blockDim.x + threadIdx.x;  // the grid covers every receiver component
   const int t = q & 1, r = q >> 1;
   const bool mine = on && q < 2 * D.nrec;
-  const float* u = (t == 0 ? ux : uz) + so;
   const long long* lin = D.rlin[t];
   const float* coef = D.rcoef[t];
   const int e0 = mine ? D.rptr[t][r] : 0, e1 = mine ? D.rptr[t][r + 1] : 0;
-  chain_wait();
+  const long long so = (long long)s * F + (chain_wait_tid() - threadIdx.x);  // zero, known after the wait only
   chain_next();
   if (!mine) return;
+  const float* u = (t == 0 ? ux : uz) + so;
   float acc = 0.0f;
 #pragma unroll 8
   for (int e = e0; e < e1; ++e) acc = __fmaf_rn(coef[e], u[lin[e]], acc);
@@ -1136,10 +1135,10 @@ __global__ void __launch_bounds__(BX) k_el_corr(const CorrArgs A) {
 // the warp edges); the z re-reads of neighbouring rows hit L1/L2.
 __global__ void __launch_bounds__(BX) k_el_corr4(const CorrArgs A) {
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
   const int grp = blockIdx.z;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int wx0 = (blockIdx.x * 4 + warp) * 128;
   const int j = blockIdx.y + 1;
   if (wx0 >= g.nx || j > g.nz) return;  // warp uniform; no block-level synchronisation

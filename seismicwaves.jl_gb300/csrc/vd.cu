@@ -234,11 +234,11 @@ struct VdPBounds {
 template <bool CORR>
 __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs A) {
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
   const int j0 = blockIdx.y * A.tz + 1;
   const int j1 = min(j0 + A.tz - 1, g.nz);
@@ -362,11 +362,11 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
 // handling of the memory variables as k_vd_p.
 __global__ void __launch_bounds__(BX, 7) k_vd_v(const VArgs A) {
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
   const int j0 = blockIdx.y * A.tz + 1;
   const int j1 = min(j0 + A.tz - 1, g.nz);
@@ -492,10 +492,10 @@ __device__ __forceinline__ ff cpml_upd64(double* psi, double a, double b, ff dv)
 template <int TZ>
 __global__ void __launch_bounds__(BX) k_vd_p_hp(const HArgs A) {
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
   const int s = blockIdx.z;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int wx0 = (blockIdx.x * 4 + warp) * 128;
   const int j0 = blockIdx.y * TZ + 1;
   const int j1 = min(j0 + TZ - 1, g.nz);
@@ -588,10 +588,10 @@ __global__ void __launch_bounds__(BX) k_vd_p_hp(const HArgs A) {
 template <int TZ>
 __global__ void __launch_bounds__(BX) k_vd_v_hp(const HArgs A) {
   chain_next();
-  chain_wait();
+  const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
   const int s = blockIdx.z;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const int wx0 = (blockIdx.x * 4 + warp) * 128;
   const int j0 = blockIdx.y * TZ + 1;
   const int j1 = min(j0 + TZ - 1, g.nz);
