@@ -411,7 +411,7 @@ int sw_acoustic_vd_forward_snapshots(sw_acoustic_vd* vd, int32_t nshots, const s
 int sw_acoustic_vd_gradient(sw_acoustic_vd* vd, int32_t nshots, const sw_acoustic_shot* shots, int32_t on_device,
                             double* grad_vp, double* grad_rho, double* misfit);
 /* Rows per thread block of the VD stencil kernels: 8, 16 or 32 (0 = default:
- * 4, fewer for launches that would leave SMs short of warps).  A tuning knob
+ * 3, fewer for launches that would leave SMs short of warps).  A tuning knob
  * of this backend; results do not depend on it. */
 int sw_acoustic_vd_set_tuning(sw_acoustic_vd* vd, int32_t tz);
 

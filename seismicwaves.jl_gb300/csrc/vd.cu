@@ -210,6 +210,13 @@ __device__ __forceinline__ unsigned xmask_vel(const Geo& g, int i0) {
   return m;
 }
 
+// The rows of a band (up to 8) of a warp's 128 columns of one array on their
+// way into L2: one line per lane, no registers held (see k_vd_p).
+__device__ __forceinline__ void prefetch_band(const float* p, int P, int rows, int cols, int lane) {
+  const int r = lane >> 2, x = (lane & 3) * 32;
+  if (r < rows && x < cols) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + r * P + x));
+}
+
 // Pressure update (update_p_CPML! on 2:nx-1, 2:nz-1; every other node copies
 // p through): four x points per thread, each warp 128 consecutive points, a
 // block 512 points x tz rows of one shot (x tiles fastest, then shots, then
@@ -223,12 +230,16 @@ __device__ __forceinline__ unsigned xmask_vel(const Geo& g, int i0) {
 // point they were a chain of four dependent loads per axis and row, which set
 // the time of every row next to a strip (one shot of 402 x 301, 600 steps:
 // 27.4 -> 14.9 ms with the same 8-row bands; 8 shots of 2001 x 801, 300 steps,
-// gradient: 120.8 -> 97.1 ms).  Bound by HBM latency and bandwidth: 7 resident
-// blocks per SM (6 for the correlating kernel, which holds two z windows)
-// against 96.0 ms run 99.1 at 6 / 6 and 96.3 at 7 / 5; at 8 / 7 the kernels spill.
+// gradient: 120.8 -> 97.1 ms).  Bound by HBM latency: a warp asks for all
+// rows of its band at the start (prefetch_band), so that the loads of the rows
+// after the first find them in L2 (the same gradient 88.8 -> 78.1 ms, with 3
+// rows per band where 4 were best without).  7 resident blocks per SM, 6 of
+// k_vd_v, 5 of the correlating kernel, which holds two z windows: 80.3 ms with
+// 7 / 7 / 5 and 4 rows, 83.1 with 7 / 7 / 6, 80.9 with 7 / 7 / 4, 84.4 with
+// 8 / 8 / 6, where the kernels spill.
 template <bool CORR>
 struct VdPBounds {
-  static constexpr int MINB = CORR ? 6 : 7;
+  static constexpr int MINB = CORR ? 5 : 7;
 };
 
 template <bool CORR>
@@ -246,6 +257,20 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
   const int i0 = wx0 + lane * 4 + 1;
   const bool ldok = i0 <= g.nx + 2;
   const long long so = (long long)s * g.F;
+  if (j1 > j0) {
+    const long long o = g.lin(wx0 + 1, j0);
+    const int n = j1 - j0 + 1, w = g.nx - wx0;
+    prefetch_band(A.vx + so + o, g.P, n, w, lane);
+    prefetch_band(A.pin + so + o, g.P, n, w, lane);
+    prefetch_band(A.vz + so + o + g.P, g.P, n, w, lane);
+    prefetch_band(A.m0 + o, g.P, n, w, lane);
+    if (CORR) {
+      prefetch_band(A.po + so + o, g.P, n, w, lane);
+      prefetch_band(A.pc + so + o + 2 * g.P, g.P, n, w, lane);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) prefetch_band(A.acc + 3 * so + q * g.F + o, g.P, n, w, lane);
+    }
+  }
   const float* __restrict__ vx = A.vx + so;
   const float* __restrict__ vz = A.vz + so;
   const float* pin = A.pin + so;
@@ -360,7 +385,7 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
 // Velocity update (update_vx_CPML! on 1:nx-1 x 1:nz, update_vy_CPML! on
 // 1:nx x 1:nz-1); p rows j-1 .. j+2 in registers, the same split and the same
 // handling of the memory variables as k_vd_p.
-__global__ void __launch_bounds__(BX, 7) k_vd_v(const VArgs A) {
+__global__ void __launch_bounds__(BX, 6) k_vd_v(const VArgs A) {
   chain_next();
   const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
@@ -374,6 +399,15 @@ __global__ void __launch_bounds__(BX, 7) k_vd_v(const VArgs A) {
   const int i0 = wx0 + lane * 4 + 1;
   const bool ldok = i0 <= g.nx + 2;
   const long long so = (long long)s * g.F;
+  if (j1 > j0) {
+    const long long o = g.lin(wx0 + 1, j0);
+    const int n = j1 - j0 + 1, w = g.nx - wx0;
+    prefetch_band(A.vx + so + o, g.P, n, w, lane);
+    prefetch_band(A.m1x + o, g.P, n, w, lane);
+    prefetch_band(A.vz + so + o, g.P, n, w, lane);
+    prefetch_band(A.m1z + o, g.P, n, w, lane);
+    prefetch_band(A.p + so + o + 2 * g.P, g.P, n, w, lane);
+  }
   const float* __restrict__ p = A.p + so;
   float* vx = A.vx + so;
   float* vz = A.vz + so;
@@ -1387,17 +1421,15 @@ void zero_state(sw_acoustic_vd* vd, int S, bool adjoint) {
 
 // Rows per block of the VD stencils.  A warp's rows run one after the other
 // (about 2 us each where the fields sit in L2), and a band re-reads the 3 rows
-// of its z window: 4 rows are fastest where the launch fills the GPU (8 x 2001
-// x 801 gradient: 97.9 ms with 2 rows, 96.0 with 4, 98.4 with 8); a launch of
-// fewer than 16 warps per SM takes shorter bands (one shot of 402 x 301: 14.9
-// us per step with 8 rows, 10.0 with 4, 7.5 with 1).
+// of its z window: 3 rows are fastest where the launch fills the GPU (8 x 2001
+// x 801 gradient: 79.9 ms with 2 rows, 78.1 with 3, 80.3 with 4, 93.5 with 8);
+// a launch of fewer than 16 warps per SM takes single rows (one shot of 402 x
+// 301: 14.9 us per step with 8 rows, 10.0 with 4, 7.5 with 1).
 int band_rows(const sw_acoustic_vd* vd, int S) {
   if (vd->tz > 0) return vd->tz;
   const int sms = vd->ctx->num_sms > 0 ? vd->ctx->num_sms : 148;
   const long long wx = (vd->g.nx + 127) / 128;
-  int tz = 4;
-  while (tz > 1 && S * wx * ((vd->g.nz + tz - 1) / tz) < 16LL * sms) tz /= 2;
-  return tz;
+  return S * wx * ((vd->g.nz + 2) / 3) < 16LL * sms ? 1 : 3;
 }
 
 struct Run {
