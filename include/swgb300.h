@@ -283,8 +283,7 @@ int sw_profile_enable(sw_ctx* ctx, int32_t on);
 int sw_profile_read(sw_ctx* ctx, int32_t kind, double* total_ms, int64_t* launches, double* bytes);
 /* Kernel launches inside the brackets that sw_profile_read counts as
  * `launches` (one bracket per step of a kind; the 3D step as two launches,
- * the variable-density adjoint pair and the elastic displacement pair launch
- * several kernels). */
+ * the variable-density and the elastic adjoint steps launch several kernels). */
 int sw_profile_read_kernels(sw_ctx* ctx, int32_t kind, int64_t* kernels);
 
 /* ---------------------------------------------------------------------------
@@ -372,9 +371,9 @@ int sw_elastic_forward_snapshots(sw_elastic* es, int32_t nshots, const sw_elasti
 /* Rows per thread block of the elastic stencil kernels: 8, 16 or 32 (0 =
  * default: 4, fewer for launches that would leave SMs short of warps; 8 for
  * the one-point kernels); + 64 selects the one-point-per-thread kernels
- * instead of the four-points-per-thread ones.  The four-point displacement
- * update runs as two launches (ux, then uz; 80 registers each, 6 resident
- * blocks per SM); + 128 selects the single launch.  A tuning knob of this backend; no reference counterpart. */
+ * instead of the four-points-per-thread ones.  The four-point kernels update
+ * ux and uz by blocks of their own; + 128 by the same threads.  A tuning knob
+ * of this backend; no reference counterpart. */
 int sw_elastic_set_tuning(sw_elastic* es, int32_t tz);
 
 /* ---------------------------------------------------------------------------

@@ -430,6 +430,59 @@ __device__ __forceinline__ unsigned xmask_half(const Geo& g, int i0) {
   return m;
 }
 
+// Unique-point CSR of one injection table: point p (padded index lin[p]) gets
+// sum over e in [ptr[p], ptr[p+1]) of coef[e] * tf(item[e]).
+struct Inj {
+  int np;
+  const long long* lin;
+  const int* ptr;
+  const int* item;
+  const float* coef;
+};
+
+struct ShotDesc {
+  int nt, kind, nsrc, nrec;
+  const float* tf;  // srctf, device: kind 0 (nt, nsrc), kind 1 (nt, 2, nsrc)
+  const float* mtp; // (3, nsrc) moment tensors, device
+  float sf;         // this shot's source scale (a power of two)
+  Inj src[2];       // sources: kind 0 -> sigma grids, kind 1 -> ux / uz grids
+  Inj adj[2];       // receivers as adjoint forces on ux / uz
+  const int* rptr[2];        // recording CSR by receiver (nrec+1)
+  const long long* rlin[2];
+  const float* rcoef[2];
+  float* tr;                 // traces (nt, 2, nrec)
+  const float* obs;          // observed
+  const float* ic;           // diagonal inverse covariance or null
+  const float* mask;         // window mask (nt) or null
+  float* adjsrc;             // adjoint source (nt, 2, nrec)
+  const float* icd;          // dense inverse covariance (nt, nt) or null
+  float* resid;              // dense case: masked residuals (nt, 2 nrec)
+  const float* cres;         // dense case: C^-1 r (nt, 2 nrec), from the dense product (dense.cu)
+  int mkind;                 // 0 L2, 1 CCTS (k_ccts writes this shot's adjoint source)
+};
+
+// trace(it, comp, r) = sum_e w_e u(p_e), scaled back by the shot's source
+// scale: receiver component q (component q & 1 of receiver q >> 1) of shot s.
+struct RecordArgs {
+  const ShotDesc* desc;
+  int it;      // 0: nothing to record
+  int nshots;  // shots active at step it
+  int bands;   // the stress bands of the launch (blockIdx.y from here on records)
+};
+__device__ __forceinline__ void record_one(const ShotDesc& D, int it, long long so, const float* ux,
+                                           const float* uz, int q) {
+  if (it > D.nt || q >= 2 * D.nrec) return;
+  const float inv_scale = 1.0f / D.sf;
+  const int t = q & 1, r = q >> 1;
+  const float* u = (t == 0 ? ux : uz) + so;
+  const long long* lin = D.rlin[t];
+  const float* coef = D.rcoef[t];
+  float acc = 0.0f;
+#pragma unroll 8
+  for (int e = D.rptr[t][r], e1 = D.rptr[t][r + 1]; e < e1; ++e) acc = __fmaf_rn(coef[e], u[lin[e]], acc);
+  D.tr[(long long)(it - 1) + (long long)D.nt * (t + 2LL * r)] = acc * inv_scale;
+}
+
 // Blocks of 512 points x A.tz rows of one shot, x tiles fastest, then shots,
 // then bands (the shots of a band share the material rows through L2).  The
 // memory variables of a thread's four points are one float4 along either
@@ -438,13 +491,21 @@ __device__ __forceinline__ unsigned xmask_half(const Geo& g, int i0) {
 // the time of every row next to a strip (one shot of 333 x 217, 400-step
 // gradient: 94.3 -> 44.7 ms with the same 8-row bands; 8 shots of 1200 x 600, 200
 // steps, gradient: 107.3 -> 82.1 ms).  Bound by HBM latency and bandwidth; 5
-// resident blocks per SM and 6 of the displacement halves: with 6 / 7 the
-// kernels spill (80.2 against 77.3 ms), with 4 / 5 too few rows are in flight
-// (79.4 ms).
-__global__ void __launch_bounds__(BX, 5) k_el_stress4(const Args A) {
+// resident blocks per SM (with 6 it spills: 80.2 against 77.3 ms, with 4 too
+// few rows are in flight: 79.4).  The blocks from band R.bands on record the
+// step before (record_one): the stress update leaves the displacements alone,
+// and a launch of its own is a link of the chain (two shots of 601 x 397, 500
+// steps: 7.8 ms against 9.4).
+__global__ void __launch_bounds__(BX, 5) k_el_stress4(const Args A, const RecordArgs R) {
   chain_next();
   const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
+  if ((int)blockIdx.y >= R.bands) {
+    const long long b = (long long)(blockIdx.y - R.bands) * gridDim.x + blockIdx.x;
+    const int rs = (int)(b % R.nshots);
+    record_one(R.desc[rs], R.it, (long long)rs * g.F, A.ux, A.uz, (int)(b / R.nshots) * BX + (int)tid);
+    return;
+  }
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
   const int lane = tid & 31, warp = tid >> 5;
@@ -587,22 +648,15 @@ __global__ void __launch_bounds__(BX, 5) k_el_stress4(const Args A) {
   }
 }
 
-// COMP: 2 updates ux and uz; 0 only ux, 1 only uz (two launches with fewer
-// registers each: the uz half loads no sigma_xx and no sigma_xz column, the ux
-// half no sigma_zz)
+// COMP: 2 updates ux and uz, 0 only ux, 1 only uz (the uz half loads no
+// sigma_xx and no sigma_xz column, the ux half no sigma_zz).
 template <int COMP>
-struct ElDispBounds {
-  static constexpr int MINB = COMP == 2 ? 5 : 6;
-};
-template <int COMP>
-__global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const Args A) {
-  chain_next();
-  const unsigned tid = chain_wait_tid();
+__device__ __forceinline__ void el_disp4(const Args& A, unsigned tid, int bx) {
   const Geo g = A.g;
   const int tx = (g.nx + 511) / 512;
-  const int s = blockIdx.x / tx;
+  const int s = bx / tx;
   const int lane = tid & 31, warp = tid >> 5;
-  const int wx0 = ((blockIdx.x - s * tx) * 4 + warp) * 128;
+  const int wx0 = ((bx - s * tx) * 4 + warp) * 128;
   const int j0 = blockIdx.y * A.tz + 1;
   const int j1 = min(j0 + A.tz - 1, g.nz);
   if (j0 > j1 || wx0 >= g.nx) return;
@@ -800,40 +854,31 @@ __global__ void __launch_bounds__(BX, ElDispBounds<COMP>::MINB) k_el_disp4(const
   }
 }
 
+__global__ void __launch_bounds__(BX, 5) k_el_disp4_both(const Args A) {
+  chain_next();
+  el_disp4<2>(A, chain_wait_tid(), blockIdx.x);
+}
+// The two halves of the displacement update, which do not touch each other's
+// arrays, as neighbouring blocks of one launch: each needs fewer registers
+// than both together, the sigma_xz rows that both read stay in L1 / L2
+// between them, and the step is one link shorter than with a launch each.
+// With the recording on the stress launch: two shots of 601 x 397, 500 steps,
+// 9.75 -> 7.7 ms (9.4 of it by this), one shot of 333 x 217, gradient, 14.4 ->
+// 10.8 (13.1 -> 11.9), 8 shots of 1200 x 600, gradient, 71.3 -> 66.9 (-> 69.6).
+// Bound by the latency of a warp's rows: 7 blocks per SM (8 spilled words;
+// the batch 68.5 ms with 6, 69.9 with 5).
+__global__ void __launch_bounds__(BX, 7) k_el_disp4_halves(const Args A) {
+  chain_next();
+  const unsigned tid = chain_wait_tid();
+  const bool z = blockIdx.x & 1;
+  const int b = blockIdx.x >> 1;
+  if (z) el_disp4<1>(A, tid, b);
+  else el_disp4<0>(A, tid, b);
+}
+
 // ---------------------------------------------------------------------------
 // Sources, receivers, misfit
 // ---------------------------------------------------------------------------
-// Unique-point CSR of one injection table: point p (padded index lin[p]) gets
-// sum over e in [ptr[p], ptr[p+1]) of coef[e] * tf(item[e]).
-struct Inj {
-  int np;
-  const long long* lin;
-  const int* ptr;
-  const int* item;
-  const float* coef;
-};
-
-struct ShotDesc {
-  int nt, kind, nsrc, nrec;
-  const float* tf;  // srctf, device: kind 0 (nt, nsrc), kind 1 (nt, 2, nsrc)
-  const float* mtp; // (3, nsrc) moment tensors, device
-  float sf;         // this shot's source scale (a power of two)
-  Inj src[2];       // sources: kind 0 -> sigma grids, kind 1 -> ux / uz grids
-  Inj adj[2];       // receivers as adjoint forces on ux / uz
-  const int* rptr[2];        // recording CSR by receiver (nrec+1)
-  const long long* rlin[2];
-  const float* rcoef[2];
-  float* tr;                 // traces (nt, 2, nrec)
-  const float* obs;          // observed
-  const float* ic;           // diagonal inverse covariance or null
-  const float* mask;         // window mask (nt) or null
-  float* adjsrc;             // adjoint source (nt, 2, nrec)
-  const float* icd;          // dense inverse covariance (nt, nt) or null
-  float* resid;              // dense case: masked residuals (nt, 2 nrec)
-  const float* cres;         // dense case: C^-1 r (nt, 2 nrec), from the dense product (dense.cu)
-  int mkind;                 // 0 L2, 1 CCTS (k_ccts writes this shot's adjoint source)
-};
-
 // sigma_xx += Mxx w tf, sigma_zz += Mzz w tf (table 0), sigma_xz += Mxz w tf (table 1)
 __global__ void k_el_inject_sigma(const ShotDesc* __restrict__ desc, int it, long long F, float* sxx, float* szz,
                                   float* sxz) {
@@ -914,27 +959,13 @@ __global__ void k_el_inject_force(const ShotDesc* __restrict__ desc, int it, int
   }
 }
 
-// trace(it, comp, r) = sum_e w_e u(p_e), scaled back by the shot's source scale
-__global__ void k_el_record(const ShotDesc* __restrict__ desc, int it, long long F, const float* __restrict__ ux,
-                            const float* __restrict__ uz) {
+// The recording of the loop's last step (and of the one-point kernels' steps).
+__global__ void k_el_record(const ShotDesc* __restrict__ desc, int it, long long F, const float* ux,
+                            const float* uz) {
   const int s = blockIdx.y;
-  const ShotDesc& D = desc[s];
-  const bool on = it <= D.nt;
-  const float inv_scale = 1.0f / D.sf;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;  // the grid covers every receiver component
-  const int t = q & 1, r = q >> 1;
-  const bool mine = on && q < 2 * D.nrec;
-  const long long* lin = D.rlin[t];
-  const float* coef = D.rcoef[t];
-  const int e0 = mine ? D.rptr[t][r] : 0, e1 = mine ? D.rptr[t][r + 1] : 0;
-  const long long so = (long long)s * F + (chain_wait_tid() - threadIdx.x);  // zero, known after the wait only
+  chain_wait();
   chain_next();
-  if (!mine) return;
-  const float* u = (t == 0 ? ux : uz) + so;
-  float acc = 0.0f;
-#pragma unroll 8
-  for (int e = e0; e < e1; ++e) acc = __fmaf_rn(coef[e], u[lin[e]], acc);
-  D.tr[(long long)(it - 1) + (long long)D.nt * (t + 2LL * r)] = acc * inv_scale;
+  record_one(desc[s], it, (long long)s * F, ux, uz, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The power of two 2^e with 2^e * max|C^-1 r| close to 2^20 (1 for a zero or
@@ -1232,19 +1263,24 @@ __global__ void __launch_bounds__(BX) k_el_corr4(const CorrArgs A) {
     }
   }
   if (!ldok) return;
+  // bit e: point e is a ux node, a uz node, an inner normal-stress node
+  const unsigned mux = i0 + 3 <= g.nx - 1 ? 15u : i0 > g.nx - 1 ? 0u : (1u << (g.nx - i0)) - 1u;
+  const unsigned muz = !on_uz ? 0u : i0 + 3 <= g.nx ? 15u : i0 > g.nx ? 0u : (1u << (g.nx + 1 - i0)) - 1u;
+  const unsigned mxx = on_uz && j >= jlo ? mux & (i0 == 1 ? 14u : 15u) : 0u;
+  auto add = [&](int q, const float (&y)[4], float f, unsigned m) {
+    if (!m) return;
+    F4 G = ld4rwz(acc + q * g.F, c), C = ld4rwz(acc + (q + 5) * g.F, c);
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int i = i0 + e;
-    const long long ce = c + e;
-    const bool on_ux = i <= g.nx - 1;
-    if (on_ux) kahan_add_el(acc + ce, acc + 5 * g.F + ce, fs1 ? 0.5f * v[0][e] : v[0][e]);
-    if (on_uz && i <= g.nx) kahan_add_el(acc + g.F + ce, acc + 6 * g.F + ce, v[1][e]);
-    if (i >= 2 && i <= g.nx - 1 && j >= jlo && on_uz) {
-      kahan_add_el(acc + 2 * g.F + ce, acc + 7 * g.F + ce, fs1 ? 0.5f * v[2][e] : v[2][e]);
-      kahan_add_el(acc + 3 * g.F + ce, acc + 8 * g.F + ce, fs1 ? v[3][e] : 2.0f * v[3][e]);
-    }
-    if (on_ux && on_uz) kahan_add_el(acc + 4 * g.F + ce, acc + 9 * g.F + ce, v[4][e]);
-  }
+    for (int e = 0; e < 4; ++e)
+      if (m >> e & 1) kahan_add_el(&G.v[e], &C.v[e], __fmul_rn(f, y[e]));
+    st4v(acc + q * g.F, c, G.v);
+    st4v(acc + (q + 5) * g.F, c, C.v);
+  };
+  add(0, v[0], fs1 ? 0.5f : 1.0f, mux);
+  add(1, v[1], 1.0f, muz);
+  add(2, v[2], fs1 ? 0.5f : 1.0f, mxx);
+  add(3, v[3], fs1 ? 1.0f : 2.0f, mxx);
+  add(4, v[4], 1.0f, on_uz ? mux : 0u);
 }
 
 // One snapshot block per shot (blockIdx.y): ux, uz, sxx, szz, sxz unpadded and
@@ -1410,7 +1446,7 @@ struct sw_elastic {
   float* const* snap_out = nullptr;  // per caller shot: nt/snapevery blocks [ux, uz, sxx, szz, sxz]
   int tz = 0;  // rows per block of the stencil kernels (0: band_rows; 8, 16 or 32)
   bool vec = true;  // four x points per thread (k_el_*4) instead of one
-  bool split_disp = true;  // the displacement update as two launches, ux then uz (tz + 128: one launch)
+  bool split_disp = true;  // ux and uz updated by blocks of their own (tz + 128: by the same threads)
   DevMem d_scales;        // [0] the forward sources' common scale, [1] the adjoint source's scale
   DevMem d_ccts, d_partial2;  // CCTS descriptors and per-trace misfit terms
   DevMem d_gout, d_mout;  // gradient / misfit of the host-buffer path (stable addresses for the graphs)
@@ -1860,7 +1896,12 @@ struct Run {
     }
     gx_src = (ns + 127) / 128;
     gx_adj = (na + 127) / 128;
-    gx_rec = (nr + 63) / 64;
+    gx_rec = (nr + BX - 1) / BX;
+  }
+  RecordArgs rec{};  // a recording that the next stress launch takes along
+  void flush_record() {
+    if (rec.it > 0) record(rec.nshots, rec.it);
+    rec.it = 0;
   }
 
   Args args(bool adjoint) const {
@@ -1914,7 +1955,7 @@ struct Run {
     if (S <= 0) return;
     cudaEvent_t ev = nullptr;
     es->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    launch_chain("record launch", k_el_record, dim3(gx_rec, S), dim3(64), st, ddesc, it, es->g.F, es->st[0].as<float>(),
+    launch_chain("record launch", k_el_record, dim3(gx_rec, S), dim3(BX), st, ddesc, it, es->g.F, es->st[0].as<float>(),
                  es->st[1].as<float>());
     es->ctx->prof.end(st, KK_SRCREC, ev);
   }
@@ -1954,20 +1995,19 @@ void launch_scalar(const sw_elastic* es, cudaStream_t st, const Args& a, int S, 
   else k_el_disp<TZ><<<grid, BX, 0, st>>>(a);
 }
 
-// returns the number of kernels launched
-int launch_stencil(const sw_elastic* es, cudaStream_t st, Args a, int S, bool stress) {
-  int nk = 1;
+void launch_stencil(const sw_elastic* es, cudaStream_t st, Args a, int S, bool stress, RecordArgs rec = {},
+                   int gx_rec = 0) {
   if (es->vec) {  // four points per thread: 512 per block
     a.tz = band_rows(es, S);
     const dim3 grid((unsigned)((es->g.nx + 511) / 512 * S), (unsigned)((es->g.nz + a.tz - 1) / a.tz));
     if (stress) {
-      launch_chain("stress launch", k_el_stress4, grid, dim3(BX), st, a);
-    } else if (es->split_disp) {  // ux and uz updates as two launches
-      launch_chain("displacement launch", k_el_disp4<0>, grid, dim3(BX), st, a);
-      launch_chain("displacement launch", k_el_disp4<1>, grid, dim3(BX), st, a);
-      nk = 2;
+      rec.bands = (int)grid.y;
+      const unsigned rb = rec.it > 0 ? ((unsigned)gx_rec * rec.nshots + grid.x - 1) / grid.x : 0;
+      launch_chain("stress launch", k_el_stress4, dim3(grid.x, grid.y + rb), dim3(BX), st, a, rec);
+    } else if (es->split_disp) {
+      launch_chain("displacement launch", k_el_disp4_halves, dim3(2 * grid.x, grid.y), dim3(BX), st, a);
     } else {
-      launch_chain("displacement launch", k_el_disp4<2>, grid, dim3(BX), st, a);
+      launch_chain("displacement launch", k_el_disp4_both, grid, dim3(BX), st, a);
     }
   } else if (es->tz == 16) {
     launch_scalar<16>(es, st, a, S, stress);
@@ -1977,7 +2017,6 @@ int launch_stencil(const sw_elastic* es, cudaStream_t st, Args a, int S, bool st
     launch_scalar<8>(es, st, a, S, stress);
   }
   check_cuda(cudaGetLastError(), stress ? "stress launch" : "displacement launch");
-  return nk;
 }
 
 // stress, [sigma sources], displacement, [force sources], [recording]
@@ -1988,14 +2027,20 @@ void full_step(Run& R, int S, int it, bool record, int kind, float* sU[2], float
   if (sU) { a.sUx = sU[0]; a.sUz = sU[1]; a.sDx = sD[0]; a.sDz = sD[1]; }
   cudaEvent_t ev = nullptr;
   es->ctx->prof.begin(R.st, kind, 0.0, &ev);
-  launch_stencil(es, R.st, a, S, true);
+  launch_stencil(es, R.st, a, S, true, R.rec, R.gx_rec);
+  R.rec.it = 0;
   es->ctx->prof.end(R.st, kind, ev);
   if (R.any_mt) R.inject_sigma(S, it);
   es->ctx->prof.begin(R.st, kind, R.step_bytes(S, sU != nullptr), &ev);
-  const int nk = launch_stencil(es, R.st, a, S, false);
-  es->ctx->prof.end(R.st, kind, ev, nk);
+  launch_stencil(es, R.st, a, S, false);
+  es->ctx->prof.end(R.st, kind, ev);
   if (R.any_force) R.inject_force(S, it, false, nullptr, sD);
-  if (record) R.record(S, it);
+  if (!record) return;
+  if (es->vec) {  // step it's recording rides on the next stress launch, which leaves the displacements alone
+    R.rec = RecordArgs{R.ddesc, it, S, 0};
+    return;
+  }
+  R.record(S, it);
 }
 
 void adjoint_step(Run& R, int S, int it) {
@@ -2004,9 +2049,9 @@ void adjoint_step(Run& R, int S, int it) {
   Args a = R.args(true);
   cudaEvent_t ev = nullptr;
   es->ctx->prof.begin(R.st, KK_ADJOINT, R.step_bytes(S, false), &ev);
-  int nk = launch_stencil(es, R.st, a, S, true);
-  nk += launch_stencil(es, R.st, a, S, false);
-  es->ctx->prof.end(R.st, KK_ADJOINT, ev, nk);
+  launch_stencil(es, R.st, a, S, true);
+  launch_stencil(es, R.st, a, S, false);
+  es->ctx->prof.end(R.st, KK_ADJOINT, ev, 2);
   R.inject_force(S, it, true, es->d_scales.as<float>() + 1, nullptr);
 }
 
@@ -2229,6 +2274,7 @@ void elastic_forward(sw_elastic* es, int nshots, const sw_elastic_shot* shots, b
         full_step(R, A, it, true, KK_STENCIL, nullptr, nullptr);
         if (es->snapevery > 0 && it % es->snapevery == 0) save_snapshots(es, group, A, it);
       }
+      R.flush_record();
     };
     if (es->snapevery > 0) {  // host copies inside the loop: no graph
       body();
@@ -2443,6 +2489,7 @@ void elastic_gradient(sw_elastic* es, int nshots, const sw_elastic_shot* shots, 
         }
         if (it % K == 0 && it / K <= M - 1) save_ck(it / K);
       }
+      R.flush_record();
       // misfit and adjoint source
       check_cuda(cudaMemsetAsync(es->d_amax.p, 0, sizeof(unsigned), st), "max clear");
       {
@@ -2555,7 +2602,7 @@ void elastic_gradient(sw_elastic* es, int nshots, const sw_elastic_shot* shots, 
 
 void elastic_set_tuning(sw_elastic* es, int tz) {
   // tz = rows per block (8, 16, 32; 0 = band_rows); + 64 selects the one-point-per-thread kernels;
-  // + 128 runs the four-point displacement update as one launch instead of two (ux, uz)
+  // + 128 updates ux and uz by the same threads instead of by blocks of their own
   const int rows = tz % 64;
   if (tz < 0 || tz >= 256 || (rows != 0 && rows != 8 && rows != 16 && rows != 32))
     fail(SW_ERR_ARG, "tz must be 0, 8, 16 or 32, optionally + 64 and + 128");
