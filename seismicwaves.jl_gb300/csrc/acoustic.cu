@@ -207,6 +207,15 @@ __global__ void k_inject_record(const ShotDesc* __restrict__ desc, const long lo
   }
 }
 
+// The recording of the last step that carried its own sources (StepRide).
+__global__ void k_ride_record(const StepShot* __restrict__ shots, const long long* __restrict__ rec_lin, FieldArg p,
+                              int it) {
+  chain_wait();
+  chain_next();
+  const int s = blockIdx.y;
+  ride_record(shots[s], it, rec_lin, fptr(p, s), blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 // Adjoint injection at the receivers (adjoint_onestep_CPML! -> inject_sources!
 // with the prescaled residuals) and the matching correlation term: the fused
 // stencil correlated interior lambda before injection, so g += a * D is added
@@ -559,6 +568,9 @@ struct sw_wavesim {
   int pair_tz = 0;                        // rows per block of the two-step kernel (0 = heuristic)
   int pair_occ = 0;                       // resident-block bound of the two-step kernel (0 = default, 1, 2)
   bool pair_ok = false;                   // the current group's shots allow two-step launches
+  DevMem d_ride;                          // 2D forward steps with their sources and recording (StepShot per shot)
+  bool ride_ok = false;                   // the current group's shots allow them
+  int ride_rec = 0;                       // 128-receiver blocks of the largest shot
   DevMem adb2, axi2[3];                   // second adjoint d / xi buffers (two-step adjoint launches)
   DevMem d_amap;                          // [shot][k][P]: receiver point (CSR index) at x on receiver row k, or -1
   bool pair_adj_ok = false;               // ... and two-step adjoint launches
@@ -628,7 +640,8 @@ void run_graph(sw_wavesim* ws, std::vector<long long> key, Work&& work) {
 
 std::vector<long long> group_key(const sw_wavesim* ws, const std::vector<HostShot>& group, bool grad) {
   std::vector<long long> k = {grad ? 1 : 0, ws->grp, ws->variant, ws->tile_tz, ws->pf, ws->adjw ? 1 : 0,
-                              ws->cpa ? 1 : 0, ws->pair_ok ? 1 : 0, ws->pair_adj_ok ? 1 : 0, ws->pair_tz,
+                              ws->cpa ? 1 : 0, ws->ride_ok ? 1 + ws->ride_rec : 0, ws->pair_ok ? 1 : 0,
+                              ws->pair_adj_ok ? 1 : 0, ws->pair_tz,
                               ws->pair_occ, ws->kind_tz[0], ws->kind_tz[1], ws->kind_tz[2], ws->precision,
                               ws->split3d ? 1 : 0, ws->xsplit ? 1 : 0,
                               (long long)group.size()};
@@ -653,6 +666,7 @@ struct Tables {
   std::vector<HostShot> order;  // sorted by nt descending
   int max_nt = 0;
   std::vector<PairShot> pair;    // two-step launches: per shot sources and receiver rows
+  std::vector<StepShot> ride;    // steps with their sources and recording
   std::vector<int> recstash;     // per receiver: stash index k * P + x (k = its row's slot)
   bool pair_ok = false;
   std::vector<int> amap;         // adjoint: receiver point on each receiver row, per x
@@ -938,6 +952,42 @@ void build_tables(sw_wavesim* ws, const sw_acoustic_shot* shots, const std::vect
     ensure(ws, ws->d_stash, (size_t)S * PAIR_MAXRR * ws->P * sizeof(float), "receiver-row stash");
   }
   ws->pair_ok = T.pair_ok;
+  // 2D forward steps that add their sources and record the step before (see
+  // StepRide): the four-warp kernels of the plain step, at most STEP_MAXSP
+  // unique source points per shot, none on the outermost grid lines.  One link
+  // less in the chain of a step (one shot of 201 x 201: 4.06 us per step
+  // against 5.1; 4 of 801 x 801, gradient: 29.8 against 32.1 ms; 16 of 2001 x
+  // 801: 104.6 against 106.6).  Not between 16 and 64 rows of 128 points per
+  // SM, where the launch is one wave that the look for sources at the end of
+  // every warp lengthens (601 x 601: 16.0 against 15.4; 801 x 801: 30.8
+  // against 30.6).
+  const long long rows = (long long)S * ((ws->P + 127) / 128) * (ws->n[1] - 2);
+  const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
+  ws->ride_ok = ws->N == 2 && ws->precision == 0 && !T.pair_ok && ws->xsplit && !ws->cpa && (ws->variant & 7) == 0 &&
+                (rows < 16LL * sms || rows >= 64LL * sms);
+  ws->ride_rec = 1;
+  T.ride.assign(S, StepShot{});
+  for (int k = 0; k < S && ws->ride_ok; ++k) {
+    const ShotDesc& D = T.desc[k];
+    StepShot& q = T.ride[k];
+    if (D.nsp > STEP_MAXSP) ws->ride_ok = false;
+    for (int u = 0; u < STEP_MAXSP && ws->ride_ok; ++u) {
+      const bool on = u < D.nsp;
+      const long long lin = on ? T.pts[D.sp_off + u] : 0;
+      if (on && T.bslot[D.sp_off + u] >= 0) ws->ride_ok = false;
+      q.sx[u] = on ? (int)(lin % ws->P) : -4;
+      q.sz[u] = on ? (int)(lin / ws->P) : -4;
+      q.k0[u] = on ? T.ptr[D.sp_ptr + u] : 0;
+      q.k1[u] = on ? T.ptr[D.sp_ptr + u + 1] : 0;
+    }
+    q.tf = D.tf;
+    q.tr = D.tr;
+    q.nt = D.nt;
+    q.nrec = D.nrec;
+    q.rec_off = D.rec_off;
+    ws->ride_rec = std::max(ws->ride_rec, (D.nrec + 127) / 128);
+  }
+  if (ws->ride_ok) upload(ws, ws->d_ride, T.ride, "step shot table");
   ensure(ws, ws->d_ring, (size_t)std::max(3 * T.nring, 4) * sizeof(float), "boundary rings");
   for (int k = 0; k < S; ++k) T.desc[k].ring = ws->d_ring.as<float>() + 3LL * ring_off[k];
   upload(ws, ws->d_desc, T.desc, "shot descriptors");
@@ -1367,14 +1417,25 @@ long long xstrip_blocks(const StepArgs& a) {
 // headline).  A small launch (small_2d) takes the one-kernel form with
 // registers for every load of a row to be in flight.  Returns the number of
 // kernels launched.
+template <int MODE, bool RIDE>
+void launch_2d(long long blocks, bool small, cudaStream_t st, const StepArgs& a) {
+  launch_chain("stencil launch",
+               small ? k_ac2d_step<MODE, 4, 1, false, 3, RIDE>
+                     : k_ac2d_step<MODE, 4, 1, true, Ac2dBounds<MODE, 4>::MINB, RIDE>,
+               dim3((unsigned)blocks), dim3(128), st, a);
+}
 template <int MODE>
-int launch_2d_xsplit(long long blocks, bool small, cudaStream_t st, const StepArgs& a) {
-  if (small) {
-    launch_chain("stencil launch", k_ac2d_step<MODE, 4, 1, false, 3>, dim3((unsigned)blocks), dim3(128), st, a);
-    return 1;
+int launch_2d_xsplit(long long blocks, bool small, cudaStream_t st, StepArgs a, int rec_blocks) {
+  if (!small) blocks += xstrip_blocks(a);
+  if constexpr (MODE == MODE_FWD || MODE == MODE_FWD_D) {
+    if (a.ride.shots) {
+      a.ride.rec_block = blocks;
+      if (a.ride.rec_it > 0) blocks += (long long)rec_blocks * a.ride.rec_shots;
+      launch_2d<MODE, true>(blocks, small, st, a);
+      return 1;
+    }
   }
-  launch_chain("stencil launch", k_ac2d_step<MODE, 4, 1, true>, dim3((unsigned)(blocks + xstrip_blocks(a))), dim3(128), st,
-               a);
+  launch_2d<MODE, false>(blocks, small, st, a);
   return 1;
 }
 
@@ -1447,7 +1508,7 @@ struct Launcher {
         enable_cpa_carveout<MODE>();
         k_ac2d_cpa<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       } else if (nw == 4 && ws->xsplit)
-        nk = launch_2d_xsplit<MODE>(blocks, small_2d(ws, a.nshots), st, a);
+        nk = launch_2d_xsplit<MODE>(blocks, small_2d(ws, a.nshots), st, a, ws->ride_rec);
       else if (nw == 4)
         k_ac2d_step<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       else if (nw == 8)
@@ -1473,7 +1534,7 @@ struct Launcher {
       }
       if (launched) {
       } else if (nw == 4 && ws->xsplit)
-        nk = launch_2d_xsplit<MODE>(blocks, small_2d(ws, a.nshots), st, a);
+        nk = launch_2d_xsplit<MODE>(blocks, small_2d(ws, a.nshots), st, a, ws->ride_rec);
       else if (nw == 4)
         k_ac2d_step<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       else if (nw == 8)
@@ -1582,6 +1643,15 @@ StepArgs base_args(sw_wavesim* ws, const StepCtx& c, int S) {
   a.dbf16 = (ws->gradient && ws->gp.snapshot_bf16 >= 1) ? (ws->gp.snapshot_bf16 == 3 ? 2 : 1) : 0;
   a.ntx = (int)((ws->P + 127) / 128);
   return a;
+}
+
+StepRide ride_args(const sw_wavesim* ws, int it) {
+  StepRide r{};
+  r.shots = ws->d_ride.as<StepShot>();
+  r.ids = ws->d_ids.as<int>();
+  r.rec_lin = ws->d_rec.as<long long>();
+  r.it = it;
+  return r;
 }
 
 // D slot `k` of every shot (the slots of a shot are contiguous; FP32 or BF16 elements).
@@ -1777,6 +1847,8 @@ void forward_group(sw_wavesim* ws, const std::vector<HostShot>& group, bool grad
   };
   auto dslot_of = [&](int it) -> long long { return K == 1 ? it - 1 : (it - 1) % K; };
   const bool snap = !grad && ws->snapevery > 0;
+  int rec_it = 0, rec_shots = 0;  // the step that the next launch records
+  FieldArg rec_p{nullptr, 0};
   for (int it = 1; it <= max_nt;) {
     const int Sa = active_count(group, it);
     const int d_first = grad ? d_first_of(it, Sa) : Sa;
@@ -1827,14 +1899,23 @@ void forward_group(sw_wavesim* ws, const std::vector<HostShot>& group, bool grad
     } else {
       double bytes = stencil_bytes(ws, Sa, grad ? MODE_FWD_D : MODE_FWD, n_dwrite, ckpt);
       if (ws->precision == 1) bytes += hp_extra_bytes(ws, Sa);
+      if (ws->ride_ok) {
+        a.ride = ride_args(ws, it);
+        a.ride.rec_it = rec_it;
+        a.ride.rec_shots = rec_shots;
+        rec_it = it;
+        rec_shots = Sa;
+        rec_p = a.pnew;
+      }
       // steps before the top segment write no D: the plain forward kernel does the same work
       // without the D store path
       if (grad && n_dwrite > 0)
         L.step<MODE_FWD_D>(a, c, bytes);
       else
         L.step<MODE_FWD>(a, c, bytes);
-      launch_inject(ws, Sa, a.pnew, a.dout, grad ? a.Dout : FieldArg{nullptr, 0}, d_first, it, 1, 0, a.plo_new,
-                    a.dlo);
+      if (!ws->ride_ok)
+        launch_inject(ws, Sa, a.pnew, a.dout, grad ? a.Dout : FieldArg{nullptr, 0}, d_first, it, 1, 0, a.plo_new,
+                      a.dlo);
     }
     if (ck_slot >= 0) pack_checkpoint(ws, Sa, ck_slot);
     const int it_end = two ? it + 1 : it;
@@ -1850,6 +1931,13 @@ void forward_group(sw_wavesim* ws, const std::vector<HostShot>& group, bool grad
       }
     }
     it = it_end + 1;
+  }
+  if (rec_it > 0) {
+    cudaEvent_t ev = nullptr;
+    ws->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
+    launch_chain("record launch", k_ride_record, dim3((unsigned)ws->ride_rec, (unsigned)rec_shots), dim3(128), st,
+                 ws->d_ride.as<StepShot>(), ws->d_rec.as<long long>(), rec_p, rec_it);
+    ws->ctx->prof.end(st, KK_SRCREC, ev);
   }
 }
 
@@ -1918,8 +2006,9 @@ void adjoint_group(sw_wavesim* ws, const std::vector<HostShot>& group) {
           launch_inject(ws, Sa, a.pnew, a.dout, b.Dout2, 0, t + 1, 0);
           t += 2;
         } else {
+          if (ws->ride_ok) a.ride = ride_args(ws, t);
           L.step<MODE_FWD_D>(a, c, stencil_bytes(ws, Sa, MODE_FWD_D, Sa, false), true);
-          launch_inject(ws, Sa, a.pnew, a.dout, a.Dout, 0, t, 0);
+          if (!ws->ride_ok) launch_inject(ws, Sa, a.pnew, a.dout, a.Dout, 0, t, 0);
           t += 1;
         }
       }

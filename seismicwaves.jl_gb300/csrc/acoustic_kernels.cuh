@@ -61,6 +61,28 @@ struct Field64 {  // FP64 per-shot array: shot k at p + k * s
   long long s;
 };
 
+// What the 2D forward step itself takes over from k_inject_record: the
+// sources of the step, added by the threads that advance their points, and the
+// recording of the step before, by blocks at the end of the launch (pcur is
+// read-only in a step).
+constexpr int STEP_MAXSP = 4;  // unique source points per shot
+struct alignas(16) StepShot {
+  int sx[STEP_MAXSP], sz[STEP_MAXSP];  // unique source points (0-based; -4 past the last)
+  int k0[STEP_MAXSP], k1[STEP_MAXSP];  // their source ids: ids[k0 .. k1)
+  const float* tf;                     // (nt, nsrc) scaled source time functions
+  float* tr;                           // (nt, nrec) traces
+  int nt, nrec;
+  long long rec_off;
+};
+struct StepRide {
+  const StepShot* shots;     // nullptr: sources and recording are left to k_inject_record
+  const int* ids;
+  const long long* rec_lin;
+  int it;                    // this step (sources)
+  int rec_it, rec_shots;     // the step to record (0: none) and the shots active in it
+  long long rec_block;       // first recording block
+};
+
 struct StepArgs {
   int n0, n1, n2;  // grid points per axis (n2 = 1 in 2D; the depth axis is n1 in 2D, n2 in 3D)
   int P;           // pitch of axis 0 in floats
@@ -95,6 +117,7 @@ struct StepArgs {
   const double* cpml64;
   Field64 psi64_in[3], psi64_out[3], xi64[3];
   double ihd[3];
+  StepRide ride;
 };
 
 struct StripIO {
@@ -575,12 +598,43 @@ __host__ __device__ __forceinline__ void xstrip_groups(int nx, int H, int P, int
   ng = nl + (P - xr > 0 ? (P - xr) / 4 : 0);
 }
 
+// Bit u: source point u of the shot lies in rows [z0, z1) at x0 .. x0 + 3.
+__device__ __forceinline__ unsigned ride_hits(const StepRide& R, int shot, int x0, int z0, int z1) {
+  const int4 X = __ldg(reinterpret_cast<const int4*>(R.shots[shot].sx));
+  const int4 Z = __ldg(reinterpret_cast<const int4*>(R.shots[shot].sz));
+  auto hit = [&](int x, int z) { return (unsigned)(x - x0) < 4u && z >= z0 && z < z1; };
+  return (hit(X.x, Z.x) ? 1u : 0u) | (hit(X.y, Z.y) ? 2u : 0u) | (hit(X.z, Z.z) ? 4u : 0u) | (hit(X.w, Z.w) ? 8u : 0u);
+}
+// The sources of this step at the points of `hits`, by the thread that has
+// just stored them; the sums of k_inject_record, in the same order.
+static __device__ __noinline__ void ride_inject(const StepRide& R, int shot, unsigned hits, int P, float* pn, float* dn,
+                                         float* Dw, int dbf16) {
+  const StepShot& Q = R.shots[shot];
+  for (int u = 0; u < STEP_MAXSP; ++u) {
+    if (!(hits >> u & 1)) continue;
+    const long long lin = (long long)Q.sz[u] * P + Q.sx[u];
+    float acc = pn[lin], add = 0.f;
+    for (int k = Q.k0[u]; k < Q.k1[u]; ++k) {
+      const float v = Q.tf[(long long)(R.it - 1) + (long long)R.ids[k] * Q.nt];
+      acc += v;
+      add += v;
+    }
+    pn[lin] = acc;
+    dn[lin] += add;
+    if (Dw) dst1(Dw, lin, dld1(Dw, lin, dbf16) + add, dbf16);
+  }
+}
+// Receiver q of a shot at step it.
+__device__ __forceinline__ void ride_record(const StepShot& Q, int it, const long long* rec_lin, const float* p, int q) {
+  if (q < Q.nrec) Q.tr[(long long)(it - 1) + (long long)q * Q.nt] = p[rec_lin[Q.rec_off + q]];
+}
+
 // The points that the main blocks of k_ac2d_step<.., XS = true> leave: work
 // item t is one (lane group of the x strips, row, shot); it loads its rows
 // and runs the general path of Ac2dRow (both strips per point), so every
 // point is advanced by the same arithmetic as in the single-path kernel.
 // Not inlined: its registers (and spills) stay out of the main blocks' path.
-template <int MODE>
+template <int MODE, bool RIDE>
 __device__ __noinline__ void xstrip_item(const StepArgs& A, long long t) {
   const int nx = A.n0, nz = A.n1, P = A.P, H = A.halo;
   int nl, xr, ng;
@@ -612,6 +666,10 @@ __device__ __noinline__ void xstrip_item(const StepArgs& A, long long t) {
     if (MODE == MODE_ADJ) ld4rw(c4, R.gcp + row + x0);
   }
   R.update(z, rm, r0, rp, o, f, dv, g4, c4, left, right);
+  if constexpr (RIDE) {
+    const unsigned hits = ride_hits(A.ride, shot, x0, z, z + 1);
+    if (hits) ride_inject(A.ride, shot, hits, P, R.pn, R.dn, R.Dw, R.dbf16);
+  }
 }
 
 // Minimum resident blocks per SM for a block of NW warps: keeps the forward
@@ -629,16 +687,26 @@ struct Ac2dBounds {
 // XS: the lanes that meet an x strip store nothing in the main blocks (the
 // first nshots x tiles_x x tiles_z); the blocks after them take the lane
 // groups of the x strips, one per thread (xstrip_item), so that this work
-// fills the tail of the launch.  MB: resident blocks per SM.
-template <int MODE, int NW, int DP = 1, bool XS = false, int MB = Ac2dBounds<MODE, NW>::MINB - (DP - 1)>
+// fills the tail of the launch.  MB: resident blocks per SM.  RIDE: the step
+// adds its sources and the blocks from A.ride.rec_block on record the step
+// before.
+template <int MODE, int NW, int DP = 1, bool XS = false, int MB = Ac2dBounds<MODE, NW>::MINB - (DP - 1),
+          bool RIDE = false>
 __global__ void __launch_bounds__(32 * NW, MB) k_ac2d_step(const StepArgs A) {
   constexpr unsigned FULL = 0xffffffffu;
   chain_next();
   const unsigned tid = chain_wait_tid();
+  if constexpr (RIDE) {
+    if (A.ride.rec_it > 0 && (long long)blockIdx.x >= A.ride.rec_block) {
+      const int b = (int)(blockIdx.x - A.ride.rec_block), s = b % A.ride.rec_shots;
+      ride_record(A.ride.shots[s], A.ride.rec_it, A.ride.rec_lin, fptr(A.pcur, s), b / A.ride.rec_shots * 128 + (int)tid);
+      return;
+    }
+  }
   if constexpr (XS) {
     const long long nb_main = (long long)A.nshots * A.tiles_x * A.tiles_y * A.tiles_z;
     if ((long long)blockIdx.x >= nb_main) {
-      xstrip_item<MODE>(A, ((long long)blockIdx.x - nb_main) * (32 * NW) + tid);
+      xstrip_item<MODE, RIDE>(A, ((long long)blockIdx.x - nb_main) * (32 * NW) + tid);
       return;
     }
   }
@@ -694,6 +762,10 @@ __global__ void __launch_bounds__(32 * NW, MB) k_ac2d_step(const StepArgs A) {
       if (MODE == MODE_ADJ) ld4rw(c4, gcp + row + xa);
     }
   }
+  // source points among this thread's; XS has no register to keep them in and looks after its rows
+  unsigned hits = 0;
+  if constexpr (RIDE)
+    if (!XS && inb) hits = ride_hits(A.ride, shot, x0, z_begin, z_end);
   // DP == 2 (forward kernels): a second row of loads in flight, issued one
   // iteration earlier (q* hold p of row z+2 and d, fact of row z+1).
   float qp[4], qo[4], qf[4];
@@ -772,6 +844,10 @@ __global__ void __launch_bounds__(32 * NW, MB) k_ac2d_step(const StepArgs A) {
       }
     }
   }
+  if constexpr (RIDE && XS)
+    if (inb && !R.xstrip) hits = ride_hits(A.ride, shot, x0, z_begin, z_end);
+  if constexpr (RIDE)
+    if (hits) ride_inject(A.ride, shot, hits, P, R.pn, R.dn, R.Dw, R.dbf16);
 }
 
 

@@ -73,6 +73,30 @@ struct Geo {
   __host__ __device__ __forceinline__ int xcol(int i) const { return i - 1 < WL ? i - 1 : WL + (i - 1 - xr); }
 };
 
+constexpr int STEP_MAXSP = 4;  // unique source points that the pressure update itself adds (step_sources)
+struct alignas(16) ShotDesc {
+  int sx[STEP_MAXSP], sz[STEP_MAXSP];  // column and row of the first unique source points (0: none)
+  int nt, nsrc, nrec;
+  int nsp, nrp;                 // unique source / receiver points
+  const long long* sp_lin;      // unique source points (padded index)
+  const int* sp_ptr;            // nsp + 1
+  const int* sp_ids;            // source index of each entry
+  const long long* rp_lin;
+  const int* rp_ptr;
+  const int* rp_ids;
+  const long long* rec_lin;     // per receiver
+  const float* tf;              // (nt, nsrc)
+  float* tr;                    // (nt, nrec)
+  const float* obs;
+  const float* ic;              // diagonal inverse covariance (nt) or null
+  const float* mask;            // window mask (nt) or null
+  float* adj;                   // prescaled adjoint sources (nt, nrec)
+  const float* icd;             // dense inverse covariance (nt, nt) or null
+  float* resid;                 // dense case: masked residuals
+  const float* cres;            // dense case: C^-1 r
+  int mkind;                    // 0 L2, 1 CCTS (k_ccts writes this shot's adjoint source)
+};
+
 struct PArgs {
   Geo g;
   const float* vx; const float* vz;  // [shot][F]
@@ -87,6 +111,8 @@ struct PArgs {
   const float* pc; const float* po;  // p[it], p[it-1], [shot][F]
   float* acc;                        // [shot][3][F]: m0 term, m1 x term, m1 z term
   float idt;
+  const ShotDesc* src;               // forward: the sources of step it are added here (null: by k_vd_srcrec)
+  int it;
 };
 
 struct VArgs {
@@ -99,6 +125,9 @@ struct VArgs {
   const float* cp; int cps;
   const float* cx4;
   int tz;
+  // recording of step rec_it (0: none) by the blocks from blockIdx.y = bands on
+  const ShotDesc* desc;
+  int rec_it, nshots, bands;
 };
 
 // (c1 f1 - c2 f2 + c2 f3 - c1 f4) / h.  Every rounding of the stencils is
@@ -215,6 +244,25 @@ __device__ __forceinline__ unsigned xmask_vel(const Geo& g, int i0) {
 __device__ __forceinline__ void prefetch_band(const float* p, int P, int rows, int cols, int lane) {
   const int r = lane >> 2, x = (lane & 3) * 32;
   if (r < rows && x < cols) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + r * P + x));
+}
+
+// The sources of step it (k_vd_srcrec's sums, in its order) at a thread's four
+// points of rows j0 .. j1, which it has just stored.  With the recording on the
+// velocity launch, which reads the pressure only, a step is two launches
+// instead of three (one shot of 402 x 301: 5.26 us per step against 5.53; one
+// of 801 x 801, 400-step gradient: 12.3 ms against 13.3; 8 of 2001 x 801: 77.7
+// against 78.4).  Shots with more source points leave both to k_vd_srcrec.
+__device__ __forceinline__ void step_sources(const ShotDesc& D, int it, int i0, int j0, int j1, float* p, const Geo& g) {
+  const int4 X = __ldg(reinterpret_cast<const int4*>(D.sx)), Z = __ldg(reinterpret_cast<const int4*>(D.sz));
+  const int x[STEP_MAXSP] = {X.x, X.y, X.z, X.w}, z[STEP_MAXSP] = {Z.x, Z.y, Z.z, Z.w};
+#pragma unroll
+  for (int u = 0; u < STEP_MAXSP; ++u) {
+    if ((unsigned)(x[u] - i0) >= 4u || z[u] < j0 || z[u] > j1) continue;
+    float* q = p + g.lin(x[u], z[u]);
+    float v = *q;
+    for (int k = D.sp_ptr[u]; k < D.sp_ptr[u + 1]; ++k) v += D.tf[(long long)(it - 1) + (long long)D.sp_ids[k] * D.nt];
+    *q = v;
+  }
 }
 
 // Pressure update (update_p_CPML! on 2:nx-1, 2:nz-1; every other node copies
@@ -380,6 +428,7 @@ __global__ void __launch_bounds__(BX, VdPBounds<CORR>::MINB) k_vd_p(const PArgs 
     }
     z0 = z1; z1 = z2; z2 = z3; z3 = zn;
   }
+  if (!CORR && A.src && ldok) step_sources(A.src[s], A.it, i0, j0, j1, pout, g);
 }
 
 // Velocity update (update_vx_CPML! on 1:nx-1 x 1:nz, update_vy_CPML! on
@@ -389,6 +438,13 @@ __global__ void __launch_bounds__(BX, 6) k_vd_v(const VArgs A) {
   chain_next();
   const unsigned tid = chain_wait_tid();
   const Geo g = A.g;
+  if ((int)blockIdx.y >= A.bands) {
+    const long long b = (long long)(blockIdx.y - A.bands) * gridDim.x + blockIdx.x;
+    const int rs = (int)(b % A.nshots), r = (int)(b / A.nshots) * BX + (int)tid;
+    const ShotDesc& D = A.desc[rs];
+    if (r < D.nrec) D.tr[(long long)(A.rec_it - 1) + (long long)r * D.nt] = A.p[(long long)rs * g.F + D.rec_lin[r]];
+    return;
+  }
   const int tx = (g.nx + 511) / 512;
   const int s = blockIdx.x / tx;
   const int lane = tid & 31, warp = tid >> 5;
@@ -719,28 +775,6 @@ __global__ void k_vd_d2f(const double* __restrict__ src, float* __restrict__ dst
 // ---------------------------------------------------------------------------
 // Sources, receivers, misfit, reductions
 // ---------------------------------------------------------------------------
-struct ShotDesc {
-  int nt, nsrc, nrec;
-  int nsp, nrp;                 // unique source / receiver points
-  const long long* sp_lin;      // unique source points (padded index)
-  const int* sp_ptr;            // nsp + 1
-  const int* sp_ids;            // source index of each entry
-  const long long* rp_lin;
-  const int* rp_ptr;
-  const int* rp_ids;
-  const long long* rec_lin;     // per receiver
-  const float* tf;              // (nt, nsrc)
-  float* tr;                    // (nt, nrec)
-  const float* obs;
-  const float* ic;              // diagonal inverse covariance (nt) or null
-  const float* mask;            // window mask (nt) or null
-  float* adj;                   // prescaled adjoint sources (nt, nrec)
-  const float* icd;             // dense inverse covariance (nt, nt) or null
-  float* resid;                 // dense case: masked residuals
-  const float* cres;            // dense case: C^-1 r
-  int mkind;                    // 0 L2, 1 CCTS (k_ccts writes this shot's adjoint source)
-};
-
 // inject_sources! then record_receivers! (the velocity update in between does
 // not touch p): one block per active shot; a point that several sources share
 // receives them in source order.
@@ -1023,6 +1057,8 @@ struct sw_acoustic_vd {
   int snapevery = 0;
   float* const* snap_out = nullptr;
   int tz = 0;  // rows per block (0: band_rows)
+  bool step_src = false;  // the group's steps add their sources and record (at most STEP_MAXSP source points a shot)
+  int gx_rec = 1;         // BX-receiver blocks of the largest shot
   // compensated forward (precision 1): low parts of p, vx, vz and of the
   // material factors, FP64 memory variables and coefficients
   int precision = 0;
@@ -1200,6 +1236,8 @@ void build_tables(sw_acoustic_vd* vd, const sw_acoustic_shot* shots, const std::
   cudaStream_t st = vd->ctx->stream;
   const int S = (int)group.size();
   Pools P;
+  vd->step_src = true;
+  vd->gx_rec = 1;
   struct Off {
     size_t sp_lin, sp_ptr, sp_ids, rp_lin, rp_ptr, rp_ids, rec_lin, mask;
     int nsp, nrp;
@@ -1323,6 +1361,13 @@ void build_tables(sw_acoustic_vd* vd, const sw_acoustic_shot* shots, const std::
     D.nsp = o.nsp;
     D.nrp = o.nrp;
     D.sp_lin = LL + o.sp_lin;
+    for (int u = 0; u < std::min(D.nsp, STEP_MAXSP); ++u) {
+      const long long lin = P.ll[o.sp_lin + u];
+      D.sx[u] = (int)(lin % vd->g.P) - XPAD + 1;
+      D.sz[u] = (int)(lin / vd->g.P) - ZPAD + 1;
+    }
+    vd->step_src = vd->step_src && D.nsp <= STEP_MAXSP;
+    vd->gx_rec = std::max(vd->gx_rec, (D.nrec + BX - 1) / BX);
     D.sp_ptr = IN + o.sp_ptr;
     D.sp_ids = IN + o.sp_ids;
     D.rp_lin = LL + o.rp_lin;
@@ -1483,7 +1528,10 @@ struct Run {
   }
   void launch_v(VArgs a, int S) const {
     a.tz = band_rows(vd, S);
-    launch_chain("velocity update launch", k_vd_v, grid(S, a.tz), dim3(BX), st, a);
+    dim3 gr = grid(S, a.tz);
+    a.bands = (int)gr.y;
+    if (a.rec_it > 0) gr.y += ((unsigned)vd->gx_rec * S + gr.x - 1) / gr.x;
+    launch_chain("velocity update launch", k_vd_v, gr, dim3(BX), st, a);
   }
   // algorithmic bytes per node and shot: pressure R vx vz p, W p (16); velocity
   // R p vx vz, W vx vz (20); shared by the shots: fact_m0, fact_m1 x2 (12)
@@ -1550,14 +1598,27 @@ struct Run {
     }
     cudaEvent_t ev = nullptr;
     vd->ctx->prof.begin(st, kind, fwd_bytes(S), &ev);
-    launch_p(pargs(false, pin, pout), S, false);
+    PArgs a = pargs(false, pin, pout);
+    VArgs b = vargs(false, pout);
+    if (vd->step_src) {
+      a.src = ddesc;
+      a.it = it;
+      b.desc = ddesc;
+      b.rec_it = record ? it : 0;
+      b.nshots = S;
+      launch_p(a, S, false);
+      launch_v(b, S);
+      vd->ctx->prof.end(st, kind, ev, 2);
+      return;
+    }
+    launch_p(a, S, false);
     vd->ctx->prof.end(st, kind, ev);
     vd->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
     launch_chain("injection launch", k_vd_srcrec, dim3(S), dim3(128), st, ddesc, it, vd->g.F, pout, record ? 1 : 0,
                  nullptr);
     vd->ctx->prof.end(st, KK_SRCREC, ev);
     vd->ctx->prof.begin(st, kind, 0.0, &ev);
-    launch_v(vargs(false, pout), S);
+    launch_v(b, S);
     vd->ctx->prof.end(st, kind, ev);
   }
   // adjoint_onestep_CPML! + correlations: velocities, p with the fused
@@ -1759,7 +1820,7 @@ void vd_forward(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, b
     if (vd->snapevery > 0) {  // host copies inside the loop: no graph
       body();
     } else {
-      std::vector<long long> key = {0, S, vd->tz, vd->precision};
+      std::vector<long long> key = {0, S, vd->tz, vd->precision, vd->step_src ? vd->gx_rec : 0};
       for (const auto& h : group) key.push_back(h.nt);
       vd->cache.run(vd->ctx, key, body);
     }
@@ -2014,7 +2075,7 @@ void vd_gradient(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, 
         vd->ctx->prof.end(st, KK_OTHER, ev);
       }
     };
-    std::vector<long long> key = {1, S, ntmax, vd->tz, vd->precision, first_group ? 1 : 0, mute ? 1 : 0, crec,
+    std::vector<long long> key = {1, S, ntmax, vd->tz, vd->precision, vd->step_src ? vd->gx_rec : 0, first_group ? 1 : 0, mute ? 1 : 0, crec,
                                   (long long)smem, (long long)(uintptr_t)out[0], (long long)(uintptr_t)out[1],
                                   (long long)(uintptr_t)mout};
     for (const auto& h : group) key.push_back(h.nt);
