@@ -237,10 +237,17 @@ int run(const sw_acoustic_params* p, const float* vp, const sw_acoustic_shot* s,
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tiles_x = (P + 511) / 512;
-  // the batched path's rule for the register-pipelined stencil: 8-row bands,
-  // 4-row bands when 8-row ones would leave the GPU under-filled
-  const int TZ = (long long)tiles_x * ((nz - 2 + 7) / 8) < 4LL * sms ? 4 : 8;
+  // the batched path's rules (small_2d, make_step_ctx): single rows without
+  // x-strip blocks below 16 rows per SM, else the x strips split off and 2- or
+  // 4-row bands; the grids that fit the scratch never fill 8-row ones
+  const long long wx = (P + 127) / 128;
+  const bool small = wx * (nz - 2) < 16LL * sms;
+  const int TZ = small ? 1 : wx * ((nz - 2 + 3) / 4) < 8LL * sms ? 2 : 4;
   const int tiles_z = (nz - 2 + TZ - 1) / TZ;
+  int nl, xr, ng;
+  xstrip_groups(nx, H, P, nl, xr, ng);
+  const unsigned blocks = (unsigned)(tiles_x * tiles_z);
+  const unsigned xblocks = (unsigned)(((long long)ng * (nz - 2) + 127) / 128);
 
   StepArgs a;
   std::memset(&a, 0, sizeof(a));
@@ -275,7 +282,10 @@ int run(const sw_acoustic_params* p, const float* vp, const sw_acoustic_shot* s,
       a.xi_in[d] = FieldArg{xi[d], 0};
       a.xi_out[d] = a.xi_in[d];
     }
-    k_ac2d_step<MODE_FWD, 4><<<(unsigned)(tiles_x * tiles_z), 128, 0, st>>>(a);
+    if (small)
+      k_ac2d_step<MODE_FWD, 4, 1, false, 3><<<blocks, 128, 0, st>>>(a);
+    else
+      k_ac2d_step<MODE_FWD, 4, 1, true><<<blocks + xblocks, 128, 0, st>>>(a);
     k_noalloc_inject_record<<<1, 128, 0, st>>>(T, pb[1 - pc], db, it);
     pc = 1 - pc;
     pk = 1 - pk;
