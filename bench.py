@@ -536,12 +536,12 @@ def measure_vd(a, name="acoustic_vd2d_2001x801", shots=0, nt_cap=0, steps=None, 
     warmup = a.warmup if warmup is None else warmup
     sw, w = _workload(name, shots, nt_cap)
     R = VDRun(sw, w, device, precision=a.precision)
-    tuned, tz = None, a.tz or 8
+    tuned, tz = None, a.tz
     if a.tz:
         R.ctx.check(R.lib.sw_acoustic_vd_set_tuning(R.h, a.tz), "sw_acoustic_vd_set_tuning")
     R.make_observed()
     if not (a.tz or a.no_autotune):
-        tz, tuned = _tune_tz(R, w, "vd", (8, 16, 32))
+        tz, tuned = _tune_tz(R, w, "vd", (0, 8, 16, 32))
     nshots = len(w.shots)
     allidx = list(range(nshots))
     pts = float(w.point_steps())
@@ -1076,12 +1076,12 @@ def measure_elastic(a, name="elastic2d_1200x600", shots=0, nt_cap=0, steps=None,
     warmup = a.warmup if warmup is None else warmup
     sw, w = _workload(name, shots, nt_cap)
     R = ElasticRun(sw, w, device)
-    tuned, tz = None, a.tz or 8
+    tuned, tz = None, a.tz
     if a.tz:
         R.ctx.check(R.lib.sw_elastic_set_tuning(R.h, a.tz), "sw_elastic_set_tuning")
     R.make_observed()
     if not (a.tz or a.no_autotune):
-        tz, tuned = _tune_tz(R, w, "elastic", (8, 16, 32, 72, 136))
+        tz, tuned = _tune_tz(R, w, "elastic", (0, 8, 16, 32, 72, 136))
     nshots = len(w.shots)
     allidx = list(range(nshots))
     pts = float(w.point_steps())

@@ -142,7 +142,7 @@ def autotune(ctx: _lib.Context, ws_handle, grid_key, shots_structs, nshots: int,
     return r
 
 
-def autotune_tz(key, set_tuning, trial, candidates=(8, 16, 32)):
+def autotune_tz(key, set_tuning, trial, candidates=(0, 8, 16, 32)):
     """Band height of a variable-density or elastic simulation: `set_tuning(tz)`
     installs a candidate, `trial()` runs one short batched call; the fastest
     of two timed trials per candidate is kept.  Returns (tz, timings)."""
