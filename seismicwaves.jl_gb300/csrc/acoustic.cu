@@ -959,14 +959,8 @@ void build_tables(sw_wavesim* ws, const sw_acoustic_shot* shots, const std::vect
   // unique source points per shot, none on the outermost grid lines.  One link
   // less in the chain of a step (one shot of 201 x 201: 4.06 us per step
   // against 5.1; 4 of 801 x 801, gradient: 29.8 against 32.1 ms; 16 of 2001 x
-  // 801: 104.6 against 106.6).  Not between 16 and 64 rows of 128 points per
-  // SM, where the launch is one wave that the look for sources at the end of
-  // every warp lengthens (601 x 601: 16.0 against 15.4; 801 x 801: 30.8
-  // against 30.6).
-  const long long rows = (long long)S * ((ws->P + 127) / 128) * (ws->n[1] - 2);
-  const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
-  ws->ride_ok = ws->N == 2 && ws->precision == 0 && !T.pair_ok && ws->xsplit && !ws->cpa && (ws->variant & 7) == 0 &&
-                (rows < 16LL * sms || rows >= 64LL * sms);
+  // 801: 104.6 against 106.6; one of 801 x 801, 400 steps: 8.1 against 9.5).
+  ws->ride_ok = ws->N == 2 && ws->precision == 0 && !T.pair_ok && ws->xsplit && !ws->cpa && (ws->variant & 7) == 0;
   ws->ride_rec = 1;
   T.ride.assign(S, StepShot{});
   for (int k = 0; k < S && ws->ride_ok; ++k) {
@@ -1202,6 +1196,17 @@ bool small_2d(const sw_wavesim* ws, int S) {
   return ws->N == 2 && (long long)S * ((ws->P + 127) / 128) * (ws->n[1] - 2) < 16LL * sms;
 }
 
+// Launches with fewer than 400 rows per SM: 4 resident blocks per SM, whose 128
+// registers spill nothing, in place of 8 (forward) or 6 (adjoint).  They do not
+// fill more warps than that for long, and every row is faster (gradient of one
+// shot of 801 x 801, 400 steps, 37 rows per SM: 8.1 ms against 11.2, of 601 x
+// 601: 7.7 against 10.7, of 8 of 801 x 801, 200 steps, 294 rows: 18.1 against
+// 19.4; 16 of 2001 x 801, 1346 rows: 43.7 against 39.7).
+bool mid_2d(const sw_wavesim* ws, int S) {
+  const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
+  return ws->N == 2 && (long long)S * ((ws->P + 127) / 128) * (ws->n[1] - 2) < 400LL * sms;
+}
+
 StepCtx make_step_ctx(sw_wavesim* ws, int S, int kind = TZ_FORWARD) {
   StepCtx c{ws, 0, 0, 1, 0};
   const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
@@ -1222,12 +1227,11 @@ StepCtx make_step_ctx(sw_wavesim* ws, int S, int kind = TZ_FORWARD) {
       // 64 shots of 2001 x 801: 55.6 Gpts/s against 48.4 at 64 rows).  A
       // warp's rows run one after the other, so smaller launches take
       // shorter bands: 4 rows below 256 warps per SM (16 shots of 2001 x 801,
-      // gradient: 109.8 against 111.1 ms; one of 801 x 801: 35.2 against 43.6
-      // with 8 and 37.2 with 2), 2 below 8, single rows for small_2d
+      // gradient: 109.8 against 111.1 ms; one of 801 x 801, 400 steps: 9.5
+      // against 10.5 with 2 rows and 10.3 with 3), single rows for small_2d
       const long long wx = (ws->P + 127) / 128;
       TZ = 8;
       if (S * wx * ((nint + 7) / 8) < 256LL * sms) TZ = 4;
-      if (S * wx * ((nint + 3) / 4) < 8LL * sms) TZ = 2;
       if (small_2d(ws, S)) TZ = 1;
     } else if (ws->N == 3 && ws->split3d) {
       // 16 planes, 8 or 4 while the inner rows make fewer than 8 blocks per SM
@@ -1419,25 +1423,28 @@ long long xstrip_blocks(const StepArgs& a) {
 // headline).  A small launch (small_2d) takes the one-kernel form with
 // registers for every load of a row to be in flight.  Returns the number of
 // kernels launched.
+enum Size2d { ROWS_2D, FEW_2D, FULL_2D };  // small_2d, mid_2d, larger
 template <int MODE, bool RIDE>
-void launch_2d(long long blocks, bool small, cudaStream_t st, const StepArgs& a) {
+void launch_2d(long long blocks, Size2d size, cudaStream_t st, const StepArgs& a) {
   launch_chain("stencil launch",
-               small ? k_ac2d_step<MODE, 4, 1, false, 3, RIDE>
-                     : k_ac2d_step<MODE, 4, 1, true, Ac2dBounds<MODE, 4>::MINB, RIDE>,
+               size == ROWS_2D  ? k_ac2d_step<MODE, 4, 1, false, 3, RIDE>
+               : size == FEW_2D ? k_ac2d_step<MODE, 4, 1, true, 4, RIDE>
+                                : k_ac2d_step<MODE, 4, 1, true, Ac2dBounds<MODE, 4>::MINB, RIDE>,
                dim3((unsigned)blocks), dim3(128), st, a);
 }
+Size2d size_2d(const sw_wavesim* ws, int S) { return small_2d(ws, S) ? ROWS_2D : mid_2d(ws, S) ? FEW_2D : FULL_2D; }
 template <int MODE>
-int launch_2d_xsplit(long long blocks, bool small, cudaStream_t st, StepArgs a, int rec_blocks) {
-  if (!small) blocks += xstrip_blocks(a);
+int launch_2d_xsplit(long long blocks, Size2d size, cudaStream_t st, StepArgs a, int rec_blocks) {
+  if (size != ROWS_2D) blocks += xstrip_blocks(a);
   if constexpr (MODE == MODE_FWD || MODE == MODE_FWD_D) {
     if (a.ride.shots) {
       a.ride.rec_block = blocks;
       if (a.ride.rec_it > 0) blocks += (long long)rec_blocks * a.ride.rec_shots;
-      launch_2d<MODE, true>(blocks, small, st, a);
+      launch_2d<MODE, true>(blocks, size, st, a);
       return 1;
     }
   }
-  launch_2d<MODE, false>(blocks, small, st, a);
+  launch_2d<MODE, false>(blocks, size, st, a);
   return 1;
 }
 
@@ -1510,7 +1517,7 @@ struct Launcher {
         enable_cpa_carveout<MODE>();
         k_ac2d_cpa<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       } else if (nw == 4 && ws->xsplit)
-        nk = launch_2d_xsplit<MODE>(blocks, small_2d(ws, a.nshots), st, a, ws->ride_rec);
+        nk = launch_2d_xsplit<MODE>(blocks, size_2d(ws, a.nshots), st, a, ws->ride_rec);
       else if (nw == 4)
         k_ac2d_step<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       else if (nw == 8)
@@ -1536,7 +1543,7 @@ struct Launcher {
       }
       if (launched) {
       } else if (nw == 4 && ws->xsplit)
-        nk = launch_2d_xsplit<MODE>(blocks, small_2d(ws, a.nshots), st, a, ws->ride_rec);
+        nk = launch_2d_xsplit<MODE>(blocks, size_2d(ws, a.nshots), st, a, ws->ride_rec);
       else if (nw == 4)
         k_ac2d_step<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       else if (nw == 8)

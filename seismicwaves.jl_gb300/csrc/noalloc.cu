@@ -237,12 +237,11 @@ int run(const sw_acoustic_params* p, const float* vp, const sw_acoustic_shot* s,
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tiles_x = (P + 511) / 512;
-  // the batched path's rules (small_2d, make_step_ctx): single rows without
-  // x-strip blocks below 16 rows per SM, else the x strips split off and 2- or
-  // 4-row bands; the grids that fit the scratch never fill 8-row ones
-  const long long wx = (P + 127) / 128;
-  const bool small = wx * (nz - 2) < 16LL * sms;
-  const int TZ = small ? 1 : wx * ((nz - 2 + 3) / 4) < 8LL * sms ? 2 : 4;
+  // the batched path's rules (small_2d, mid_2d): single rows without x-strip
+  // blocks below 16 rows per SM, else 4-row bands with the x strips split off;
+  // the grids that fit the scratch stay below 400 rows per SM
+  const bool small = (long long)((P + 127) / 128) * (nz - 2) < 16LL * sms;
+  const int TZ = small ? 1 : 4;
   const int tiles_z = (nz - 2 + TZ - 1) / TZ;
   int nl, xr, ng;
   xstrip_groups(nx, H, P, nl, xr, ng);
@@ -285,7 +284,7 @@ int run(const sw_acoustic_params* p, const float* vp, const sw_acoustic_shot* s,
     if (small)
       k_ac2d_step<MODE_FWD, 4, 1, false, 3><<<blocks, 128, 0, st>>>(a);
     else
-      k_ac2d_step<MODE_FWD, 4, 1, true><<<blocks + xblocks, 128, 0, st>>>(a);
+      k_ac2d_step<MODE_FWD, 4, 1, true, 4><<<blocks + xblocks, 128, 0, st>>>(a);
     k_noalloc_inject_record<<<1, 128, 0, st>>>(T, pb[1 - pc], db, it);
     pc = 1 - pc;
     pk = 1 - pk;

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape,halo,nshots,nrec", [((150, 61), 12, 2, 300), ((33, 40), 0, 1, 1), ((517, 123), 9, 18, 130),
-                                                    ((131, 411), 20, 16, 5)])
+                                                    ((131, 411), 20, 16, 5), ((1100, 411), 9, 18, 40)])
 @pytest.mark.parametrize("check_freq", [1, 7])
 def test_sources_with_the_step(shape, halo, nshots, nrec, check_freq):
     h = (9.0, 8.0)
