@@ -2417,6 +2417,7 @@ void acoustic_gradient(sw_wavesim* ws, int nshots, const sw_acoustic_shot* shots
       // adjoint, shot sum -- as one graph
       std::vector<long long> key = group_key(ws, group, true);
       for (const auto& h : group) key.push_back(shots[h.orig].misfit_kind);
+      key.push_back(ccts_rec);  // the CCTS launch covers this many receivers
       for (int k = 0; k < S; ++k)  // the dense products' operands are launch arguments
         if (T.desc[k].icd) key.insert(key.end(), {k, T.desc[k].nrec, (long long)(uintptr_t)T.desc[k].icd});
       key.insert(key.end(), {accumulate ? 1 : 0, (long long)(uintptr_t)gout, (long long)(uintptr_t)mout});
