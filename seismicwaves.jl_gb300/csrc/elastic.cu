@@ -2469,7 +2469,7 @@ void elastic_gradient(sw_elastic* es, int nshots, const sw_elastic_shot* shots, 
       upload(es, es->d_scales, sc, "source scales");
     }
     std::vector<long long> key = {1, S, ntmax, es->tz, es->vec ? 1 : 0, es->split_disp ? 1 : 0, first_group ? 1 : 0,
-                                  mute ? 1 : 0,
+                                  mute ? 1 : 0, ccts_rec, (long long)ccts_smem,
                                   R.gx_src, R.gx_adj, R.gx_rec, (long long)(uintptr_t)out[0],
                                   (long long)(uintptr_t)out[1], (long long)(uintptr_t)out[2],
                                   (long long)(uintptr_t)mout};

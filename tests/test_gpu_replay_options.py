@@ -97,7 +97,7 @@ SEQUENCES = {
 }
 
 
-@pytest.mark.parametrize("family", ["cd", "vd"])
+@pytest.mark.parametrize("family", ["cd", "vd", "mt", "force"])
 @pytest.mark.parametrize("sequence", sorted(SEQUENCES))
 def test_every_call_is_bitwise_a_first_call(family, sequence):
     mute = 3 if sequence == "muting" else 0
