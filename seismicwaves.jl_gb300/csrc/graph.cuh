@@ -17,8 +17,9 @@ namespace swgb {
 // replayed afterwards, at most 32 graphs per simulation, later keys directly.
 // A time loop is thousands of short launches, which the host issues more
 // slowly than small grids execute them.  Work runs directly while profiling
-// (the events belong to single launches) and when the caller's stream is
-// itself being captured (the launches then join the caller's graph).
+// (the events belong to single launches), when the caller's stream is itself
+// being captured (the launches then join the caller's graph) and on the legacy
+// default stream, on which CUDA lets no capture begin.
 // `key` holds everything the captured launches depend on besides the device
 // buffers; `gen` is bumped whenever one of those is (re)allocated.
 struct GraphCache {
@@ -41,7 +42,7 @@ struct GraphCache {
     cudaStream_t st = ctx->stream;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     check_cuda(cudaStreamIsCapturing(st, &cs), "cudaStreamIsCapturing");
-    if (ctx->prof.on || cs != cudaStreamCaptureStatusNone) {
+    if (ctx->prof.on || cs != cudaStreamCaptureStatusNone || st == nullptr || st == cudaStreamLegacy) {
       work();
       return;
     }
