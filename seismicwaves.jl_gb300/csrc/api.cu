@@ -58,6 +58,7 @@ void vd_delete(sw_acoustic_vd* vd);
 
 void check_cuda(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return;
+  cudaGetLastError();  // a refused call also stays behind as the last error, which the next launch check would report
   const int code = (e == cudaErrorMemoryAllocation) ? SW_ERR_OOM : SW_ERR_CUDA;
   fail(code, std::string(what) + ": " + cudaGetErrorString(e));
 }
