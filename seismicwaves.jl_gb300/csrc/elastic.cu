@@ -63,6 +63,7 @@ namespace el {
 constexpr int XPAD = 32; // columns left of i = 1 (keeps each warp's 32 points on one 128-byte line)
 constexpr int ZPAD = 2;  // rows above j = 1
 constexpr int BX = 128;  // threads per block (x)
+constexpr int MAX_GRID_Y = 65535;
 constexpr int CTZ = 2;   // rows per block (correlation); the stencil kernels take theirs as a template parameter
 
 struct Geo {
@@ -1979,14 +1980,16 @@ void zero_state(sw_elastic* es, int S, bool adjoint) {
 // the launch fills the GPU (8 x 1200 x 600 gradient: 79.3 ms with 2 rows, 77.3
 // with 4, 79.7 with 8); a launch of fewer than 16 warps per SM takes shorter
 // bands (one shot of 333 x 217, gradient: 41.1 ms with 8 rows, 28.4 with 4,
-// 18.7 with 1).
-int band_rows(const sw_elastic* es, int S) {
-  if (es->tz > 0) return es->tz;
+// 18.7 with 1).  Always as many rows as it takes for the bands and `extra`
+// block rows to fit one grid.
+int band_rows(const sw_elastic* es, int S, int extra = 0) {
+  const int fit = MAX_GRID_Y - extra, least = (es->g.nz + fit - 1) / fit;
+  if (es->tz > 0) return std::max(es->tz, least);
   const int sms = es->ctx->num_sms > 0 ? es->ctx->num_sms : 148;
   const long long wx = (es->g.nx + 127) / 128;
   int tz = 4;
   while (tz > 1 && S * wx * ((es->g.nz + tz - 1) / tz) < 16LL * sms) tz /= 2;
-  return tz;
+  return std::max(tz, least);
 }
 
 // the one-point kernels (set_tuning + 64)
@@ -1997,14 +2000,20 @@ void launch_scalar(const sw_elastic* es, cudaStream_t st, const Args& a, int S, 
   else k_el_disp<TZ><<<grid, BX, 0, st>>>(a);
 }
 
+// Block rows that a recording of gx_rec blocks per shot adds to a stress launch of S shots.
+long long record_rows(const sw_elastic* es, int S, const RecordArgs& rec, int gx_rec) {
+  const long long columns = (long long)(es->g.nx + 511) / 512 * S;
+  return rec.it > 0 ? ((long long)gx_rec * rec.nshots + columns - 1) / columns : 0;
+}
+
 void launch_stencil(const sw_elastic* es, cudaStream_t st, Args a, int S, bool stress, RecordArgs rec = {},
                    int gx_rec = 0) {
   if (es->vec) {  // four points per thread: 512 per block
-    a.tz = band_rows(es, S);
+    const int rb = (int)record_rows(es, S, rec, gx_rec);
+    a.tz = band_rows(es, S, rb);
     const dim3 grid((unsigned)((es->g.nx + 511) / 512 * S), (unsigned)((es->g.nz + a.tz - 1) / a.tz));
     if (stress) {
       rec.bands = (int)grid.y;
-      const unsigned rb = rec.it > 0 ? ((unsigned)gx_rec * rec.nshots + grid.x - 1) / grid.x : 0;
       launch_chain("stress launch", k_el_stress4, dim3(grid.x, grid.y + rb), dim3(BX), st, a, rec);
     } else if (es->split_disp) {
       launch_chain("displacement launch", k_el_disp4_halves, dim3(2 * grid.x, grid.y), dim3(BX), st, a);
@@ -2027,6 +2036,7 @@ void full_step(Run& R, int S, int it, bool record, int kind, float* sU[2], float
   sw_elastic* es = R.es;
   Args a = R.args(false);
   if (sU) { a.sUx = sU[0]; a.sUz = sU[1]; a.sDx = sD[0]; a.sDz = sD[1]; }
+  if (record_rows(es, S, R.rec, R.gx_rec) > MAX_GRID_Y / 2) R.flush_record();  // leaves no room for the bands
   cudaEvent_t ev = nullptr;
   es->ctx->prof.begin(R.st, kind, 0.0, &ev);
   launch_stencil(es, R.st, a, S, true, R.rec, R.gx_rec);

@@ -73,6 +73,7 @@ struct Geo {
   __host__ __device__ __forceinline__ int xcol(int i) const { return i - 1 < WL ? i - 1 : WL + (i - 1 - xr); }
 };
 
+constexpr int MAX_GRID_Y = 65535;
 constexpr int STEP_MAXSP = 4;  // unique source points that the pressure update itself adds (step_sources)
 struct alignas(16) ShotDesc {
   int sx[STEP_MAXSP], sz[STEP_MAXSP];  // column and row of the first unique source points (0: none)
@@ -1231,6 +1232,12 @@ void unique_points(const sw_acoustic_vd* vd, const int32_t* idx, int count, std:
   }
 }
 
+// Block rows that the recording adds to a velocity launch, whose grid has (nx + 511) / 512 columns per shot.
+int record_rows(const sw_acoustic_vd* vd) {
+  const int tiles = (vd->g.nx + 511) / 512;
+  return (vd->gx_rec + tiles - 1) / tiles;
+}
+
 void build_tables(sw_acoustic_vd* vd, const sw_acoustic_shot* shots, const std::vector<HostShot>& group,
                   bool on_device, bool grad, std::vector<ShotDesc>& desc) {
   cudaStream_t st = vd->ctx->stream;
@@ -1398,6 +1405,7 @@ void build_tables(sw_acoustic_vd* vd, const sw_acoustic_shot* shots, const std::
       }
     }
   }
+  if (record_rows(vd) > MAX_GRID_Y / 2) vd->step_src = false;  // leaves no room for the bands
   upload(vd, vd->d_desc, desc, "shot descriptors");
 }
 
@@ -1469,12 +1477,14 @@ void zero_state(sw_acoustic_vd* vd, int S, bool adjoint) {
 // of its z window: 3 rows are fastest where the launch fills the GPU (8 x 2001
 // x 801 gradient: 79.9 ms with 2 rows, 78.1 with 3, 80.3 with 4, 93.5 with 8);
 // a launch of fewer than 16 warps per SM takes single rows (one shot of 402 x
-// 301: 14.9 us per step with 8 rows, 10.0 with 4, 7.5 with 1).
-int band_rows(const sw_acoustic_vd* vd, int S) {
-  if (vd->tz > 0) return vd->tz;
+// 301: 14.9 us per step with 8 rows, 10.0 with 4, 7.5 with 1).  Always as many
+// rows as it takes for the bands and `extra` block rows to fit one grid.
+int band_rows(const sw_acoustic_vd* vd, int S, int extra = 0) {
   const int sms = vd->ctx->num_sms > 0 ? vd->ctx->num_sms : 148;
   const long long wx = (vd->g.nx + 127) / 128;
-  return S * wx * ((vd->g.nz + 2) / 3) < 16LL * sms ? 1 : 3;
+  const int fit = MAX_GRID_Y - extra;
+  const int tz = vd->tz > 0 ? vd->tz : S * wx * ((vd->g.nz + 2) / 3) < 16LL * sms ? 1 : 3;
+  return std::max(tz, (vd->g.nz + fit - 1) / fit);
 }
 
 struct Run {
@@ -1527,10 +1537,11 @@ struct Run {
     launch_chain("pressure update launch", corr ? k_vd_p<true> : k_vd_p<false>, grid(S, a.tz), dim3(BX), st, a);
   }
   void launch_v(VArgs a, int S) const {
-    a.tz = band_rows(vd, S);
+    const int rec_rows = a.rec_it > 0 ? record_rows(vd) : 0;
+    a.tz = band_rows(vd, S, rec_rows);
     dim3 gr = grid(S, a.tz);
     a.bands = (int)gr.y;
-    if (a.rec_it > 0) gr.y += ((unsigned)vd->gx_rec * S + gr.x - 1) / gr.x;
+    gr.y += rec_rows;
     launch_chain("velocity update launch", k_vd_v, gr, dim3(BX), st, a);
   }
   // algorithmic bytes per node and shot: pressure R vx vz p, W p (16); velocity
