@@ -210,11 +210,11 @@ __global__ void k_inject_record(const ShotDesc* __restrict__ desc, const long lo
 
 // The recording of the last step that carried its own sources (StepRide).
 __global__ void k_ride_record(const StepShot* __restrict__ shots, const long long* __restrict__ rec_lin, FieldArg p,
-                              int it) {
+                              int it, int nshots) {
   chain_wait();
   chain_next();
-  const int s = blockIdx.y;
-  ride_record(shots[s], it, rec_lin, fptr(p, s), blockIdx.x * blockDim.x + threadIdx.x);
+  const int s = blockIdx.x % nshots;
+  ride_record(shots[s], it, rec_lin, fptr(p, s), blockIdx.x / nshots * blockDim.x + threadIdx.x);
 }
 
 // Adjoint injection at the receivers (adjoint_onestep_CPML! -> inject_sources!
@@ -1959,8 +1959,8 @@ void forward_group(sw_wavesim* ws, const std::vector<HostShot>& group, bool grad
   if (rec_it > 0) {
     cudaEvent_t ev = nullptr;
     ws->ctx->prof.begin(st, KK_SRCREC, 0.0, &ev);
-    launch_chain("record launch", k_ride_record, dim3((unsigned)ws->ride_rec, (unsigned)rec_shots), dim3(128), st,
-                 ws->d_ride.as<StepShot>(), ws->d_rec.as<long long>(), rec_p, rec_it);
+    launch_chain("record launch", k_ride_record, dim3((unsigned)((long long)ws->ride_rec * rec_shots)), dim3(128), st,
+                 ws->d_ride.as<StepShot>(), ws->d_rec.as<long long>(), rec_p, rec_it, rec_shots);
     ws->ctx->prof.end(st, KK_SRCREC, ev);
   }
 }

@@ -59,3 +59,17 @@ def test_elastic_recording_of_many_shots_that_end_together():
     run.close()
     ctx.close()
     assert all(np.abs(w).max() > 0 and np.array_equal(k[0], w) for k, w in zip(keep, want))
+
+
+def test_constant_density_recording_of_many_shots():
+    """More shots than a grid has block rows (the last step's recording is a launch of its own)."""
+    vp = C.smooth_model((33, 13), 1700.0, 3100.0, 5)
+    case = C.Case(vp=vp, h=(8.0, 8.0), dt=C.stable_dt(vp, (8.0, 8.0)), halo=2, freetop=False)
+    shots = [C.make_shot(case.h, None, n, case.dt, 120.0, [[128.0, 48.0]], [[128.0, 56.0]]) for n in (7, 7)]
+    run = C.GpuRun(sw, case)
+    want = [np.array(t) for t in run.forward(shots)]
+    arr, keep, outs = run._structs(shots, False)
+    many = _repeat(sw._lib.SwAcousticShot, arr[1], 66000, arr[0])
+    run.ctx.check(run.ctx.lib.sw_acoustic_forward(run.h, len(many), many, 0), "forward")
+    run.close()
+    assert all(np.abs(w).max() > 0 and np.array_equal(o, w) for o, w in zip(outs, want))
