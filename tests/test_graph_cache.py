@@ -104,3 +104,22 @@ def test_captured_on_the_second_call(probe):
 @pytest.mark.parametrize("legacy", [0, 1])
 def test_legacy_default_stream_runs_directly(probe, legacy):
     assert probe(legacy, 5, 5, 5, 5) == ("dddd", 0)
+
+
+def test_graphs_of_freed_buffers_are_given_back(probe):
+    assert probe(64, 5, 5, 6, 6, "+", 5, 5, 5) == ("dcdcdcr", 1)
+
+
+def test_other_keys_take_over_from_unused_ones(probe):
+    """32 graphs whose keys do not come back (other output arrays, say) make room for those in use."""
+    old = [k for key in range(100, 132) for k in (key, key)]
+    how, held = probe(64, *old, *[7] * 300)
+    assert how[:64] == "dc" * 32 and held == 32
+    late = how[64:]
+    assert "c" in late and late == "d" * late.index("c") + "c" + "r" * (299 - late.index("c"))
+
+
+def test_more_keys_than_graphs_in_turn(probe):
+    """40 keys in turn: 32 are replayed throughout, the others run directly, none is captured twice."""
+    how, held = probe(64, *list(range(40)) * 20)
+    assert held == 32 and how.count("c") == 32 and how.count("r") == 32 * 18
