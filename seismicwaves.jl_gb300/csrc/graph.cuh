@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <limits>
 #include <map>
 #include <utility>
 #include <vector>
@@ -86,6 +87,12 @@ struct GraphCache {
       cudaGraphExec_t ex = nullptr;
       const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
       cudaGraphDestroy(g);
+      if (e == cudaErrorMemoryAllocation) {  // no memory for the graph: this key goes on running directly
+        cudaGetLastError();
+        uses[key] = std::numeric_limits<int>::min();
+        work();
+        return;
+      }
       check_cuda(e, "graph instantiate");
       it = graphs.emplace(key, Held{ex, 0}).first;
     }

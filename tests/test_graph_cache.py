@@ -17,6 +17,7 @@ PROBE = r"""
 
 namespace {
 bool capturing = false;
+bool full = false;
 long long made = 0, live = 0, launched = 0;
 }
 extern "C" {
@@ -36,6 +37,7 @@ cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
 }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+  if (full) return cudaErrorMemoryAllocation;
   *e = reinterpret_cast<cudaGraphExec_t>(++made);
   ++live;
   return cudaSuccess;
@@ -53,8 +55,9 @@ void check_cuda(cudaError_t e, const char* what) {
 Profiler::~Profiler() {}
 }  // namespace swgb
 
-// argv: stream handle, then per call "key" or "+" (a buffer was reallocated); prints per call whether the work ran
-// directly (d), was captured (c) or replayed (r), then the number of graphs held
+// argv: stream handle, then per call "key", "+" (a buffer was reallocated) or "!" (the device's memory is full from
+// here on); prints per call whether the work ran directly (d), was captured (c) or replayed (r) or the call failed (x),
+// then the number of graphs held
 int main(int argc, char** argv) {
   sw_ctx ctx;
   ctx.stream = reinterpret_cast<cudaStream_t>(std::atoll(argv[1]));
@@ -62,6 +65,10 @@ int main(int argc, char** argv) {
   for (int k = 2; k < argc; ++k) {
     if (argv[k][0] == '+') {
       ++cache.gen;
+      continue;
+    }
+    if (argv[k][0] == '!') {
+      full = true;
       continue;
     }
     char how = 'r';
@@ -123,3 +130,7 @@ def test_more_keys_than_graphs_in_turn(probe):
     """40 keys in turn: 32 are replayed throughout, the others run directly, none is captured twice."""
     how, held = probe(64, *list(range(40)) * 20)
     assert held == 32 and how.count("c") == 32 and how.count("r") == 32 * 18
+
+
+def test_no_memory_for_a_graph(probe):
+    assert probe(64, 5, 5, "!", 6, 6, 6, 5, 6) == ("dcdddrd", 1)
