@@ -1190,7 +1190,11 @@ enum { TZ_FORWARD = 0, TZ_RECOMPUTE = 1, TZ_ADJOINT = 2 };
 // one row is all there is to win (one shot of 201 x 201: 5.2 us per step
 // against 7.0 with the strips split off in 2-row bands, 5.6 at 4 blocks per
 // SM; 2 shots of 301 x 187, gradient: 6.3 against 8.3 ms; one of 801 x 801, 37
-// rows per SM: 38.2 against 31.1).
+// rows per SM: 38.2 against 31.1).  The kernel is for single rows only: with
+// explicit taller bands (set_tuning, set_band_heights) the kernels of mid_2d
+// are faster at every size (one shot of 201 x 201, 300 steps: 1.12 ms with
+// single rows against 1.20; 1.46 against 1.21 with 2 rows, 3.7 against 2.2 with
+// 8, 19.9 against 8.8 with 64).
 bool small_2d(const sw_wavesim* ws, int S) {
   const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
   return ws->N == 2 && (long long)S * ((ws->P + 127) / 128) * (ws->n[1] - 2) < 16LL * sms;
@@ -1420,10 +1424,10 @@ long long xstrip_blocks(const StepArgs& a) {
 // `blocks` main blocks for the lanes outside the x strips, then one block
 // per 128 lane groups of the x strips (rows x shots), which run in the tail
 // of the launch (79.5 against 78.4 Gpts/s as a second launch on the 64-shot
-// headline).  A small launch (small_2d) takes the one-kernel form with
-// registers for every load of a row to be in flight.  Returns the number of
-// kernels launched.
-enum Size2d { ROWS_2D, FEW_2D, FULL_2D };  // small_2d, mid_2d, larger
+// headline).  The single rows of a small launch (small_2d) take the one-kernel
+// form with registers for every load of a row to be in flight.  Returns the
+// number of kernels launched.
+enum Size2d { ROWS_2D, FEW_2D, FULL_2D };  // single rows of small_2d, mid_2d, larger
 template <int MODE, bool RIDE>
 void launch_2d(long long blocks, Size2d size, cudaStream_t st, const StepArgs& a) {
   launch_chain("stencil launch",
@@ -1432,7 +1436,9 @@ void launch_2d(long long blocks, Size2d size, cudaStream_t st, const StepArgs& a
                                 : k_ac2d_step<MODE, 4, 1, true, Ac2dBounds<MODE, 4>::MINB, RIDE>,
                dim3((unsigned)blocks), dim3(128), st, a);
 }
-Size2d size_2d(const sw_wavesim* ws, int S) { return small_2d(ws, S) ? ROWS_2D : mid_2d(ws, S) ? FEW_2D : FULL_2D; }
+Size2d size_2d(const sw_wavesim* ws, int S, int tz) {
+  return tz == 1 && small_2d(ws, S) ? ROWS_2D : mid_2d(ws, S) ? FEW_2D : FULL_2D;
+}
 template <int MODE>
 int launch_2d_xsplit(long long blocks, Size2d size, cudaStream_t st, StepArgs a, int rec_blocks) {
   if (size != ROWS_2D) blocks += xstrip_blocks(a);
@@ -1517,7 +1523,7 @@ struct Launcher {
         enable_cpa_carveout<MODE>();
         k_ac2d_cpa<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       } else if (nw == 4 && ws->xsplit)
-        nk = launch_2d_xsplit<MODE>(blocks, size_2d(ws, a.nshots), st, a, ws->ride_rec);
+        nk = launch_2d_xsplit<MODE>(blocks, size_2d(ws, a.nshots, c.TZ), st, a, ws->ride_rec);
       else if (nw == 4)
         k_ac2d_step<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       else if (nw == 8)
@@ -1543,7 +1549,7 @@ struct Launcher {
       }
       if (launched) {
       } else if (nw == 4 && ws->xsplit)
-        nk = launch_2d_xsplit<MODE>(blocks, size_2d(ws, a.nshots), st, a, ws->ride_rec);
+        nk = launch_2d_xsplit<MODE>(blocks, size_2d(ws, a.nshots, c.TZ), st, a, ws->ride_rec);
       else if (nw == 4)
         k_ac2d_step<MODE, 4><<<(unsigned)blocks, 128, 0, st>>>(a);
       else if (nw == 8)
