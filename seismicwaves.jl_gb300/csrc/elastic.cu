@@ -187,7 +187,9 @@ __global__ void __launch_bounds__(BX) k_el_stress(const Args A) {
   float* pzF = A.pz[3] + (long long)s * A.zs;
   int colE = 0, colG = 0;
   const int kE = cpml_full(i, g.nx, g.halo, colE);  // dux/dx at sigma_xx nodes (ux has nx-1 points)
+  colE = g.xcol(i);
   const int kG = cpml_half(i, g.nx, g.halo, colG);  // duz/dx at sigma_xz nodes (uz has nx points)
+  colG = g.xcol(i);
   const int jlo = g.ft ? 1 : 2;
   const int P = g.P;
   long long c = g.lin(i, j0);
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(BX) k_el_stress(const Args A) {
         else if (g.ft && j == 2) duz = d4(zu1, zu1, zu2, zu3, g.idz);
         else duz = d4(zu0, zu1, zu2, zu3, g.idz);
         float duxc = dux, duzc = duz;
-        if (kE) duxc = cpml_upd(pxE + (long long)(j - 1) * g.W + g.xcol(i), cx[kE - 1], cx[na + nh + kE - 1], dux);
+        if (kE) duxc = cpml_upd(pxE + (long long)(j - 1) * g.W + colE, cx[kE - 1], cx[na + nh + kE - 1], dux);
         int colF = 0;
         const int kF = cpml_full(j, g.nz, g.halo, colF);  // duz/dz (uz has nz-1 points)
         if (kF) duzc = cpml_upd(pzF + (long long)colF * P + (i - 1), cz[kF - 1], cz[na + nh + kF - 1], duz);
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(BX) k_el_stress(const Args A) {
       const float dzx = d4(uzm1, zu2, uzp1, uzp2, g.idx);
       const float dxz = (g.ft && j == 1) ? d4(xu2, xu1, xu2, xu3, g.idz) : d4(xu0, xu1, xu2, xu3, g.idz);
       float dzxc = dzx, dxzc = dxz;
-      if (kG) dzxc = cpml_upd(pxG + (long long)(j - 1) * g.W + g.xcol(i), cx[na + kG - 1], cx[2 * na + nh + kG - 1], dzx);
+      if (kG) dzxc = cpml_upd(pxG + (long long)(j - 1) * g.W + colG, cx[na + kG - 1], cx[2 * na + nh + kG - 1], dzx);
       int colH = 0;
       const int kH = cpml_half(j, g.nz, g.halo, colH);  // dux/dz (ux has nz points)
       if (kH) dxzc = cpml_upd(pzH + (long long)colH * P + (i - 1), cz[na + kH - 1], cz[2 * na + nh + kH - 1], dxz);
@@ -271,7 +273,9 @@ __global__ void __launch_bounds__(BX) k_el_disp(const Args A) {
   float* pzB = A.pz[1] + (long long)s * A.zs;
   int colA = 0, colC = 0;
   const int kA = cpml_half(i, g.nx, g.halo, colA);  // dsxx/dx at ux nodes (sigma_xx has nx points)
+  colA = g.xcol(i);
   const int kC = cpml_full(i, g.nx, g.halo, colC);  // dsxz/dx at uz nodes (sigma_xz has nx-1 points)
+  colC = g.xcol(i);
   const bool slots = A.sUx != nullptr;
   const int P = g.P;
   long long c = g.lin(i, j0);
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__(BX) k_el_disp(const Args A) {
       else if (g.ft && j == 2) d2 = d4(-q1, q1, q2, q3, g.idz);
       else d2 = d4(q0, q1, q2, q3, g.idz);
       float d1c = d1, d2c = d2;
-      if (kA) d1c = cpml_upd(pxA + (long long)(j - 1) * g.W + g.xcol(i), cx[na + kA - 1], cx[2 * na + nh + kA - 1], d1);
+      if (kA) d1c = cpml_upd(pxA + (long long)(j - 1) * g.W + colA, cx[na + kA - 1], cx[2 * na + nh + kA - 1], d1);
       int colB = 0;
       const int kB = cpml_full(j, g.nz, g.halo, colB);  // dsxz/dz (sigma_xz has nz-1 points)
       if (kB) d2c = cpml_upd(pzB + (long long)colB * P + (i - 1), cz[kB - 1], cz[na + nh + kB - 1], d2);
@@ -317,7 +321,7 @@ __global__ void __launch_bounds__(BX) k_el_disp(const Args A) {
       const float d1 = d4(qm2, qm1, q2, qp1, g.idx);
       const float d2 = (g.ft && j == 1) ? d4(-w2, w1, w2, w3, g.idz) : d4(w0, w1, w2, w3, g.idz);
       float d1c = d1, d2c = d2;
-      if (kC) d1c = cpml_upd(pxC + (long long)(j - 1) * g.W + g.xcol(i), cx[kC - 1], cx[na + nh + kC - 1], d1);
+      if (kC) d1c = cpml_upd(pxC + (long long)(j - 1) * g.W + colC, cx[kC - 1], cx[na + nh + kC - 1], d1);
       int colD = 0;
       const int kD = cpml_half(j, g.nz, g.halo, colD);  // dszz/dz (sigma_zz has nz points)
       if (kD) d2c = cpml_upd(pzD + (long long)colD * P + (i - 1), cz[na + kD - 1], cz[2 * na + nh + kD - 1], d2);
