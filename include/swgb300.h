@@ -370,10 +370,10 @@ int sw_elastic_forward_snapshots(sw_elastic* es, int32_t nshots, const sw_elasti
 
 /* Rows per thread block of the elastic stencil kernels: 8, 16 or 32 (0 =
  * default: 4, fewer for launches that would leave SMs short of warps; 8 for
- * the one-point kernels); + 64 selects the one-point-per-thread kernels
- * instead of the four-points-per-thread ones.  The four-point kernels update
- * ux and uz by blocks of their own; + 128 by the same threads.  A tuning knob
- * of this backend; no reference counterpart. */
+ * the one-point kernels; bands grow on grids too deep for them); + 64 selects
+ * the one-point-per-thread kernels instead of the four-points-per-thread ones.
+ * The four-point kernels update ux and uz by blocks of their own; + 128 by the
+ * same threads.  A tuning knob of this backend; no reference counterpart. */
 int sw_elastic_set_tuning(sw_elastic* es, int32_t tz);
 
 /* ---------------------------------------------------------------------------

@@ -564,7 +564,7 @@ struct sw_wavesim {
   DevMem d_pair, d_recstash, d_stash;     // two-step launches: per-shot source / receiver-row table,
                                           // receiver -> stash index, first-step pressure of receiver rows
   bool pair_on = false;                   // 2D: two time steps per launch where possible (tuning variant)
-  bool split3d = true;                    // 3D: inner rows and strip rows as two launches (variant bit 16: one)
+  bool split3d = true;                    // 3D: x-strip groups and all other rows as two launches (variant bit 16: one)
   bool xsplit = true;                     // 2D 4-warp stencil: x strips as extra blocks (variant bit 18: not)
   int pair_tz = 0;                        // rows per block of the two-step kernel (0 = heuristic)
   int pair_occ = 0;                       // resident-block bound of the two-step kernel (0 = default, 1, 2)
@@ -1204,8 +1204,10 @@ bool small_2d(const sw_wavesim* ws, int S) {
 // registers spill nothing, in place of 8 (forward) or 6 (adjoint).  They do not
 // fill more warps than that for long, and every row is faster (gradient of one
 // shot of 801 x 801, 400 steps, 37 rows per SM: 8.1 ms against 11.2, of 601 x
-// 601: 7.7 against 10.7, of 8 of 801 x 801, 200 steps, 294 rows: 18.1 against
-// 19.4; 16 of 2001 x 801, 1346 rows: 43.7 against 39.7).
+// 601: 7.7 against 10.7).  The two meet between 300 and 400 rows: gradient, 200
+// steps, of 8 of 801 x 801 (294 rows) 18.2 against 19.3, of 4 of 2001 x 801 (336)
+// 19.8 against 19.7, of 10 of 801 x 801 (368) 24.3 against 24.7, of 19 of 601 x
+// 601 (374) 27.5 against 26.9; 16 of 2001 x 801 (1346) 43.7 against 39.7.
 bool mid_2d(const sw_wavesim* ws, int S) {
   const int sms = ws->ctx->num_sms > 0 ? ws->ctx->num_sms : 148;
   return ws->N == 2 && (long long)S * ((ws->P + 127) / 128) * (ws->n[1] - 2) < 400LL * sms;
@@ -1980,6 +1982,7 @@ void adjoint_group(sw_wavesim* ws, const std::vector<HostShot>& group) {
   const bool bf16 = ws->gp.snapshot_bf16 == 2;
   const long long slot = bf16 ? ws->strip_total : 2 * F + ws->strip_total;
   Launcher L{ws, st};
+  // also the full dependency between the misfit kernels and the chained launches, which read the adjoint sources early
   zero_state(ws, S, true);
   check_cuda(cudaMemsetAsync(ws->g.p, 0, (size_t)S * F * sizeof(float), st), "reset g");
   check_cuda(cudaMemsetAsync(ws->gc.p, 0, (size_t)S * F * sizeof(float), st), "reset gc");

@@ -21,12 +21,17 @@
 // Rules that keep the chain safe: a kernel launched with launch_chain calls
 // chain_wait in every thread before it returns or touches anything that an
 // earlier kernel of the chain reads or writes (so a kernel completes after its
-// predecessor, and its successor's wait covers the whole chain); the tables
-// read before the wait are uploaded by copies or memsets, which the first
-// kernel of a chain waits for in full; a kernel that reads what the loop writes
-// through the read-only path takes its thread index from chain_wait_tid.  A kernel launched plainly, a copy or
-// a memset waits for everything before it as always, and chain_wait in a
-// plainly launched kernel returns at once.
+// predecessor, and its successor's wait covers the whole chain); what a kernel
+// reads before its wait (shot tables, source time functions, adjoint sources
+// and their scale) is written before a full dependency that lies ahead of the
+// chain: a copy, a memset or a plainly launched kernel, none of which starts
+// before everything ahead of it is complete.  For the adjoint sources, which
+// the misfit kernels write, the memsets between these and the adjoint loop are
+// that dependency; they may not become chained kernels.  A kernel that reads
+// what the loop writes through the read-only path takes its thread index from
+// chain_wait_tid.  A kernel launched plainly, a copy or a memset waits for
+// everything before it as always, and chain_wait in a plainly launched kernel
+// returns at once.
 #pragma once
 
 #include <cuda_runtime.h>

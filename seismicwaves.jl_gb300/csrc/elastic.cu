@@ -396,7 +396,10 @@ __device__ __forceinline__ float d4r(float f1, float f2, float f3, float f4, flo
   return __fmul_rn(__fmaf_rn(-c1, f4, u), inv);
 }
 // d4 along x at a thread's four points from the seven values around them; bit
-// e of ROUND3 sets point e's rounding.
+// e of ROUND3 sets point e's rounding.  The masks that the kernels pass are the
+// choices that nvcc had made in them before the rounding was spelled out: with
+// them every result keeps its bits, and nothing else speaks for one mask or
+// another.
 template <unsigned ROUND3>
 __device__ __forceinline__ void d4x(float (&d)[4], const float (&a)[7], float inv) {
   d[0] = d4r<(ROUND3 & 1) != 0>(a[0], a[1], a[2], a[3], inv);
@@ -2537,7 +2540,8 @@ void elastic_gradient(sw_elastic* es, int nshots, const sw_elastic_shot* shots, 
       }
       k_el_adj_scale<<<1, 1, 0, st>>>(es->d_amax.as<unsigned>(), es->d_scales.as<float>());
       check_cuda(cudaGetLastError(), "adjoint scale launch");
-      // adjoint with recompute and correlation
+      // adjoint with recompute and correlation; the memsets are also the full dependency between the
+      // misfit kernels and the chained launches, which read the adjoint sources early
       zero_state(es, S, true);
       check_cuda(cudaMemsetAsync(es->acc.p, 0, (size_t)ngroups * 10 * F * sizeof(float), st), "accumulators clear");
       Args ca = R.args(true);

@@ -238,8 +238,10 @@ int run(const sw_acoustic_params* p, const float* vp, const sw_acoustic_shot* s,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tiles_x = (P + 511) / 512;
   // the batched path's rules (small_2d, mid_2d): single rows without x-strip
-  // blocks below 16 rows per SM, else 4-row bands with the x strips split off;
-  // the grids that fit the scratch stay below 400 rows per SM
+  // blocks below 16 rows per SM, else 4-row bands with the x strips split off
+  // and four blocks per SM.  Of the grids that fit the scratch only very deep
+  // ones of at most 64 columns pass the 400 rows per SM of mid_2d (32 x 100000,
+  // 200 steps: 13.2 ms, 20.3 as one kernel with 8-row bands).
   const bool small = (long long)((P + 127) / 128) * (nz - 2) < 16LL * sms;
   const int TZ = small ? 1 : 4;
   const int tiles_z = (nz - 2 + TZ - 1) / TZ;

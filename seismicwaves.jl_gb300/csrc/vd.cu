@@ -144,7 +144,10 @@ __device__ __forceinline__ float d4(float f1, float f2, float f3, float f4, floa
   return __fmul_rn(__fmaf_rn(-c1, f4, u), inv);
 }
 // d4 along x at a thread's four points from the seven values around them; bit
-// e of ROUND3 sets point e's rounding.
+// e of ROUND3 sets point e's rounding.  The masks that the kernels pass are the
+// choices that nvcc had made in them before the rounding was spelled out: with
+// them every result keeps its bits, and nothing else speaks for one mask or
+// another.
 template <unsigned ROUND3>
 __device__ __forceinline__ void d4x(float (&d)[4], const float (&a)[7], float inv) {
   d[0] = d4<(ROUND3 & 1) != 0>(a[0], a[1], a[2], a[3], inv);
@@ -2050,7 +2053,8 @@ void vd_gradient(sw_acoustic_vd* vd, int nshots, const sw_acoustic_shot* shots, 
         }
         vd->ctx->prof.end(st, KK_OTHER, ev);
       }
-      // adjoint with recompute, fused correlation and window flushes
+      // adjoint with recompute, fused correlation and window flushes; the memsets are also the full
+      // dependency between the misfit kernels and the chained launches, which read the adjoint sources early
       zero_state(vd, S, true);
       check_cuda(cudaMemsetAsync(vd->acc.p, 0, (size_t)S * 3 * F * sizeof(float), st), "window sums clear");
       check_cuda(cudaMemsetAsync(vd->tot.p, 0, (size_t)ngroups * 3 * F * sizeof(double), st), "totals clear");
